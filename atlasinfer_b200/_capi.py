@@ -21,7 +21,7 @@ DTYPE_F16, DTYPE_BF16 = 0, 1
 EXPORTS = (
     "atlas_version", "atlas_last_error", "atlas_status_string",
     "atlas_quantize_workspace_bytes", "atlas_quantize", "atlas_quantize_noalloc", "atlas_dequantize",
-    "atlas_tiles_bytes", "atlas_repack", "atlas_qlinear_gemv",
+    "atlas_tiles_bytes", "atlas_repack", "atlas_repack_many", "atlas_qlinear_gemv",
     "atlas_qlinear_stream_workspace_bytes", "atlas_qlinear_stream", "atlas_qlinear_stream_gather",
     "atlas_peer_wait", "atlas_peer_push", "atlas_peer_alloc", "atlas_peer_free", "atlas_peer_export", "atlas_peer_import",
     "atlas_peer_release",
@@ -38,6 +38,18 @@ class PeerGather(ctypes.Structure):
     _fields_ = [("world", ctypes.c_int32), ("rank", ctypes.c_int32),
                 ("y_dst", ctypes.c_void_p * MAX_PEERS), ("flags_dst", ctypes.c_void_p * MAX_PEERS),
                 ("state", ctypes.c_void_p), ("wait_flags", ctypes.c_void_p), ("poll_limit", ctypes.c_int64)]
+
+
+
+class RepackItem(ctypes.Structure):
+    """``AtlasRepackItem`` of include/atlas_b200.h."""
+
+    _fields_ = [("codes", ctypes.c_void_p), ("n_codes", ctypes.c_int64), ("outlier_vals", ctypes.c_void_p),
+                ("outlier_idx", ctypes.c_void_p), ("n_outliers", ctypes.c_int64), ("scales", ctypes.c_void_p),
+                ("n_rows", ctypes.c_int64), ("n_cols", ctypes.c_int64), ("block_size", ctypes.c_int64),
+                ("tiles", ctypes.c_void_p), ("scales_tiled", ctypes.c_void_p), ("outlier_row_ptr", ctypes.c_void_p),
+                ("outlier_chunk_ptr", ctypes.c_void_p), ("outlier_entries", ctypes.c_void_p),
+                ("outlier_vals_sorted", ctypes.c_void_p), ("entry_base", ctypes.c_int64)]
 
 
 _lib: Optional[ctypes.CDLL] = None
@@ -78,6 +90,8 @@ def load() -> ctypes.CDLL:
     L.atlas_tiles_bytes.argtypes = [i64, i64]
     L.atlas_repack.restype = i32
     L.atlas_repack.argtypes = [vp, i64, vp, vp, i64, vp, i64, i64, i32, vp, vp, vp, vp, vp, vp, vp]
+    L.atlas_repack_many.restype = i32
+    L.atlas_repack_many.argtypes = [i32, ctypes.POINTER(RepackItem), vp]
     lin = [vp, i32, i64, i64, vp, vp, vp, vp, vp, i64, i64, i32, vp, vp, i64]
     L.atlas_qlinear_gemv.restype = i32
     L.atlas_qlinear_gemv.argtypes = lin + [vp, vp]

@@ -102,33 +102,63 @@ def kernel_layout_supported(shape, block_size: int) -> Optional[str]:
 
 def build_kernel_layout(q: QuantizedTensor) -> KernelLayout:
     """Expand the compacted code stream of ``q`` (on a CUDA device) into the kernel layout."""
-    reason = kernel_layout_supported(q.original_shape, int(q.block_size))
-    if reason is not None:
-        raise NotImplementedError("QuantizedLinear: " + reason)
+    return build_joined_layout([q])[0]
+
+
+def build_joined_layout(qs):
+    """The kernel layouts of ``qs`` (one device, in_features and block size) as the rows of one layout, back to back.
+
+    Returns ``(layout, row offsets)``.  Every member but the last is padded to whole 128-row tiles, as in
+    ``concat_layouts``, but the members are expanded straight into the joined buffers by one launch.  The CSR row
+    pointers of the canonical streams are only written for a single tensor."""
+    for q in qs:
+        reason = kernel_layout_supported(q.original_shape, int(q.block_size))
+        if reason is not None:
+            raise NotImplementedError("QuantizedLinear: " + reason)
     L = _capi.load()
-    dev = q.fp8_data.device
-    n, k = int(q.original_shape[0]), int(q.original_shape[1])
-    n_out = q.outlier_indices.numel()
-    bs = int(q.block_size)
-    n_pad = (n + 127) // 128 * 128
+    dev = qs[0].fp8_data.device
+    k, bs = int(qs[0].original_shape[1]), int(qs[0].block_size)
+    if any((int(q.original_shape[1]), int(q.block_size)) != (k, bs) for q in qs):
+        raise ValueError("fused linears must share in_features and block size")
+    rows = [int(q.original_shape[0]) for q in qs]
+    padded = [(n + 127) // 128 * 128 for n in rows]
+    n_pad, n_out = sum(padded), sum(q.outlier_indices.numel() for q in qs)
+    chunks = k // 64 + 1
     with torch.cuda.device(dev):
-        tiles = torch.empty(int(L.atlas_tiles_bytes(n, k)), dtype=torch.uint8, device=dev)
+        tiles = torch.empty(n_pad * k, dtype=torch.uint8, device=dev)
         scales_tiled = torch.empty(n_pad * (k // bs), dtype=torch.float16, device=dev)
-        row_ptr = torch.empty(n + 1, dtype=torch.int32, device=dev)
-        chunk_ptr = torch.empty((n_pad // 16) * (k // 64 + 1), dtype=torch.int32, device=dev)
+        row_ptr = torch.empty(rows[0] + 1 if len(qs) == 1 else 0, dtype=torch.int32, device=dev)
+        chunk_ptr = torch.empty((n_pad // 16) * chunks, dtype=torch.int32, device=dev)
         entries = torch.empty(n_out, dtype=torch.int32, device=dev)
         vals_sorted = torch.empty(n_out, dtype=torch.float16, device=dev)
-        codes, oidx = q.fp8_data.contiguous(), q.outlier_indices.contiguous()
-        ovals, scales = q.fp16_outliers.contiguous(), q.scale_factors.contiguous()
-        status = L.atlas_repack(_capi.ptr(codes), codes.numel(), _capi.ptr(ovals), _capi.ptr(oidx), n_out,
-                                scales.data_ptr(), n, k, bs, tiles.data_ptr(), scales_tiled.data_ptr(),
-                                row_ptr.data_ptr(), chunk_ptr.data_ptr(), _capi.ptr(entries),
-                                _capi.ptr(vals_sorted), _capi.stream_ptr(dev))
+        items = (_capi.RepackItem * len(qs))()
+        offsets, held, row, entry = [], [], 0, 0
+        for item, q, n, n_p in zip(items, qs, rows, padded):
+            codes, oidx = q.fp8_data.contiguous(), q.outlier_indices.contiguous()
+            ovals, scales = q.fp16_outliers.contiguous(), q.scale_factors.contiguous()
+            held.append((codes, oidx, ovals, scales))   # alive until the kernel has read them
+            item.codes, item.n_codes = _capi.ptr(codes), codes.numel()
+            item.outlier_vals, item.outlier_idx, item.n_outliers = _capi.ptr(ovals), _capi.ptr(oidx), oidx.numel()
+            item.scales, item.n_rows, item.n_cols, item.block_size = scales.data_ptr(), n, k, bs
+            item.tiles = tiles.data_ptr() + row * k
+            item.scales_tiled = scales_tiled.data_ptr() + row * (k // bs) * 2
+            item.outlier_row_ptr = _capi.ptr(row_ptr)
+            item.outlier_chunk_ptr = chunk_ptr.data_ptr() + (row // 16) * chunks * 4
+            if n_out:
+                item.outlier_entries = entries.data_ptr() + entry * 4
+                item.outlier_vals_sorted = vals_sorted.data_ptr() + entry * 2
+            item.entry_base = entry
+            offsets.append(row)
+            row += n_p
+            entry += oidx.numel()
+        status = L.atlas_repack_many(len(qs), items, _capi.stream_ptr(dev))
     _capi.check(status, "atlas_repack")
     # the linear kernels read the weight-side buffers before the stream's earlier work has completed
     # (programmatic dependent launch), so the layout must be final before any of them is launched
     torch.cuda.current_stream(dev).synchronize()
-    return KernelLayout(q, tiles, scales_tiled, row_ptr, chunk_ptr, entries, vals_sorted, n, k, bs)
+    source = qs[0] if len(qs) == 1 else tuple(qs)
+    return KernelLayout(source, tiles, scales_tiled, row_ptr, chunk_ptr, entries, vals_sorted,
+                        n_pad - padded[-1] + rows[-1], k, bs), offsets
 
 
 def quantized_linear_forward(x: torch.Tensor, layout: KernelLayout, bias: Optional[torch.Tensor],
@@ -247,29 +277,33 @@ class FusedLinearGroup:
             mod._group_index = i
 
     def build(self, dev: torch.device) -> None:
-        layouts = []
         for mod in self.members:
             q = mod.quantized_weights
             if q.fp8_data.device != dev:
-                q = q.to(dev)
-                mod.quantized_weights = q
+                mod.quantized_weights = q.to(dev)
             if mod.bias is not None and mod.bias.device != dev:
                 mod.bias = mod.bias.to(dev)
-            layouts.append(mod._layout_for(q))
-        fused = concat_layouts(layouts)
-        self.offsets, off = [], 0
-        for lay in layouts:
-            self.offsets.append(off)
-            off += (lay.n_rows + 127) // 128 * 128
+        sources = [mod.quantized_weights for mod in self.members]
+        if any(mod._has_layout_for(q) for mod, q in zip(self.members, sources)):
+            # members that are laid out already are joined as they are
+            layouts = [mod._layout_for(q) for mod, q in zip(self.members, sources)]
+            fused = concat_layouts(layouts)
+            self.offsets, off = [], 0
+            for lay in layouts:
+                self.offsets.append(off)
+                off += (lay.n_rows + 127) // 128 * 128
+        else:
+            fused, self.offsets = build_joined_layout(sources)
+        rows = [int(q.original_shape[0]) for q in sources]
         if any(mod.bias is not None for mod in self.members):
             b = torch.zeros(fused.n_rows, dtype=torch.float16, device=dev)
-            for mod, lay, o in zip(self.members, layouts, self.offsets):
+            for mod, n, o in zip(self.members, rows, self.offsets):
                 if mod.bias is not None:
-                    b[o:o + lay.n_rows] = mod.bias.to(torch.float16)
+                    b[o:o + n] = mod.bias.to(torch.float16)
             self.bias = b
         # the members now look at the joined buffers; their own copies are released
-        for mod, lay, o in zip(self.members, layouts, self.offsets):
-            mod._kernel_layout = slice_layout(fused, o, lay.n_rows, lay.source)
+        for mod, q, n, o in zip(self.members, sources, rows, self.offsets):
+            mod._kernel_layout = slice_layout(fused, o, n, q)
         self.layout = fused
         torch.cuda.current_stream(dev).synchronize()
 
@@ -333,12 +367,14 @@ class QuantizedLinear(nn.Module):
             self._bias_f16 = cached
         return cached[1]
 
-    def _layout_for(self, q: QuantizedTensor) -> KernelLayout:
+    def _has_layout_for(self, q: QuantizedTensor) -> bool:
         lay = self._kernel_layout
-        if lay is None or lay.source is not q or lay.tiles.device != q.fp8_data.device:
-            lay = build_kernel_layout(q)
-            self._kernel_layout = lay
-        return lay
+        return lay is not None and lay.source is q and lay.tiles.device == q.fp8_data.device
+
+    def _layout_for(self, q: QuantizedTensor) -> KernelLayout:
+        if not self._has_layout_for(q):
+            self._kernel_layout = build_kernel_layout(q)
+        return self._kernel_layout
 
     def offload_canonical(self, device="cpu") -> None:
         """Keep only the kernel layout on the GPU: the canonical streams move to ``device`` (host by default).

@@ -153,6 +153,29 @@ ATLAS_API int atlas_repack(const int8_t *codes, int64_t n_codes, const void *out
                            void *scales_tiled, int32_t *outlier_row_ptr, int32_t *outlier_chunk_ptr,
                            uint32_t *outlier_entries, void *outlier_vals_sorted, void *stream);
 
+/* Several tensors in one launch (8 at a time).  The arguments of one tensor are those of atlas_repack, except that
+ * outlier_row_ptr may be NULL (not wanted) and that entry_base is added to what outlier_chunk_ptr holds: a tensor
+ * whose tiles, scales, chunk pointers and entries are written behind one another's into common buffers (rows padded
+ * to 128, entry_base = entries of the tensors before it) becomes a run of rows of one joined weight. */
+typedef struct AtlasRepackItem {
+    const int8_t *codes;
+    int64_t n_codes;
+    const void *outlier_vals;
+    const int64_t *outlier_idx;
+    int64_t n_outliers;
+    const void *scales;
+    int64_t n_rows, n_cols;
+    int64_t block_size;
+    uint8_t *tiles;
+    void *scales_tiled;
+    int32_t *outlier_row_ptr;
+    int32_t *outlier_chunk_ptr;
+    uint32_t *outlier_entries;
+    void *outlier_vals_sorted;
+    int64_t entry_base;
+} AtlasRepackItem;
+ATLAS_API int atlas_repack_many(int count, const AtlasRepackItem *items, void *stream);
+
 /* ---- quantized linear forward ----------------------------------------------------
  * Replaces QuantizedLinear.forward (integration/atlas_wrappers.py:30-74):
  * y[m][n] = sum_k x[m][k] * W[n][k] + bias[n], W being the dequantized weight
