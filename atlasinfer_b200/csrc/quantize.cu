@@ -326,37 +326,49 @@ __global__ void __launch_bounds__(QT_THREADS) quantize_kernel(QuantParams p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Fast variant for block sizes 32 / 64 / 128 / 256 (EPT = block_size / 8 values per thread, kept
-// in registers).  Same results as quantize_kernel above, bit for bit, with most of the IEEE
-// divisions and all of the fp64 work moved off the common path:
-//   * the second moment is accumulated in fp32 (error <= ~1e-6 relative); only if rounding the
-//     standard deviation to fp16 could go either way within 4e-6 is it recomputed in fp64;
-//   * |fp16(d / den)| > thr is decided from d * (1 / den) against the real number at which the
-//     rounded quotient crosses thr, with a 2^-21 guard band inside which the exact quotient is used;
-//   * fp16(x / scale) is taken from x * (1 / scale) when nudging the product by 2^-22 either way
-//     rounds to the same fp16 number, else from the exact quotient.
-// Codes are written once, uncompacted, to shared memory by the threads that computed the block
-// statistics; the compaction pass only moves bytes.
+// Fast variant for block sizes 32 / 64 / 128 / 256.  Same results as quantize_kernel above, bit for bit, at a quarter of
+// its instructions; issue slots, not HBM, are what a quantizer of this format runs out of.
+//
+// Four threads work on a block; thread t plays ATen's SIMD lanes 2t and 2t + 1, whose elements are neighbours, so the
+// values stay packed two to a register and most steps cost one instruction per pair.  What replaces the IEEE divisions
+// and the fp64 moment, and why the results are the same:
+//   * code.  x and the scale have 11-bit significands, so a quotient x / scale is never the midpoint of two fp16 numbers
+//     (scale times a midpoint's odd 12-bit significand needs more than 11 bits) and is more than 2^-23 away from one,
+//     relatively: |a 2^k - m b| >= 1 with m < 2^12, b < 2^11.  x * (1 / scale), two roundings to fp32, is within 2^-23:
+//     it rounds to the same fp16 number.  (Quotients below the fp16 normal range give code 0 either way.)  Adding 1536
+//     in fp16, where the spacing is 1, rounds half to even and leaves the two's-complement code in the low byte.
+//   * scale.  maxabs * (1 / 127) instead of maxabs / 127 by the same argument.
+//   * z test.  fp16(|d| / den) > thr iff |d| lies above T * den, T the midpoint between thr and the next fp16 number:
+//     12 by 11 bits, exact in fp32.  |d| is an fp16 number, so it is compared in fp16 with the largest one that does not
+//     exceed T * den.  A tie (only possible for subnormal thresholds) goes to the even neighbour: if thr is odd, |d| =
+//     T * den is an outlier too.
+//   * d = fp16(x - mean) is one fp16 subtraction.
+//   * standard deviation.  fp32 sum of squares minus the squared sum, if the mean takes less than a fifth of it away (worst
+//     case error 2.5e-6 relative, else a second pass about the mean); only if rounding it to fp16 could go either way
+//     within 4e-6 is it recomputed in fp64 (about 1 % of blocks).
+// The dense codes of a tile go to shared memory once; the compaction is driven by the output: a thread finds where its 16
+// bytes of the code stream start in the tile, takes them with one unaligned read, and squeezes out the places of outliers.
 struct FastConsts {
-    float t_lo, t_hi;  // guard band around the |z| decision boundary
-    float thr_f;
+    float T;         // |z| decision boundary
+    int tie_out;     // an exact tie is an outlier
 };
 
-template <int EPT>
-__global__ void __launch_bounds__(QT_THREADS, (EPT <= 16 ? 5 : 2)) quantize_fast_kernel(QuantParams p, FastConsts fc) {
-    constexpr int BS = EPT * 8;
+// Byte offset of element e's code in the dense tile: 16-byte pieces permuted so that the eight blocks a warp works on
+// fall on different banks.
+__device__ __forceinline__ int dense_byte(int e) { return e ^ (((e >> 7) & 7) << 4); }
+
+template <int BS>
+__global__ void __launch_bounds__(QT_THREADS, 5) quantize_fast_kernel(QuantParams p, FastConsts fc) {
+    constexpr int NP = BS / 8;                // pairs per thread
     constexpr int TILE_BLOCKS = QT_TILE / BS;
-    // Blocks are padded (16 bytes of values, 8 bytes of codes) so that the four blocks a warp works
-    // on at a time fall on different banks.
-    constexpr int XSTRIDE = BS * 2 + 16;  // bytes
-    constexpr int DSTRIDE = BS + 8;
+    // blocks are padded by 16 bytes so that the eight blocks a warp works on at a time fall on different banks
+    constexpr int XSTRIDE = BS * 2 + 16;      // bytes
     __shared__ __align__(16) uint8_t s_xb[TILE_BLOCKS * XSTRIDE];
-    __shared__ __align__(16) uint8_t s_dense[TILE_BLOCKS * DSTRIDE];
+    __shared__ __align__(16) uint8_t s_dense[QT_TILE + 128];
     auto xref = [&](int e) -> uint16_t & {
         return *reinterpret_cast<uint16_t *>(s_xb + (e / BS) * XSTRIDE + (e % BS) * 2);
     };
-    __shared__ __align__(16) uint8_t s_codes[QT_TILE + 32];
-    __shared__ uint32_t s_mask[QT_WORDS];
+    __shared__ uint32_t s_mask[QT_WORDS + 1];
     __shared__ uint32_t s_wordpre[QT_WORDS];
     __shared__ uint16_t s_scale[TILE_BLOCKS];
     __shared__ uint32_t s_warp_tot[QT_THREADS / 32];
@@ -369,6 +381,7 @@ __global__ void __launch_bounds__(QT_THREADS, (EPT <= 16 ? 5 : 2)) quantize_fast
     const int warp = tid >> 5;
     const uint16_t eps_h = f2h_bits(1e-6f);
     const float eps_f = h2f_bits(eps_h);
+    if (tid == 0) s_mask[QT_WORDS] = 0u;
 
     for (;;) {
         __syncthreads();  // previous tile's shared state is no longer read
@@ -384,8 +397,9 @@ __global__ void __launch_bounds__(QT_THREADS, (EPT <= 16 ? 5 : 2)) quantize_fast
         // ---- stage the tile (zero padding included) -------------------------------
         if (p.in_aligned) {
             const uint4 *src = reinterpret_cast<const uint4 *>(p.x + tile_base);
-            for (int v = tid; v < QT_TILE / 8; v += QT_THREADS) {
-                int e0 = v * 8;
+#pragma unroll
+            for (int i = 0; i < QT_TILE / 8 / QT_THREADS; ++i) {
+                const int v = tid + i * QT_THREADS, e0 = v * 8;
                 if (e0 + 8 <= tile_real) {
                     *reinterpret_cast<uint4 *>(s_xb + (e0 / BS) * XSTRIDE + (e0 % BS) * 2) = __ldg(src + v);
                 } else if (e0 < tile_elems) {
@@ -396,115 +410,135 @@ __global__ void __launch_bounds__(QT_THREADS, (EPT <= 16 ? 5 : 2)) quantize_fast
             for (int e = tid; e < tile_elems; e += QT_THREADS)
                 xref(e) = (e < tile_real) ? p.x[tile_base + e] : (uint16_t)0;
         }
-        for (int w = tid; w < QT_WORDS; w += QT_THREADS) s_mask[w] = 0u;
+        s_mask[tid] = 0u;   // QT_WORDS == QT_THREADS
         __syncthreads();
 
-        // ---- phase A: statistics and codes of whole blocks, 8 threads per block ----------
+        // ---- statistics and codes of whole blocks, 4 threads per block ----------
         {
-            const int l = tid & 7;    // ATen SIMD lane this thread plays
-            const int grp = tid >> 3;
-            const unsigned gmask = 0xffu << (lane & 24);
-            for (int b = grp; b < tile_blocks; b += QT_THREADS / 8) {
-                const uint16_t *xb = reinterpret_cast<const uint16_t *>(s_xb + b * XSTRIDE);
-                float f[EPT];
+            const int t = tid & 3;
+            const unsigned gmask = 0xfu << (lane & 28);
+            for (int b = tid >> 2; b < tile_blocks; b += QT_THREADS / 4) {
+                const uint32_t *xb = reinterpret_cast<const uint32_t *>(s_xb + b * XSTRIDE) + t;
+                // (read from shared memory again in every pass: keeping 32 floats costs the fifth CTA of an SM)
+                auto pair = [&](int j) { return __half22float2(*reinterpret_cast<const __half2 *>(xb + j * 4)); };
+                // fp32 sum in ATen's order, and the sum of squares
+                float lo4[4] = {0.f, 0.f, 0.f, 0.f}, hi4[4] = {0.f, 0.f, 0.f, 0.f}, sq = 0.f, sq_hi = 0.f;
 #pragma unroll
-                for (int j = 0; j < EPT; ++j) f[j] = h2f_bits(xb[j * 8 + l]);
-                // fp32 sum in ATen's order
-                float a4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int j = 0; j < EPT; ++j) a4[j & 3] = __fadd_rn(a4[j & 3], f[j]);
-                const float lane_sum = __fadd_rn(__fadd_rn(__fadd_rn(a4[0], a4[1]), a4[2]), a4[3]);
+                for (int j = 0; j < NP; ++j) {
+                    const float2 f = pair(j);
+                    lo4[j & 3] = __fadd_rn(lo4[j & 3], f.x);
+                    hi4[j & 3] = __fadd_rn(hi4[j & 3], f.y);
+                    sq = fmaf(f.x, f.x, sq);
+                    sq_hi = fmaf(f.y, f.y, sq_hi);
+                }
+                asm volatile("" ::: "memory");
+                const float lo_sum = __fadd_rn(__fadd_rn(__fadd_rn(lo4[0], lo4[1]), lo4[2]), lo4[3]);
+                const float hi_sum = __fadd_rn(__fadd_rn(__fadd_rn(hi4[0], hi4[1]), hi4[2]), hi4[3]);
                 float fin = 0.f;
 #pragma unroll
-                for (int s = 0; s < 8; ++s) fin = __fadd_rn(fin, __shfl_sync(gmask, lane_sum, s, 8));
-                const float mean32 = __fdiv_rn(fin, (float)BS);
-                const float mean_f = h2f_bits(f2h_bits(mean32));
-                // second moment: fp32 first
-                // (about mean32, with the first moment about it taken out again, so that the rounding
-                // of mean32 itself only enters to second order)
-                float m2f = 0.f, r1 = 0.f;
-#pragma unroll
-                for (int j = 0; j < EPT; ++j) {
-                    const float d = f[j] - mean32;
-                    r1 += d;
-                    m2f = fmaf(d, d, m2f);
+                for (int s = 0; s < 4; ++s) {
+                    fin = __fadd_rn(fin, __shfl_sync(gmask, lo_sum, s, 4));
+                    fin = __fadd_rn(fin, __shfl_sync(gmask, hi_sum, s, 4));
                 }
-#pragma unroll
-                for (int o = 1; o < 8; o <<= 1) {
-                    m2f += __shfl_xor_sync(gmask, m2f, o, 8);
-                    r1 += __shfl_xor_sync(gmask, r1, o, 8);
-                }
-                m2f = fmaxf(fmaf(-r1, r1 * (1.f / (float)BS), m2f), 0.f);
-                const float std32 = __fsqrt_rn(__fdiv_rn(m2f, (float)(BS - 1)));
-                uint16_t std_h = f2h_bits(std32 * (1.f - 4e-6f));
-                if (std_h != f2h_bits(std32 * (1.f + 4e-6f))) {
-                    // the fp16 rounding is within reach of the fp32 error: redo it in fp64 (group-uniform)
-                    double dsum = 0.0;
-#pragma unroll
-                    for (int j = 0; j < EPT; ++j) dsum += (double)f[j];
-#pragma unroll
-                    for (int o = 1; o < 8; o <<= 1) dsum += __shfl_xor_sync(gmask, dsum, o, 8);
-                    const double mean_d = dsum / (double)BS;
-                    double m2 = 0.0;
-#pragma unroll
-                    for (int j = 0; j < EPT; ++j) {
-                        const double d = (double)f[j] - mean_d;
-                        m2 = fma(d, d, m2);
+                const float mean32 = fin * (1.f / (float)BS);   // a power of two: exact
+                const uint16_t mean_h = f2h_bits(mean32);
+                sq += sq_hi;
+                sq += __shfl_xor_sync(gmask, sq, 1, 4);
+                sq += __shfl_xor_sync(gmask, sq, 2, 4);
+                float m2f = fmaf(-fin, mean32, sq);
+                if (!(sq <= 1.25f * m2f)) {   // (the same decision in all four threads)
+                    // about mean32, with the first moment about it taken out again, so that the rounding of mean32
+                    // itself only enters to second order
+                    float r1 = 0.f;
+                    m2f = 0.f;
+#pragma unroll 1
+                    for (int j = 0; j < NP; ++j) {
+                        const float2 f = pair(j);
+                        const float d0 = f.x - mean32, d1 = f.y - mean32;
+                        r1 += d0 + d1;
+                        m2f = fmaf(d0, d0, fmaf(d1, d1, m2f));
                     }
 #pragma unroll
-                    for (int o = 1; o < 8; o <<= 1) m2 += __shfl_xor_sync(gmask, m2, o, 8);
+                    for (int o = 1; o < 4; o <<= 1) {
+                        m2f += __shfl_xor_sync(gmask, m2f, o, 4);
+                        r1 += __shfl_xor_sync(gmask, r1, o, 4);
+                    }
+                    m2f = fmaxf(fmaf(-r1, r1 * (1.f / (float)BS), m2f), 0.f);
+                }
+                float std32;
+                asm("sqrt.approx.f32 %0, %1;" : "=f"(std32) : "f"(m2f * (1.f / (float)(BS - 1))));
+                uint16_t std_h = f2h_bits(std32 * (1.f - 4e-6f));
+                if (std_h != f2h_bits(std32 * (1.f + 4e-6f))) {
+                    // the fp16 rounding is within reach of the fp32 error: redo it in fp64
+                    double dsum = 0.0;
+#pragma unroll 1
+                    for (int j = 0; j < NP; ++j) { const float2 f = pair(j); dsum += (double)f.x + (double)f.y; }
+#pragma unroll
+                    for (int o = 1; o < 4; o <<= 1) dsum += __shfl_xor_sync(gmask, dsum, o, 4);
+                    const double mean_d = dsum / (double)BS;
+                    double m2 = 0.0;
+#pragma unroll 1
+                    for (int j = 0; j < NP; ++j) {
+                        const float2 f = pair(j);
+                        const double d0 = (double)f.x - mean_d, d1 = (double)f.y - mean_d;
+                        m2 = fma(d0, d0, fma(d1, d1, m2));
+                    }
+#pragma unroll
+                    for (int o = 1; o < 4; o <<= 1) m2 += __shfl_xor_sync(gmask, m2, o, 4);
                     std_h = f2h_bits(__double2float_rn(sqrt(m2 / (double)(BS - 1))));
                 }
                 const float den_f = h2f_bits(f2h_bits(__fadd_rn(h2f_bits(std_h), eps_f)));
-                // |d| / den against the threshold = |d| against threshold * den: the block's two bounds are one
-                // rounding away from exact, well inside the guard band they delimit
-                const float lo_b = fc.t_lo * den_f, hi_b = fc.t_hi * den_f;
-                // z test, outlier mask, absmax of the rest
-                unsigned int omask = 0;   // bit j: element j of this thread is an outlier
-                unsigned int maxabs = 0;  // fp32 bits of the largest |x| kept (bit patterns order like the values)
+                // the largest |d| that is not an outlier
+                const float bound = fc.T * den_f;
+                uint16_t cut = __half_as_ushort(__float2half_rd(bound));
+                if (fc.tie_out && h2f_bits(cut) == bound) --cut;
+                const __half2 cut2 = __half2half2(__ushort_as_half(cut)), mean2 = __half2half2(__ushort_as_half(mean_h));
+                // z test, outlier mask (low half: even elements, high half: odd ones), absmax of the rest
+                constexpr int NM = (NP + 15) / 16;
+                uint32_t omask[NM], maxabs = 0u;
 #pragma unroll
-                for (int j = 0; j < EPT; ++j) {
-                    const float d = h2f_bits(f2h_bits(__fsub_rn(f[j], mean_f)));
-                    const float a = fabsf(d);
-                    bool is_out = a > hi_b;
-                    if (!is_out && a >= lo_b) {   // inside the guard band: the exact rounded quotient decides
-                        const float z = h2f_bits(f2h_bits(__fdiv_rn(d, den_f)));
-                        is_out = fabsf(z) > fc.thr_f;
-                    }
-                    if (is_out) omask |= 1u << j;
-                    else maxabs = max(maxabs, __float_as_uint(f[j]) & 0x7fffffffu);
-                }
-                int cnt = __popc(omask);
+                for (int i = 0; i < NM; ++i) omask[i] = 0u;
 #pragma unroll
-                for (int o = 1; o < 8; o <<= 1) {
-                    cnt += __shfl_xor_sync(gmask, cnt, o, 8);
-                    maxabs = max(maxabs, __shfl_xor_sync(gmask, maxabs, o, 8));
+                for (int j = 0; j < NP; ++j) {
+                    const uint32_t x2 = xb[j * 4];
+                    const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&x2), mean2);
+                    const uint32_t out = __hgt2_mask(__habs2(d), cut2);
+                    omask[j >> 4] |= out & (0x00010001u << (j & 15));
+                    maxabs = __vmaxu2(maxabs, x2 & 0x7fff7fffu & ~out);   // fp16 magnitude bits order like the values
                 }
+                asm volatile("" ::: "memory");
+                int cnt = 0;
+#pragma unroll
+                for (int i = 0; i < NM; ++i) cnt += __popc(omask[i]);
+                const bool any_out = cnt != 0;
+#pragma unroll
+                for (int o = 1; o < 4; o <<= 1) {
+                    cnt += __shfl_xor_sync(gmask, cnt, o, 4);
+                    maxabs = __vmaxu2(maxabs, __shfl_xor_sync(gmask, maxabs, o, 4));
+                }
+                maxabs = max(maxabs & 0xffffu, maxabs >> 16);
                 uint16_t sc = 0x3c00u;  // 1.0 when the block has no non-outliers
-                if (cnt < BS) {
-                    sc = f2h_bits(__fdiv_rn(__uint_as_float(maxabs), 127.0f));
-                    if (h2f_bits(sc) < eps_f) sc = eps_h;
-                }
-                if (l == 0) s_scale[b] = sc;
-                const float sc_f = h2f_bits(sc);
-                const float rsc = __frcp_rn(sc_f);
-                uint8_t *db = s_dense + b * DSTRIDE + l;
+                if (cnt < BS) sc = max(f2h_bits(h2f_bits((uint16_t)maxabs) * (1.0f / 127.0f)), eps_h);
+                if (t == 0) s_scale[b] = sc;
+                const float rsc = __frcp_rn(h2f_bits(sc));
+                uint8_t *db = s_dense;
+                const int e0 = b * BS + 2 * t;
+                const __half2 lim = __float2half2_rn(127.f), nlim = __float2half2_rn(-127.f), magic = __float2half2_rn(1536.f);
 #pragma unroll
-                for (int j = 0; j < EPT; ++j) {
-                    const float v = f[j] * rsc;   // within 2^-22 of x / scale
-                    uint16_t qh = f2h_bits(v);
-                    // fp16 keeps 10 of the 23 mantissa bits: v rounds the other way only if its 13 low bits are within a
-                    // few units of the midpoint 0x1000 (results below the fp16 normal range give code 0 either way)
-                    if (((__float_as_uint(v) & 0x1fffu) - (0x1000u - 8u)) <= 16u) qh = f2h_bits(__fdiv_rn(f[j], sc_f));
-                    int r = __half2int_rn(__ushort_as_half(qh));   // half to even, as torch.round
-                    r = max(-127, min(127, r));
-                    db[j * 8] = (uint8_t)r;
+                for (int j = 0; j < NP; ++j) {
+                    const float2 f = pair(j);
+                    __half2 q = __floats2half2_rn(f.x * rsc, f.y * rsc);
+                    q = __hmax2(__hmin2(q, lim), nlim);
+                    q = __hadd2(q, magic);
+                    const uint32_t bits = *reinterpret_cast<uint32_t *>(&q);
+                    *reinterpret_cast<uint16_t *>(db + dense_byte(e0 + j * 8)) = (uint16_t)__byte_perm(bits, 0u, 0x4420);
                 }
-                if (omask) {
+                if (any_out) {
 #pragma unroll
-                    for (int j = 0; j < EPT; ++j)
-                        if ((omask >> j) & 1u) {
-                            const int pos = b * BS + j * 8 + l;
+                    for (int i = 0; i < NM; ++i)
+                        for (uint32_t m = omask[i]; m; m &= m - 1) {
+                            const int bit = __ffs(m) - 1;
+                            const int pos = e0 + ((bit & 15) + i * 16) * 8 + (bit >> 4);
                             atomicOr(&s_mask[pos >> 5], 1u << (pos & 31));
                         }
                 }
@@ -574,22 +608,6 @@ __global__ void __launch_bounds__(QT_THREADS, (EPT <= 16 ? 5 : 2)) quantize_fast
                     p.counts[1] = total_out;
                 }
             }
-        } else {
-            // ---- meanwhile, warps 1..7 compact the codes in shared memory (needs no prefix) ----------
-            for (int i = (tid - 32) * 4; i < tile_elems; i += (QT_THREADS - 32) * 4) {
-                const uint32_t word = s_mask[i >> 5];
-                const uint32_t m4 = (word >> (i & 31)) & 0xfu;
-                const int before = (int)s_wordpre[i >> 5] + __popc(word & ((1u << (i & 31)) - 1u));
-                const uint32_t c4 = *reinterpret_cast<const uint32_t *>(s_dense + (i / BS) * DSTRIDE + (i % BS));
-                int dst = i - before;
-                if (m4 == 0u && (dst & 3) == 0) {
-                    *reinterpret_cast<uint32_t *>(s_codes + dst) = c4;
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (!((m4 >> e) & 1u)) s_codes[dst++] = (uint8_t)(c4 >> (8 * e));
-                }
-            }
         }
         __syncthreads();
 
@@ -611,29 +629,70 @@ __global__ void __launch_bounds__(QT_THREADS, (EPT <= 16 ? 5 : 2)) quantize_fast
             }
         }
 
-        // ---- copy the compacted codes out: 16-byte stores to aligned global addresses, the shared-memory side is
-        // read at whatever byte offset the tile's start in the code stream leaves (five words and a funnel shift)
+        // ---- the compacted codes, 16 bytes to an aligned global address per thread and step ------------------------
         {
             const int total = tile_elems - s_tile_total;  // code bytes of this tile
             const int end = shift + total;
             int8_t *gdst = p.codes + (code_base - shift);  // 16-byte aligned when out_aligned
             const int nchunks = (end + 15) >> 4;
-            const uint32_t *s32 = reinterpret_cast<const uint32_t *>(s_codes);
+            const uint32_t *s32 = reinterpret_cast<const uint32_t *>(s_dense);
             for (int c = tid; c < nchunks; c += QT_THREADS) {
-                const int lo = c << 4;
-                if (p.out_aligned && lo >= shift && lo + 16 <= end) {
-                    const int o = lo - shift;
-                    const int wi = o >> 2, r = (o & 3) * 8;
-                    const uint32_t w0 = s32[wi], w1 = s32[wi + 1], w2 = s32[wi + 2], w3 = s32[wi + 3], w4 = s32[wi + 4];
-                    uint4 v;
-                    v.x = __funnelshift_r(w0, w1, r);
-                    v.y = __funnelshift_r(w1, w2, r);
-                    v.z = __funnelshift_r(w2, w3, r);
-                    v.w = __funnelshift_r(w3, w4, r);
-                    *reinterpret_cast<uint4 *>(gdst + lo) = v;
+                const int lo = c << 4, a = max(lo, shift), z = min(lo + 16, end);
+                const int o0 = a - shift;                    // first code of the piece, counted in the tile
+                int w = o0 >> 5;                             // the mask word it lies in
+                while (w < QT_WORDS - 1 && (w + 1) * 32 - (int)s_wordpre[w + 1] <= o0) ++w;
+                const int skip = o0 - (w * 32 - (int)s_wordpre[w]);   // codes of that word in front of it
+                const uint32_t word = s_mask[w];
+                int in_word = skip;
+                if (word) {                                  // position of code number `skip` among the word's codes
+                    for (int i = 0; i < 32; ++i) {
+                        const int next = skip + __popc(word & (0xffffffffu >> (31 - min(in_word, 31))));
+                        if (next == in_word) break;
+                        in_word = next;
+                    }
+                }
+                const int pos = w * 32 + in_word;
+                // 20 dense codes from there and their outlier bits
+                uint32_t m = __funnelshift_r(s_mask[pos >> 5], s_mask[min((pos >> 5) + 1, QT_WORDS)], pos & 31) & 0xfffffu;
+                uint32_t v[5];
+                {
+                    const int wi = pos >> 2, r = (pos & 3) * 8;
+                    uint32_t raw[6];
+#pragma unroll
+                    for (int i = 0; i < 6; ++i) raw[i] = s32[(wi + i) ^ ((((wi + i) >> 5) & 7) << 2)];
+#pragma unroll
+                    for (int i = 0; i < 5; ++i) v[i] = __funnelshift_r(raw[i], raw[i + 1], r);
+                }
+                if (__popc(m) <= 4) {
+                    while (m & 0xffffu) {                    // squeeze out the first outlier's place
+                        const int j = __ffs(m) - 1, jw = j >> 2;
+                        const uint32_t low = (1u << (8 * (j & 3))) - 1u;
+#pragma unroll
+                        for (int i = 0; i < 5; ++i) {
+                            const uint32_t down = __funnelshift_r(v[i], i < 4 ? v[i < 4 ? i + 1 : 4] : 0u, 8);
+                            v[i] = i < jw ? v[i] : (i == jw ? ((v[i] & low) | (down & ~low)) : down);
+                        }
+                        m = (m >> 1) & ~((1u << j) - 1u);
+                    }
+                } else {                                     // dense outliers: code by code
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[i] = 0u;
+                    int q = pos;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        if (a + i < z) {
+                            while ((s_mask[q >> 5] >> (q & 31)) & 1u) ++q;
+                            v[i >> 2] |= (uint32_t)s_dense[dense_byte(q)] << (8 * (i & 3));
+                            ++q;
+                        }
+                    }
+                }
+                if (p.out_aligned && z - a == 16) {
+                    *reinterpret_cast<uint4 *>(gdst + lo) = make_uint4(v[0], v[1], v[2], v[3]);
                 } else {
-                    const int a = max(lo, shift), z = min(lo + 16, end);
-                    for (int q = a; q < z; ++q) gdst[q] = (int8_t)s_codes[q - shift];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (a + i < z) gdst[a + i] = (int8_t)(v[i >> 2] >> (8 * (i & 3)));
                 }
             }
             const int64_t block0 = tile_base / BS;
@@ -643,20 +702,18 @@ __global__ void __launch_bounds__(QT_THREADS, (EPT <= 16 ? 5 : 2)) quantize_fast
 }
 
 // |fp16(q)| > thr_h  <=>  |q| beyond T, the midpoint between thr_h and the next fp16 number above it
-// (a tie goes to the even neighbour).  Returns T; the kernel uses the exact quotient inside a guard band.
+// (a tie goes to the even neighbour).
 FastConsts make_fast_consts(uint16_t thr_h) {
     FastConsts fc;
     const float thr = __half2float(__ushort_as_half(thr_h));
-    fc.thr_f = thr;
-    float T;
-    if ((thr_h & 0x7fffu) > 0x7c00u) T = INFINITY;            // NaN threshold: nothing compares greater
-    else if (thr_h == 0x7c00u) T = INFINITY;                   // +inf
-    else if (thr_h & 0x8000u) T = -1.f;                        // negative threshold: every |z| is greater
-    else if (thr_h == 0x7bffu) T = 65520.f;                    // next above the largest finite is inf
-    else T = 0.5f * (thr + __half2float(__ushort_as_half((uint16_t)(thr_h + 1))));
-    if (T == INFINITY) { fc.t_lo = INFINITY; fc.t_hi = INFINITY; }
-    else if (T < 0.f) { fc.t_lo = -2.f; fc.t_hi = -1.f; }
-    else { fc.t_lo = T * (1.f - 4.8e-7f); fc.t_hi = T * (1.f + 4.8e-7f); }
+    fc.tie_out = 0;
+    if ((thr_h & 0x7fffu) > 0x7c00u) fc.T = INFINITY;          // NaN threshold: nothing compares greater
+    else if (thr_h == 0x7c00u) fc.T = INFINITY;                 // +inf
+    else if (thr_h > 0x8000u) fc.T = -1.f;                      // negative: every |z| is greater
+    else if (thr_h == 0x8000u) fc.T = 0x1p-25f;                 // as +0
+    else if (thr_h == 0x7bffu) fc.T = 65520.f;                  // next above the largest finite is inf
+    else fc.T = 0.5f * (thr + __half2float(__ushort_as_half((uint16_t)(thr_h + 1))));
+    if (!(thr_h & 0x8000u) && fc.T != INFINITY) fc.tie_out = thr_h & 1;
     return fc;
 }
 
@@ -751,16 +808,16 @@ int atlas_quantize(const void *w, int64_t numel, int block_size, double z_thresh
     rc = device_info(di);
     if (rc) return rc;
     const bool fast = block_size == 32 || block_size == 64 || block_size == 128 || block_size == 256;
-    const int per_sm = fast ? (block_size == 256 ? 2 : 5) : di.quant_ctas_per_sm;   // resident CTAs of the fast kernels
+    const int per_sm = fast ? 5 : di.quant_ctas_per_sm;   // resident CTAs of the fast kernels
     const int64_t max_ctas = (int64_t)di.sms * per_sm;
     const int grid = (int)(p.num_tiles < max_ctas ? p.num_tiles : max_ctas);
     if (fast) {
         const FastConsts fc = make_fast_consts(p.thr_h);
         switch (block_size) {
-            case 32: quantize_fast_kernel<4><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
-            case 64: quantize_fast_kernel<8><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
-            case 128: quantize_fast_kernel<16><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
-            default: quantize_fast_kernel<32><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
+            case 32: quantize_fast_kernel<32><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
+            case 64: quantize_fast_kernel<64><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
+            case 128: quantize_fast_kernel<128><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
+            default: quantize_fast_kernel<256><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
         }
         return check_cuda(cudaGetLastError(), "quantize_fast_kernel launch");
     }

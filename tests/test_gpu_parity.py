@@ -284,3 +284,20 @@ def test_apply_to_tiny_opt_model_and_generate(cuda_device):
         ref_logits = ref_model(ids).logits.float()
     assert out.shape == (1, 28)
     assert rel_max_err(logits, ref_logits) < 2e-2
+
+
+# the fast quantizer's own branches: a mean that takes the sum of squares away (second pass), subnormal scales (clamp),
+# thresholds whose ties decide (odd subnormal), zero and negative ones, the largest finite one, pieces with more than
+# four outliers, tiles that end inside a block
+@pytest.mark.parametrize("bs", [32, 64, 128, 256])
+@pytest.mark.parametrize("offset,sigma,thr", [(1.0, 0.02, 3.0), (-300.0, 0.5, 2.0), (0.0, 2e-6, 3.0), (0.0, 1e-7, 1.0),
+                                              (0.0, 0.02, 0.0), (0.0, 0.02, 3 * 2.0 ** -24), (0.0, 0.02, 2.0 ** -23),
+                                              (0.0, 0.02, -0.5), (0.0, 0.02, 65504.0), (0.01, 0.02, 1.5)])
+def test_quantize_fast_kernel_branches(bs, offset, sigma, thr, cuda_device):
+    gen = torch.Generator().manual_seed(bs)
+    for n in (8192 - 1, 8192 + 1, 3 * 8192 + bs + 5):
+        w = (torch.randn(n, generator=gen) * sigma + offset).half()
+        w[::97] = w[0]                       # equal values: exact ties in the z test
+        w[n // 2:n // 2 + 2 * bs] = offset   # constant blocks
+        q = ab.quantize_tensor(w.to(cuda_device), bs, thr)
+        assert_streams_equal(q, O.quantize(w, bs, thr), what=f"n {n} bs {bs} offset {offset} sigma {sigma} thr {thr}: ")
