@@ -4,7 +4,7 @@
 // Replaces dequantize_tensor (atlasinfer_core/quant/adaptive_quantizer.py:156-251).
 // The reference keeps a running offset into the code stream and, per block,
 // masks the whole outlier index list (:194-196, O(blocks x outliers)).  Here the
-// sorted outlier index list is searched once per span of 8192 elements: the
+// sorted outlier index list is searched once per span of 16384 elements: the
 // number of outliers before the span both locates the span's outliers and
 // gives the span's offset into the compacted code stream (position minus
 // outliers before it), so every span is independent.
@@ -19,9 +19,9 @@ namespace atlas {
 namespace {
 
 constexpr int DQ_THREADS = 256;
-constexpr int DQ_SPAN = 8192;                 // padded elements per CTA
-constexpr int DQ_WORDS = DQ_SPAN / 32;        // outlier-mask words: one per thread
-static_assert(DQ_WORDS == DQ_THREADS, "one mask word per thread");
+constexpr int DQ_SPAN = 16384;                // padded elements per CTA
+constexpr int DQ_WORDS = DQ_SPAN / 32;        // outlier-mask words: two per thread
+static_assert(DQ_WORDS == 2 * DQ_THREADS, "two mask words per thread");
 constexpr int DQ_MAX_REPACK = 8;              // tensors one repack launch takes
 constexpr int RP_STRIP_CAP = 2560;            // outliers of a strip kept in shared memory (16 x 4096 weights: 200 at 0.3 %)
 constexpr int RP_SCALE_KB = 16;               // scale blocks per CTA of the scale transposition (one 32-byte sector a row)
@@ -41,8 +41,8 @@ __device__ __forceinline__ int64_t warp_lower_bound(const int64_t *idx, int64_t 
 }
 
 struct Span {
-    uint32_t mask[DQ_WORDS];                  // bit p: position p of the span is an outlier
-    uint32_t before[DQ_WORDS];                // outliers of the span before the word
+    __align__(16) uint32_t mask[DQ_WORDS];                  // bit p: position p of the span is an outlier
+    __align__(16) uint32_t before[DQ_WORDS];                // outliers of the span before the word
     uint32_t warp_total[DQ_THREADS / 32];
     int64_t lo, hi;                           // the span's outliers in the outlier streams
     __align__(16) uint8_t codes[DQ_SPAN + 48];
@@ -54,7 +54,7 @@ struct Span {
 __device__ __forceinline__ void stage_span(Span &s, const int8_t *codes, int64_t n_codes, const int64_t *oidx,
                                            int64_t n_out, int64_t span0, int64_t span1) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    s.mask[tid] = 0u;
+    *reinterpret_cast<uint2 *>(s.mask + 2 * tid) = make_uint2(0u, 0u);
     if (warp < 2) {
         const int64_t r = warp_lower_bound(oidx, n_out, warp == 0 ? span0 : span1, lane);
         if (lane == 0) (warp == 0 ? s.lo : s.hi) = r;
@@ -84,7 +84,8 @@ __device__ __forceinline__ void stage_span(Span &s, const int8_t *codes, int64_t
         *reinterpret_cast<uint4 *>(s.codes + c * 16) = v;
     }
     __syncthreads();
-    const uint32_t own = __popc(s.mask[tid]);
+    const uint2 words = *reinterpret_cast<const uint2 *>(s.mask + 2 * tid);
+    const uint32_t own = __popc(words.x) + __popc(words.y);
     uint32_t inc = own;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -95,7 +96,7 @@ __device__ __forceinline__ void stage_span(Span &s, const int8_t *codes, int64_t
     __syncthreads();
     uint32_t base = 0;
     for (int w = 0; w < warp; ++w) base += s.warp_total[w];
-    s.before[tid] = base + inc - own;
+    *reinterpret_cast<uint2 *>(s.before + 2 * tid) = make_uint2(base + inc - own, base + inc - __popc(words.y));
     __syncthreads();
 }
 
@@ -265,7 +266,7 @@ __device__ __forceinline__ void write_strip(const RepackTensor &t, int64_t strip
 }
 
 // One launch expands up to DQ_MAX_REPACK tensors; a CTA does one of three jobs: the outlier lists of a strip (first in
-// the grid: the longest chain of dependent loads), a 128-row x 16-block piece of the scale transposition, or 8192
+// the grid: the longest chain of dependent loads), a 128-row x 16-block piece of the scale transposition, or 16384
 // positions of the code tiles, 16 codes (one unit of the layout; n_cols is a multiple of 64, so a unit never straddles
 // rows) per thread and step.  Rows beyond n_rows in the last 128-row tile get code 0 and scale 0.
 __global__ void __launch_bounds__(DQ_THREADS) repack_kernel(const __grid_constant__ RepackParams p) {
