@@ -6,6 +6,8 @@ sm_100a GPU is usable, calls raise -- there is no CPU or PyTorch fallback.
 from __future__ import annotations
 
 import ctypes
+import glob
+import importlib.util
 import os
 from typing import Optional
 
@@ -123,6 +125,26 @@ def load() -> ctypes.CDLL:
     L.atlas_qlinear_gemm.argtypes = lin + [vp, sz, vp, vp]
     _lib = L
     return L
+
+
+_native = None
+
+
+def native():
+    """The host-path module (``csrc/native.cpp``), loaded on first use; raises with build instructions if it is missing."""
+    global _native
+    if _native is None:
+        load()
+        path = [p for p in glob.glob(os.path.join(_PKG, "lib", "_atlas_native.*.so"))]
+        if not path:
+            raise RuntimeError(
+                "atlasinfer_b200: the module _atlas_native is missing. Build it with "
+                "`python -m atlasinfer_b200.build`; there is no fallback path.")
+        spec = importlib.util.spec_from_file_location("_atlas_native", path[0])
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _native = mod
+    return _native
 
 
 def check(status: int, what: str) -> None:

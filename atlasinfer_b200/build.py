@@ -3,7 +3,9 @@
     python -m atlasinfer_b200.build [--force] [--verbose]
 
 The library is compiled from ``csrc/*.cu`` against ``include/atlas_b200.h`` and
-written to ``atlasinfer_b200/lib/``.  nvcc cross-compiles without a GPU.
+written to ``atlasinfer_b200/lib/``, and beside it the module ``csrc/native.cpp``
+(the host path of the Python surface, which calls the library).  nvcc
+cross-compiles without a GPU.
 """
 from __future__ import annotations
 
@@ -11,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
@@ -41,15 +44,57 @@ def _inputs():
     return files, deps
 
 
-def is_stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+NATIVE_NAME = "_atlas_native"
+NATIVE_SRC = os.path.join(CSRC, "native.cpp")
+NATIVE_PATH = os.path.join(LIB_DIR, NATIVE_NAME + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def _stale(target: str, sources) -> bool:
+    if not os.path.exists(target):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    return any(os.path.getmtime(d) > t for d in _inputs()[1])
+    t = os.path.getmtime(target)
+    return any(os.path.getmtime(d) > t for d in sources)
+
+
+def build_native(force: bool = False, verbose: bool = False) -> str:
+    """Compile the host path (``csrc/native.cpp``, against torch's headers) if it is missing or old; return its path."""
+    header = os.path.join(ROOT, "include", "atlas_b200.h")
+    if not force and not _stale(NATIVE_PATH, [NATIVE_SRC, header]):
+        return NATIVE_PATH
+    import torch
+    from torch.utils import cpp_extension
+
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    dirs = [*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"],
+            os.path.join(ROOT, "include")]
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else (shutil.which("g++") or "c++")
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-DTORCH_EXTENSION_NAME={NATIVE_NAME}",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{d}" for d in dirs), NATIVE_SRC,
+           "-o", NATIVE_PATH, f"-L{LIB_DIR}", "-l:libatlas_b200.so", "-Wl,-rpath,$ORIGIN", f"-L{torch_lib}",
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+    if verbose:
+        print(res.stdout + res.stderr)
+    return NATIVE_PATH
+
+
+def is_stale() -> bool:
+    return _stale(LIB_PATH, _inputs()[1])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if it is missing or older than its sources; return its path."""
+    """Compile what is missing or older than its sources: the C-ABI library and the host path on top of it.
+
+    Returns the path of the C-ABI library."""
+    build_library(force, verbose)
+    build_native(force, verbose)
+    return LIB_PATH
+
+
+def build_library(force: bool = False, verbose: bool = False) -> str:
     if not force and not is_stale():
         return LIB_PATH
     os.makedirs(LIB_DIR, exist_ok=True)

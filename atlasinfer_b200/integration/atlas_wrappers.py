@@ -26,6 +26,7 @@ from ..quant.adaptive_quantizer import QuantizedTensor
 # column-parallel linear with the fused gather runs on and can be asked for with force="stream".
 GEMV_MAX_ROWS = 16
 STREAM_MAX_ROWS = 32
+_ANY_ROWS = 1 << 62
 
 _VERBOSE = os.environ.get("ATLAS_VERBOSE", "0") not in ("", "0")
 
@@ -50,11 +51,13 @@ _status_words = {}
 
 def status_word(dev: torch.device) -> torch.Tensor:
     """The device int32 kernels set non-zero when a bounded wait ran out (one per device)."""
-    key = (dev.type, dev.index if dev.index is not None else torch.cuda.current_device())
-    t = _status_words.get(key)
+    index = dev.index
+    if index is None:
+        index = torch.cuda.current_device()
+    t = _status_words.get(index)
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=dev)
-        _status_words[key] = t
+        _status_words[index] = t
     return t
 
 
@@ -167,14 +170,24 @@ def quantized_linear_forward(x: torch.Tensor, layout: KernelLayout, bias: Option
 
     ``force``: "gemv" (per-strip streaming kernel), "gemm" (tcgen05 kernel) or "stream" (persistent streaming
     kernel, one pass for up to 32 rows); default: "gemv" up to 16 rows of x, "gemm" above."""
+    if x.dtype is not torch.float16 and x.dtype is not torch.bfloat16:
+        raise RuntimeError(f"QuantizedLinear expects fp16 (or bf16) activations, got {x.dtype}")
+    if force is None:
+        gemv_rows = GEMV_MAX_ROWS
+    elif force == "stream":
+        return _stream_forward(x, layout, bias)
+    elif force in ("gemv", "gemm"):
+        gemv_rows = _ANY_ROWS if force == "gemv" else 0
+    else:
+        raise ValueError(f"force={force!r}")
+    return _capi.native().linear(x, layout.tiles, layout.scales_tiled, layout.chunk_ptr, layout.entries, layout.vals_sorted,
+                                 layout.n_rows, layout.n_cols, layout.block_size, bias, status_word(x.device), gemv_rows)
+
+
+def _stream_forward(x: torch.Tensor, layout: KernelLayout, bias: Optional[torch.Tensor]) -> torch.Tensor:
+    """``quantized_linear_forward`` on the persistent streaming kernel."""
     L = _capi.load()
     dev = x.device
-    if x.dtype == torch.float16:
-        dtype = _capi.DTYPE_F16
-    elif x.dtype == torch.bfloat16:
-        dtype = _capi.DTYPE_BF16
-    else:
-        raise RuntimeError(f"QuantizedLinear expects fp16 (or bf16) activations, got {x.dtype}")
     n, k = layout.n_rows, layout.n_cols
     if x.shape[-1] != k:
         raise RuntimeError(f"QuantizedLinear: input has {x.shape[-1]} features, weight expects {k}")
@@ -184,33 +197,16 @@ def quantized_linear_forward(x: torch.Tensor, layout: KernelLayout, bias: Option
     m = x2.shape[0]
     ldx = x2.stride(0) if m > 1 else k
     y = torch.empty((m, n), dtype=x.dtype, device=dev)
-    if m == 0:
-        return y.view(*x.shape[:-1], n)
-    b = None
-    if bias is not None:
-        b = bias if bias.dtype == torch.float16 else bias.to(torch.float16)
-        b = b.contiguous()
-    if force is None:
-        force = "gemv" if m <= GEMV_MAX_ROWS else "gemm"
-    if force not in ("stream", "gemv", "gemm"):
-        raise ValueError(f"force={force!r}")
-    args = [x2.data_ptr(), dtype, m, ldx, layout.tiles.data_ptr(), layout.scales_tiled.data_ptr(),
-            layout.chunk_ptr.data_ptr(), _capi.ptr(layout.entries), _capi.ptr(layout.vals_sorted), n, k,
-            layout.block_size, _capi.ptr(b), y.data_ptr(), n]
-    flag = status_word(dev).data_ptr()
-    with torch.cuda.device(dev):
-        if force == "stream":
-            ws = stream_workspace(dev)
-            status = L.atlas_qlinear_stream(*args, ws.data_ptr(), ws.numel(), flag, _capi.stream_ptr(dev))
-            _capi.check(status, "atlas_qlinear_stream")
-        elif force == "gemv":
-            status = L.atlas_qlinear_gemv(*args, flag, _capi.stream_ptr(dev))
-            _capi.check(status, "atlas_qlinear_gemv")
-        else:
-            ws_bytes = int(L.atlas_qlinear_gemm_workspace_bytes(m, n, k))
-            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-            status = L.atlas_qlinear_gemm(*args, ws.data_ptr(), ws_bytes, flag, _capi.stream_ptr(dev))
-            _capi.check(status, "atlas_qlinear_gemm")
+    if m:
+        b = None if bias is None else bias.to(torch.float16).contiguous()
+        ws = stream_workspace(dev)
+        with torch.cuda.device(dev):
+            status = L.atlas_qlinear_stream(
+                x2.data_ptr(), _capi.DTYPE_F16 if x.dtype == torch.float16 else _capi.DTYPE_BF16, m, ldx,
+                layout.tiles.data_ptr(), layout.scales_tiled.data_ptr(), layout.chunk_ptr.data_ptr(),
+                _capi.ptr(layout.entries), _capi.ptr(layout.vals_sorted), n, k, layout.block_size, _capi.ptr(b),
+                y.data_ptr(), n, ws.data_ptr(), ws.numel(), status_word(dev).data_ptr(), _capi.stream_ptr(dev))
+        _capi.check(status, "atlas_qlinear_stream")
     return y.view(*x.shape[:-1], n)
 
 
@@ -309,10 +305,7 @@ class FusedLinearGroup:
 
     def member_forward(self, index: int, x: torch.Tensor) -> Optional[torch.Tensor]:
         """Member ``index``'s output for ``x``, or None if the group does not apply (the member computes alone)."""
-        if x.device.type != "cuda" or x.dtype not in (torch.float16, torch.bfloat16):
-            return None
-        rows = x.numel() // x.shape[-1] if x.shape[-1] else 0
-        if rows == 0:
+        if not x.is_cuda or (x.dtype is not torch.float16 and x.dtype is not torch.bfloat16) or x.numel() == 0:
             return None
         if self.layout is None or self.layout.tiles.device != x.device:
             self.build(x.device)
@@ -325,7 +318,7 @@ class FusedLinearGroup:
         c[3].add(index)
         off = self.offsets[index]
         n = self.members[index].original_shape[0]
-        out = c[2][..., off:off + n]
+        out = c[2].narrow(-1, off, n)
         if len(c[3]) == len(self.members):
             self._cache = None   # everyone has been served: do not keep x and y alive
         return out
@@ -403,9 +396,13 @@ class QuantizedLinear(nn.Module):
             y = self._group.member_forward(self._group_index, x)
             if y is not None:
                 return y
+        lay = self._kernel_layout
+        bias = self.bias
+        if lay is not None and lay.source is q_tensor and x.is_cuda and lay.tiles.device == x.device and (
+                bias is None or bias.device == x.device):
+            return quantized_linear_forward(x, lay, self._bias_for(bias))
         # the kernels need a GPU; CPU activations are staged through it and the result returned
         compute_device = x.device if x.device.type == "cuda" else _capi.require_cuda()
-        lay = self._kernel_layout
         if lay is not None and lay.source is q_tensor and lay.tiles.device == compute_device:
             # the kernel image of these very streams is already on the device (the streams themselves may have
             # been moved off it by offload_canonical)

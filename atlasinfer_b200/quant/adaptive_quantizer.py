@@ -56,59 +56,12 @@ class QuantizedTensor(NamedTuple):
         return total + (128 if include_overhead else 0)
 
 
-def _launch_quantize(flat: torch.Tensor, block_size: int, z_threshold: float, counts: torch.Tensor, capacity: int):
-    """Enqueue the quantize kernel for a flat fp16 CUDA tensor; nothing is read back here."""
-    L = _capi.load()
-    dev = flat.device
-    numel = flat.numel()
-    n_blocks = (numel + block_size - 1) // block_size
-    padded = n_blocks * block_size
-    ws_bytes = int(L.atlas_quantize_workspace_bytes(numel, block_size))
-    with torch.cuda.device(dev):
-        codes = torch.empty(padded, dtype=torch.int8, device=dev)
-        scales = torch.empty(n_blocks, dtype=torch.float16, device=dev)
-        workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
-        ovals = torch.empty(capacity, dtype=torch.float16, device=dev)
-        oidx = torch.empty(capacity, dtype=torch.int64, device=dev)
-        status = L.atlas_quantize(
-            flat.data_ptr(), numel, block_size, float(z_threshold), codes.data_ptr(),
-            _capi.ptr(ovals), _capi.ptr(oidx), capacity, scales.data_ptr(), counts.data_ptr(),
-            workspace.data_ptr(), ws_bytes, _capi.stream_ptr(dev))
-    _capi.check(status, "atlas_quantize")
-    return dict(flat=flat, codes=codes, scales=scales, ovals=ovals, oidx=oidx, workspace=workspace,
-                capacity=capacity, padded=padded)
-
-
-def _first_capacity(padded: int) -> int:
-    # |z| > t bounds the outliers of a block by (block_size - 1) / t^2, but weight-like data has well under
-    # 1 %: start with 1/32 of the tensor and retry with full capacity in the rare case that is short
-    return min(padded, padded // 32 + 1024)
-
-
 def _quantize_many_on_device(flats, block_size: int, z_threshold: float):
     """Quantize several flat fp16 CUDA tensors (one device): all kernels are enqueued first, the stream
     lengths of all of them come back in one device-to-host copy.  Returns the four streams per tensor."""
-    dev = flats[0].device
-    with torch.cuda.device(dev):
-        counts = torch.empty((len(flats), 4), dtype=torch.int64, device=dev)
-    jobs = []
-    for i, flat in enumerate(flats):
-        padded = (flat.numel() + block_size - 1) // block_size * block_size
-        jobs.append(_launch_quantize(flat, block_size, z_threshold, counts[i], _first_capacity(padded)))
-    host = counts.cpu()   # the one synchronisation
-    out = []
-    for i, job in enumerate(jobs):
-        n_codes, n_out, timed_out, _ = (int(v) for v in host[i])
-        if timed_out:
-            raise _capi.AtlasError(_capi.ERR_TIMEOUT, "atlas_quantize: device-side wait timed out")
-        if n_out > job["capacity"]:   # rare: more outliers than the first buffer holds
-            job = _launch_quantize(job["flat"], block_size, z_threshold, counts[i], job["padded"])
-            n_codes, n_out, timed_out, _ = (int(v) for v in counts[i].cpu())
-            if timed_out:
-                raise _capi.AtlasError(_capi.ERR_TIMEOUT, "atlas_quantize: device-side wait timed out")
-        # codes: a view (the buffer is 0.3 % longer than the stream); outliers: copied out of their roomy buffers
-        out.append((job["codes"][:n_codes], job["ovals"][:n_out].clone(), job["oidx"][:n_out].clone(), job["scales"]))
-    return out
+    if not 32 <= block_size <= 512 or block_size % 32:
+        raise NotImplementedError(f"atlas_quantize: block_size {block_size} is not a multiple of 32 in [32, 512]")
+    return _capi.native().quantize_many(flats, block_size, z_threshold)
 
 
 def _quantize_on_device(flat: torch.Tensor, block_size: int, z_threshold: float):
