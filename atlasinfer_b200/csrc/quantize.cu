@@ -353,6 +353,47 @@ struct FastConsts {
     int tie_out;     // an exact tie is an outlier
 };
 
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// Outliers of all tiles before `tile` (whole warp).  All resident CTAs finish a tile at about the same time and find only
+// counts, no prefixes, among each other's, so the walk back covers 256 tiles per round trip.  A status word holds all
+// that is passed on, so relaxed accesses do.
+__device__ __forceinline__ long long look_back(const unsigned long long *status, int64_t tile, int lane, int64_t *counts) {
+    long long prefix = 0;
+    int64_t look = tile - 1;
+    for (int spins = 0; spins <= QT_SPIN_LIMIT; ++spins) {
+        unsigned long long v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int64_t idx = look - k * 32 - lane;
+            v[k] = idx >= 0 ? ld_relaxed_u64(status + idx) : ST_PREFIX;   // tiles before the first count as prefix 0
+        }
+        int taken = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (taken != k) continue;
+            const unsigned pm = __ballot_sync(0xffffffffu, (v[k] >> 62) == 2), none = __ballot_sync(0xffffffffu, (v[k] >> 62) == 0);
+            const int first = pm ? __ffs(pm) - 1 : 31;
+            if (none & (0xffffffffu >> (31 - first))) continue;          // not there yet
+            unsigned int contrib = lane < first || (!pm && lane == first) ? (unsigned int)(v[k] & ST_VALUE) : 0u;   // a tile's own count
+            prefix += (long long)__reduce_add_sync(0xffffffffu, contrib);
+            if (pm) return prefix + (long long)(__shfl_sync(0xffffffffu, v[k], first) & ST_VALUE);
+            ++taken;
+        }
+        look -= taken * 32;
+        if (taken == 0) __nanosleep(32);
+    }
+    if (lane == 0) atomicExch((unsigned long long *)&counts[2], 1ull);   // record and leave; the host reports ATLAS_ERR_TIMEOUT
+    return prefix;
+}
+
 // Byte offset of element e's code in the dense tile: 16-byte pieces permuted so that the eight blocks a warp works on
 // fall on different banks.
 __device__ __forceinline__ int dense_byte(int e) { return e ^ (((e >> 7) & 7) << 4); }
@@ -569,36 +610,11 @@ __global__ void __launch_bounds__(QT_THREADS, 5) quantize_fast_kernel(QuantParam
             const unsigned long long agg = (unsigned long long)s_tile_total;
             long long prefix = 0;
             if (tile == 0) {
-                if (lane == 0) st_release_u64(p.status, ST_PREFIX | agg);
+                if (lane == 0) st_relaxed_u64(p.status, ST_PREFIX | agg);
             } else {
-                if (lane == 0) st_release_u64(p.status + tile, ST_AGG | agg);
-                int64_t look = tile - 1;
-                bool done = false;
-                while (!done) {
-                    const int64_t idx = look - lane;
-                    unsigned long long v = ST_PREFIX;  // tiles before the first count as prefix 0
-                    int spins = 0;
-                    bool gave_up = false;
-                    for (;;) {
-                        if (idx >= 0) v = ld_acquire_u64(p.status + idx);
-                        const bool ready = (v >> 62) != 0;
-                        if (__all_sync(0xffffffffu, ready)) break;
-                        if (++spins > QT_SPIN_LIMIT) { gave_up = true; break; }
-                        __nanosleep(64);
-                    }
-                    if (gave_up) {  // record and leave; the host reports ATLAS_ERR_TIMEOUT
-                        if (lane == 0) atomicExch((unsigned long long *)&p.counts[2], 1ull);
-                        break;
-                    }
-                    const unsigned pm = __ballot_sync(0xffffffffu, (v >> 62) == 2);
-                    const int first = pm ? (__ffs(pm) - 1) : 32;
-                    long long contrib = (lane <= first) ? (long long)(v & ST_VALUE) : 0;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
-                    prefix += contrib;
-                    if (pm) done = true; else look -= 32;
-                }
-                if (lane == 0) st_release_u64(p.status + tile, ST_PREFIX | (unsigned long long)(prefix + (long long)agg));
+                if (lane == 0) st_relaxed_u64(p.status + tile, ST_AGG | agg);
+                prefix = look_back(p.status, tile, lane, p.counts);
+                if (lane == 0) st_relaxed_u64(p.status + tile, ST_PREFIX | (unsigned long long)(prefix + (long long)agg));
             }
             if (lane == 0) {
                 s_tile_prefix = prefix;
