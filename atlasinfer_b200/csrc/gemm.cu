@@ -771,6 +771,8 @@ gemm_finish_kernel(const float *partials, int splits, int m, int n_rows, const u
 // bf16 -> fp16 (saturating) into a dense [m][k] buffer; also used to make strided fp16 rows dense.  When x is a
 // gathered buffer that the other ranks fill (`wait_flags`), every CTA first waits, bounded, until all ranks'
 // arrival counts have reached this rank's own (state[1]).
+// VEC: the rows allow 16-byte loads.
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 to_f16_kernel(const uint16_t *x, int64_t ldx, int m, int k, int from_bf16, uint16_t *out, const unsigned int *wait_flags,
               int wait_world, const unsigned int *state, long long poll_limit, int *status) {
@@ -793,6 +795,18 @@ to_f16_kernel(const uint16_t *x, int64_t ldx, int m, int k, int from_bf16, uint1
             if (!__all_sync(0xffffffffu, ok) && lane == 0 && status) atomicExch(status, 1);   // reported; the copy goes on
         }
         __syncthreads();
+    }
+    if (VEC) {
+        // 8 elements per thread (n_cols is a multiple of 64, so a piece never straddles rows)
+        const int per_row = k >> 3;
+        const int64_t total = (int64_t)m * per_row;
+        for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
+            const int row = (int)(i / per_row), piece = (int)(i - (int64_t)row * per_row);
+            uint4 v = __ldcg(reinterpret_cast<const uint4 *>(x + (int64_t)row * ldx) + piece);
+            if (from_bf16) v = make_uint4(bf16x2_to_f16x2(v.x), bf16x2_to_f16x2(v.y), bf16x2_to_f16x2(v.z), bf16x2_to_f16x2(v.w));
+            reinterpret_cast<uint4 *>(out)[i] = v;
+        }
+        return;
     }
     const int64_t total = (int64_t)m * (k >> 1);
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
@@ -979,10 +993,9 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
     const bool wait_in_copy = wait_flags && !direct;
     if (!direct) {
         uint16_t *xf = (uint16_t *)((char *)workspace + GM_WS_HEADER);
-        const int64_t pairs = m * (n_cols / 2);
-        const int64_t blocks = ceil_div_i64(pairs, 256);
+        const int64_t blocks = ceil_div_i64(m * (n_cols / (tma_ok ? 8 : 2)), 256);
         cudaLaunchConfig_t cfg = pdl_config(dim3((unsigned)(blocks < 65535 ? blocks : 65535)), dim3(256), 0, st);
-        rc = check_cuda(cudaLaunchKernelEx(&cfg, to_f16_kernel, (const uint16_t *)x, ldx, (int)m, (int)n_cols,
+        rc = check_cuda(cudaLaunchKernelEx(&cfg, tma_ok ? to_f16_kernel<true> : to_f16_kernel<false>, (const uint16_t *)x, ldx, (int)m, (int)n_cols,
                                            (int)(dtype == ATLAS_DTYPE_BF16), xf, wait_in_copy ? wait_flags : (const unsigned int *)nullptr,
                                            gather ? (int)gather->world : 0,
                                            gather ? (const unsigned int *)gather->state : (const unsigned int *)nullptr,
