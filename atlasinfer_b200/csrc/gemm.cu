@@ -1,10 +1,11 @@
-// Prefill-time quantized linear: y[m][n] = sum_k x[m][k] * W[n][k] + bias[n], m >= 128.
+// Quantized linear for prompts: y[m][n] = sum_k x[m][k] * W[n][k] + bias[n], m > 128 (fewer rows: gemm_tile.cu), and
+// the decode-sized form whose output is gathered over the ranks of a node (m <= 64).
 //
 // Replaces the dequantize-then-F.linear of QuantizedLinear.forward
 // (integration/atlas_wrappers.py:56,67) for prompt-sized batches.  The fp16
 // weight the reference materialises (adaptive_quantizer.py:216:
 // fp16(fp16(code) * scale), outliers patched in at :221-229) is rebuilt here
-// tile by tile in shared memory and consumed at once by the 5th-generation
+// tile by tile in tensor memory and consumed at once by the 5th-generation
 // tensor cores, so it never exists in global memory.
 //
 // One CTA computes a 128 (output features) x BN (tokens) tile.  The rebuilt fp16 weights never touch
@@ -34,14 +35,22 @@
 // Every mbarrier wait is bounded; if one runs out the CTA sets the caller's status word,
 // skips the rest of its work, frees its TMEM and returns.
 //
-// bf16 activations are first converted to fp16 into the workspace (the MMA
-// takes both operands as fp16; |x| > 65504 saturates).
+// bf16 activations are first converted to fp16 into the workspace, 16 bytes per thread (the MMA takes both operands as
+// fp16; |x| > 65504 saturates).  Two bytes at a time that kernel cost 5 % of a 2048-token linear (965 -> 1020 TFLOP/s at
+// 11008 x 4096).
+//
+// Not taken: a CTA pair per 256-row tile (cta_group::2, half the activation tile in each CTA, the arrivals of the second
+// CTA passed on to the first one's barriers).  It halves the activation traffic of an SM's shared memory, but every
+// stage then waits for the slower CTA's dequantizers and a round trip between the SMs: 812 against 1018 TFLOP/s at
+// 2048 x 22016 x 4096.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <cstring>
 
 #include "common.cuh"
+#include "gemm_tile.cuh"
+#include "tensor_core.cuh"
 
 namespace atlas {
 namespace {
@@ -83,132 +92,10 @@ struct Smem {
     static_assert((BN * (GM_BM + 4)) * 4 <= XS * GM_SK * B_BYTES + CS * GM_SK * C_BYTES, "epilogue staging does not fit");
     static_assert(TOTAL <= 227 * 1024, "shared memory");
 };
-constexpr int GM_SPIN_LIMIT = 1 << 20;       // polls per wait
-
-// ---- PTX wrappers ----------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded wait: false if the phase did not complete within the poll limit.  NS > 0 sleeps between polls, which
-// keeps a waiting warp out of the issue slots of the warps that work on the same scheduler.
-template <int NS = 0>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < GM_SPIN_LIMIT; ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (NS > 0) __nanosleep(NS);
-    }
-    return false;
-}
-// Same, agreed on by the whole (converged) warp, so that warp-wide instructions after it stay warp-wide.
-template <int NS = 0>
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const volatile int *abort_flag) {
-    return __all_sync(0xffffffffu, mbar_wait<NS>(bar, parity) && !*abort_flag) != 0;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
-__device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-        ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// D[tmem] (+)= A[tmem] * B[smem]: A is 128 lanes x 8 columns (16 fp16 along K, two per cell)
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// 32 lanes (this warp's quarter) x 32 columns: thread t writes v[0..31] to lane t, columns taddr.col .. + 31
-__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-          "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
-          "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
-          "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// Shared-memory matrix descriptor: K-major operand tile, rows of 128 bytes (64 fp16), 128-byte
-// swizzle, 8-row groups 1024 bytes apart.  Fields: start address >> 4 at bit 0, leading byte
-// offset >> 4 at bit 16 (not used by swizzled K-major layouts; 1), stride byte offset >> 4 at bit
-// 32, descriptor version 1 at bit 46, swizzle mode 2 (128 B) at bit 61.
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3ffffu) >> 4);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
 // Instruction descriptor, kind::f16: D fp32 (1 at bit 4), A and B fp16 (0 at bits 7 and 10),
 // both K-major (0 at bits 15, 16), N >> 3 at bit 17, M >> 4 at bit 24.
 template <int BN>
 constexpr uint32_t gm_idesc() { return (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(GM_BM >> 4) << 24); }
-
-// Two bf16 (low, high half of v) -> two fp16, saturating at +-65504.
-__device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t v) {
-    uint32_t r;
-    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(__uint_as_float(v & 0xffff0000u)), "f"(__uint_as_float(v << 16)));
-    return r;
-}
-
-// Four biased codes -> two half2 of fp16(fp16(code) * scale), as in the streaming kernel.
-__device__ __forceinline__ void dequant4(uint32_t w, __half2 scale2, uint32_t &lo, uint32_t &hi) {
-    const uint32_t l = __byte_perm(w, 0x64646464u, 0x5140);
-    const uint32_t h = __byte_perm(w, 0x64646464u, 0x5342);
-    const __half2 bias = __halves2half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480));
-    __half2 lv = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&l), bias), scale2);
-    __half2 hv = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&h), bias), scale2);
-    lo = *reinterpret_cast<uint32_t *>(&lv);
-    hi = *reinterpret_cast<uint32_t *>(&hv);
-}
 
 struct GemmParams {
     const uint8_t *tiles;
@@ -863,22 +750,23 @@ cudaLaunchConfig_t pdl_config(dim3 grid, dim3 block, size_t smem, cudaStream_t s
     return cfg;
 }
 
-// tokens per tile for a batch of m rows
-int gemm_bn_for(int64_t m) { return m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256)); }
+// tokens per tile for a batch of m rows (up to 128 rows that are not gathered go to the kernel in gemm_tile.cu)
+int gemm_bn_for(int64_t m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 256); }
 
-// K slices for decode-sized batches (one CTA per SM, `tiles` output tiles): the count that minimises
-// waves x (k-tiles per CTA + the fixed cost of a CTA, about 12 k-tiles' worth of streaming), so that neither a
-// nearly empty last wave nor many short CTAs dominate.
+// K slices (one CTA per SM, `tiles` output tiles).
+// Decode-sized tiles: the count that minimises waves x (k-tiles per CTA + the fixed cost of a CTA, about 12 k-tiles'
+// worth of streaming), so that neither a nearly empty last wave nor many short CTAs dominate.
 int gemm_splits_for(int64_t m, int64_t n_rows, int64_t n_cols, int sms) {
     const int bn = gemm_bn_for(m);
     if (bn > 64) return 1;
     const int64_t tiles = ceil_div_i64(n_rows, GM_BM) * ceil_div_i64(m, bn);
     const int k_tiles = (int)(n_cols / 64);
     int best = 1;
-    int64_t best_cost = 0;
+    double best_cost = 0;
     for (int s = 1; s <= 16; s *= 2) {
         if (s > 1 && k_tiles / s < 8) break;
-        const int64_t cost = ceil_div_i64(tiles * s, sms) * (ceil_div_i64(k_tiles, s) + 12);
+        const double waves = (double)ceil_div_i64(tiles * s, sms);
+        const double cost = waves * (double)(ceil_div_i64(k_tiles, s) + 12);
         if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
     }
     return best;
@@ -916,13 +804,12 @@ int launch_gemm(const CUtensorMap &x_map, const CUtensorMap &c_map, const GemmPa
 
 extern "C" size_t atlas_qlinear_gemm_workspace_bytes(int64_t m, int64_t n_rows, int64_t n_cols) {
     if (m <= 0 || n_cols <= 0 || n_rows <= 0) return atlas::GM_WS_HEADER;
-    // fp16 copy of x (bf16 or strided input), then room for up to 8 fp32 K-slice partial outputs
-    // (only decode-sized batches are ever sliced)
+    // fp16 copy of x (bf16 or strided input), then room for the fp32 partial outputs of the K slices
     const size_t xcopy = ((size_t)m * (size_t)n_cols * 2 + 255) & ~(size_t)255;
     // (one fp32 slice of the output per K slice; one even without slicing, for the gathered form)
-    const size_t part = atlas::gemm_bn_for(m) <= 64
-                            ? (size_t)atlas::gemm_splits_for(m, n_rows, n_cols, atlas::gemm_sm_count()) * (size_t)m * (size_t)n_rows * 4
-                            : 0;
+    const int splits = atlas::gemm_splits_for(m, n_rows, n_cols, atlas::gemm_sm_count());
+    const size_t part = m > atlas::TILE_MAX_TOKENS ? (splits > 1 ? (size_t)splits * (size_t)m * (size_t)n_rows * 4 : 0)
+                        : (m <= 64 ? (size_t)splits * (size_t)m * (size_t)n_rows * 4 : 0);
     return atlas::GM_WS_HEADER + xcopy + part;
 }
 
@@ -974,7 +861,9 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
     if (rc) return rc;
     if (m == 0) return ATLAS_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    const int bn = gemm_bn_for(m);
+    // (the gathered form's arrival protocol lives in the kernels below)
+    const bool tile = !gather && m <= TILE_MAX_TOKENS;
+    const int bn = tile ? tile_tokens_for(m) : gemm_bn_for(m);
 
     // operand B must be fp16 with rows on 16-byte boundaries for the tensor map
     const void *xb = x;
@@ -984,9 +873,10 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
     // Rows the tensor map can take as they are: 16-byte aligned, fp16 -- or bf16 for decode-sized token tiles,
     // which the kernel converts in shared memory.  Anything else is copied to a dense fp16 buffer first.
     const bool tma_ok = ((uintptr_t)x & 15) == 0 && (ldx % 8) == 0;
-    // (in the kernel when the weight is small: one more kernel in the chain then costs more than the conversion's
-    // share of the producer warp over the few stages of a CTA)
-    const bool small_weight = n_rows * n_cols <= ((int64_t)32 << 20);
+    // (in the kernel when the weight is small: one more kernel in the chain then costs more than the conversion by one
+    // warp over the few stages of a CTA.  16 rows of 4096 x 4096: 11.2 us with the copy, 10.5 without; 64 rows: 14.0
+    // and 16.0, but 9.6 and 9.4 at 2048 x 2048)
+    const bool small_weight = n_rows * n_cols <= ((int64_t)(tile && bn == 64 ? 8 : 32) << 20);
     const bool in_kernel_bf16 = dtype == ATLAS_DTYPE_BF16 && bn <= 64 && tma_ok && small_weight;
     const bool direct = tma_ok && (dtype == ATLAS_DTYPE_F16 || in_kernel_bf16);
     // a gathered input is waited for by whichever kernel reads x first: the copy kernel, or the linear kernel itself
@@ -1029,6 +919,26 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
         ATLAS_RETURN_IF(cr != CUDA_SUCCESS, ATLAS_ERR_LAUNCH, "cuTensorMapEncodeTiled (codes) failed with %d", (int)cr);
     }
 
+    if (tile) {
+        TileParams t;
+        t.scales_t = (const uint16_t *)scales_tiled;
+        t.chunk_ptr = outlier_chunk_ptr;
+        t.entries = outlier_entries;
+        t.ovals = (const uint16_t *)outlier_vals_sorted;
+        t.bias = (const uint16_t *)bias;
+        t.y = y;
+        t.ldy = ldy;
+        t.m = (int)m;
+        t.n_rows = (int)n_rows;
+        t.bs = block_size;
+        t.k_tiles = (int)(n_cols / GM_BK);
+        t.blocks_per_row = (int)(n_cols / block_size);
+        t.bs_tiles = block_size % GM_BK == 0 ? block_size / GM_BK : 0;
+        t.out_bf16 = dtype == ATLAS_DTYPE_BF16;
+        t.x_bf16 = in_kernel_bf16;
+        t.error_flag = status;
+        return launch_tile(x_map, c_map, t, gemm_sm_count(), st);
+    }
     GemmParams p;
     p.tiles = tiles;
     p.scales_t = (const uint16_t *)scales_tiled;
@@ -1058,7 +968,6 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
     switch (bn) {
         case 32: rc = launch_gemm<32>(x_map, c_map, p, st); break;
         case 64: rc = launch_gemm<64>(x_map, c_map, p, st); break;
-        case 128: rc = launch_gemm<128>(x_map, c_map, p, st); break;
         default: rc = launch_gemm<256>(x_map, c_map, p, st); break;
     }
     if (rc) return rc;

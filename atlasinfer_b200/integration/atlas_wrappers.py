@@ -21,8 +21,9 @@ import torch.nn as nn
 from .. import _capi
 from ..quant.adaptive_quantizer import QuantizedTensor
 
-# rows of x up to which the per-strip streaming kernel is used (8 rows per pass over the weight); above it the
-# tcgen05 kernel.  The persistent streaming kernel takes up to STREAM_MAX_ROWS rows in one pass; it is what the
+# rows of x up to which the per-strip streaming kernel is used (16 rows per pass over the weight); above it the tcgen05
+# kernels.  At 16 rows the two are within 10 % of each other either way (4096 x 4096 9.1 against 10.8 us, 10240 x 8192
+# 37 against 32).  The persistent streaming kernel takes up to STREAM_MAX_ROWS rows in one pass; it is what the
 # column-parallel linear with the fused gather runs on and can be asked for with force="stream".
 GEMV_MAX_ROWS = 16
 STREAM_MAX_ROWS = 32

@@ -197,13 +197,14 @@ ATLAS_API int atlas_repack_many(int count, const AtlasRepackItem *items, void *s
  * earlier work has completed.  The kernel has no bounded wait: `status` is
  * accepted for symmetry and never written.
  *
- * atlas_qlinear_gemm: larger batches (any m >= 1 accepted).  The code tiles
- * come in by TMA, are dequantised by 16 warps straight into tensor memory as
- * the fp16 A operand of tcgen05.mma (the activations are the B operand, from
- * shared memory; fp32 accumulators in tensor memory); the token tile is 32,
- * 64, 128 or 256 wide by m, and for decode-sized batches K is sliced over CTAs
- * with the fp32 partial tiles added in slice order by a second kernel
- * (deterministic).
+ * atlas_qlinear_gemm: larger batches (any m >= 1 accepted).  Code tiles and
+ * activations come in by TMA and go through tcgen05.mma with fp32 accumulators
+ * in tensor memory.  Up to 128 rows: the weights are rebuilt into shared memory
+ * (token tiles of 16 to 128), K is sliced over the CTAs of a cluster, which add
+ * their fp32 tiles in slice order.  More rows: the weights are rebuilt straight
+ * into tensor memory (token tiles of 256); where that leaves much of the chip
+ * idle K is sliced and a second kernel adds the partial tiles in slice order.
+ * Deterministic either way.
  * `workspace` must hold atlas_qlinear_gemm_workspace_bytes(m, n_rows, n_cols)
  * bytes, 256-byte aligned.
  */
