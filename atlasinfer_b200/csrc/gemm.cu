@@ -756,17 +756,20 @@ int gemm_bn_for(int64_t m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 256); }
 // K slices (one CTA per SM, `tiles` output tiles).
 // Decode-sized tiles: the count that minimises waves x (k-tiles per CTA + the fixed cost of a CTA, about 12 k-tiles'
 // worth of streaming), so that neither a nearly empty last wave nor many short CTAs dominate.
+// Prompts: a CTA takes 0.4 us per k-tile and 7 us besides; slicing adds a second kernel (2.5 us) and the fp32 partial
+// sums' way through L2 and back (about 4 TB/s).  Few row tiles and one or two token tiles leave most of the chip idle
+// otherwise: 4096 x 11008 at 301 tokens is 64 tiles.
 int gemm_splits_for(int64_t m, int64_t n_rows, int64_t n_cols, int sms) {
     const int bn = gemm_bn_for(m);
-    if (bn > 64) return 1;
     const int64_t tiles = ceil_div_i64(n_rows, GM_BM) * ceil_div_i64(m, bn);
     const int k_tiles = (int)(n_cols / 64);
     int best = 1;
     double best_cost = 0;
-    for (int s = 1; s <= 16; s *= 2) {
+    for (int s = 1; s <= 16; s = bn > 64 ? s + 1 : s * 2) {
         if (s > 1 && k_tiles / s < 8) break;
         const double waves = (double)ceil_div_i64(tiles * s, sms);
-        const double cost = waves * (double)(ceil_div_i64(k_tiles, s) + 12);
+        double cost = waves * (double)(ceil_div_i64(k_tiles, s) + 12);
+        if (bn > 64) cost = waves * (0.4 * (double)ceil_div_i64(k_tiles, s) + 7.0) + (s > 1 ? 2.5 + 2e-6 * s * (double)m * (double)n_rows : 0.0);
         if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
     }
     return best;
