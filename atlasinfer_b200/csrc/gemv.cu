@@ -115,16 +115,22 @@ __device__ __forceinline__ void load_x16(const uint16_t *src, uint32_t (&xv)[8])
 //
 // FAST (whole 256-column chunks, blocks of whole 64-column tiles): every batch of a warp is full and a step has one
 // scale block, so the K loop carries no bounds predicates and no per-lane block index.
-template <bool BF16, bool VEC, int MT, bool STAGE, bool FAST>
+//
+// RS (strips per CTA; 2 only with FAST and one MMA tile): a step is one k-tile of both strips instead of two k-tiles of
+// one, so the activations of a step are loaded (and converted) once for two strips and a warp's set-up serves twice the
+// codes.  The bytes in flight stay the same.
+template <bool BF16, bool VEC, int MT, bool STAGE, bool FAST, int RS = 1>
 __global__ void __launch_bounds__((MT == 1 ? GS_MAX_WARPS : GS_WARPS2) * 32, 2) gemv_strip_kernel(GemvParams p) {
     constexpr int U = MT == 1 ? GS_UNROLL : 2 * GS_UNROLL;
-    __shared__ float4 part[MT][MT == 1 ? GS_MAX_WARPS : GS_WARPS2][32];
+    constexpr int NT = RS * MT;   // 16 x 8 accumulator tiles of a warp
+    static_assert(RS == 1 || (MT == 1 && FAST), "two strips: one token tile, whole chunks");
+    __shared__ float4 part[NT][MT == 1 ? GS_MAX_WARPS : GS_WARPS2][32];
     extern __shared__ __align__(16) unsigned char xs_raw[];   // STAGE: [m][n_cols fp16 + 16 bytes of padding]
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const int g = lane >> 2, tig = lane & 3;
-    const int strip = blockIdx.x;
+    const int strip = blockIdx.x * RS;   // (an even one with RS 2: both strips lie in one 128-row tile)
     // (a CTA has 16 warps unless K is short: the split of the chunks over them then needs no division)
     const int c0 = nwarps == 16 ? (p.n_chunks * warp) >> 4 : (nwarps == 8 ? (p.n_chunks * warp) >> 3 : (p.n_chunks * warp) / nwarps);
     const int c1 = nwarps == 16 ? (p.n_chunks * (warp + 1)) >> 4 : (nwarps == 8 ? (p.n_chunks * (warp + 1)) >> 3 : (p.n_chunks * (warp + 1)) / nwarps);
@@ -146,7 +152,14 @@ __global__ void __launch_bounds__((MT == 1 ? GS_MAX_WARPS : GS_WARPS2) * 32, 2) 
     auto load_batch = [&](int kt) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (FAST || kt + u < kt1) {
+            if (RS == 2) {
+                const uint8_t *tp = wbase + (size_t)((uint32_t)kt << 13) + u * 1024;
+                wa[u] = ldg_stream(tp);
+                wb[u] = ldg_stream(tp + 512);
+                const uint16_t *sp = sbase + (size_t)((uint32_t)(kt >> (p.bs_shift - 6)) << 7) + u * 16;
+                sa[u] = __ldg(sp);
+                sb[u] = __ldg(sp + 8);
+            } else if (FAST || kt + u < kt1) {
                 const uint8_t *tp = wbase + (FAST ? (size_t)((uint32_t)(kt + u) << 13) : (size_t)(kt + u) * 8192);
                 wa[u] = ldg_stream(tp);
                 wb[u] = ldg_stream(tp + 512);
@@ -160,25 +173,32 @@ __global__ void __launch_bounds__((MT == 1 ? GS_MAX_WARPS : GS_WARPS2) * 32, 2) 
     load_batch(kt0);
     // first group of outlier entries of the strip inside this warp's columns, and the bias
     const int32_t *cptr = p.chunk_ptr + (size_t)strip * (p.k_tiles + 1);
-    int e_begin = 0, e_end = 0;
-    if (kt0 < kt1) { e_begin = __ldg(cptr + kt0); e_end = __ldg(cptr + kt1); }
+    int e_begin[RS], e_end[RS];
     // an empty slot of an outlier group: row 255 matches no lane; its column is one of this warp's own (with the staged
     // row a warp reads only what it has written itself)
     const uint32_t no_entry = 0xff000000u | (uint32_t)(kt0 * 64);
-    uint32_t pre_ent[4], pre_val[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int e = e_begin + 2 * tig + (q & 1) + (q >> 1) * 8;
-        pre_ent[q] = no_entry;
-        pre_val[q] = 0;
-        if (e < e_end) { pre_ent[q] = __ldg(p.entries + e); pre_val[q] = __ldg(p.ovals + e); }
+    for (int r = 0; r < RS; ++r) {
+        e_begin[r] = e_end[r] = 0;
+        if (kt0 < kt1) { e_begin[r] = __ldg(cptr + r * (p.k_tiles + 1) + kt0); e_end[r] = __ldg(cptr + r * (p.k_tiles + 1) + kt1); }
     }
+    uint32_t pre_ent[4], pre_val[4];
+    auto load_group = [&](int r, int e0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = e0 + 2 * tig + (q & 1) + (q >> 1) * 8;
+            pre_ent[q] = no_entry;
+            pre_val[q] = 0;
+            if (e < e_end[r]) { pre_ent[q] = __ldg(p.entries + e); pre_val[q] = __ldg(p.ovals + e); }
+        }
+    };
+    load_group(0, e_begin[0]);
     // (MMA tile, lane, component) this thread reduces at the end: 128 outputs per tile
     const int rT = tid >> 7, rL = (tid >> 2) & 31, rj = tid & 3;
-    const int out_row = (rL >> 2) + (rj >> 1) * 8, out_m = rT * 8 + (rL & 3) * 2 + (rj & 1);
-    const int out_n = strip * 16 + out_row;
+    const int out_row = (rL >> 2) + (rj >> 1) * 8, out_m = (RS == 1 ? rT * 8 : 0) + (rL & 3) * 2 + (rj & 1);
+    const int out_n = (strip + (RS == 1 ? 0 : rT)) * 16 + out_row;
     float bias_v = 0.f;
-    if (tid < 128 * MT && p.bias && out_n < p.n_rows) bias_v = __half2float(__ushort_as_half(__ldg(p.bias + out_n)));
+    if (tid < 128 * NT && p.bias && out_n < p.n_rows) bias_v = __half2float(__ushort_as_half(__ldg(p.bias + out_n)));
 
     // ---- activations: only after the earlier kernels of the stream have completed ------------------
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -205,12 +225,12 @@ __global__ void __launch_bounds__((MT == 1 ? GS_MAX_WARPS : GS_WARPS2) * 32, 2) 
     // this lane's row of staged activations (rows that do not exist read row 0, as above)
     const unsigned char *xs_lane = xs_raw + (size_t)(g < p.m ? g : 0) * xs_row_bytes;
 
-    float acc[MT][4];
+    float acc[NT][4];
 #pragma unroll
-    for (int nt = 0; nt < MT; ++nt)
+    for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[nt][c] = 0.f;
-    auto outlier_mma = [&](const uint32_t (&ent)[4], const uint32_t (&val)[4]) {
+    auto outlier_mma = [&](int r, const uint32_t (&ent)[4], const uint32_t (&val)[4]) {
         int rws[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) rws[q] = (int)(ent[q] >> 24);
@@ -230,13 +250,39 @@ __global__ void __launch_bounds__((MT == 1 ? GS_MAX_WARPS : GS_WARPS2) * 32, 2) 
                 asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(b0) : "f"(__uint_as_float(xq[1] << 16)), "f"(__uint_as_float(xq[0] << 16)));
                 asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(b1) : "f"(__uint_as_float(xq[3] << 16)), "f"(__uint_as_float(xq[2] << 16)));
             }
-            mma_f16(acc[nt], a0, a1, a2, a3, b0, b1);
+            mma_f16(acc[RS == 1 ? nt : r], a0, a1, a2, a3, b0, b1);
         }
     };
-    if (e_begin < e_end) outlier_mma(pre_ent, pre_val);   // its activation gathers overlap the K loop's loads
+    if (e_begin[0] < e_end[0]) outlier_mma(0, pre_ent, pre_val);   // its activation gathers overlap the K loop's loads
+    if (RS == 2) load_group(RS - 1, e_begin[RS - 1]);   // the second strip's first group travels during the K loop
 
-    for (int kt = kt0; kt < kt1; kt += U) {
+    for (int kt = kt0; kt < kt1; kt += RS == 2 ? 1 : U) {
         if (kt != kt0) load_batch(kt);
+        if (RS == 2) {
+            uint32_t xv[8];
+            if (STAGE) {
+                const uint4 a = *reinterpret_cast<const uint4 *>(xs_lane + (kt * 64 + tig * 16) * 2);
+                const uint4 b = *reinterpret_cast<const uint4 *>(xs_lane + (kt * 64 + tig * 16) * 2 + 16);
+                xv[0] = a.x; xv[1] = a.y; xv[2] = a.z; xv[3] = a.w;
+                xv[4] = b.x; xv[5] = b.y; xv[6] = b.z; xv[7] = b.w;
+            } else {
+                load_x16<BF16, VEC>(xrow[0] + kt * 64, xv);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t wav[4] = {wa[u].x, wa[u].y, wa[u].z, wa[u].w};
+                const uint32_t wbv[4] = {wb[u].x, wb[u].y, wb[u].z, wb[u].w};
+                const __half2 sa2 = __half2half2(__ushort_as_half(sa[u])), sb2 = __half2half2(__ushort_as_half(sb[u]));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    uint32_t alo, ahi, blo, bhi;
+                    dequant4(wav[i], sa2, alo, ahi);
+                    dequant4(wbv[i], sb2, blo, bhi);
+                    mma_f16(acc[RS == 2 ? u : 0], alo, blo, ahi, bhi, xv[2 * i], xv[2 * i + 1]);
+                }
+            }
+            continue;
+        }
         if (MT == 1) {
             // all activations of the batch first, then the arithmetic
             uint32_t xv[U][8];
@@ -289,22 +335,18 @@ __global__ void __launch_bounds__((MT == 1 ? GS_MAX_WARPS : GS_WARPS2) * 32, 2) 
             }
         }
     }
-    for (int e0 = e_begin + 16; e0 < e_end; e0 += 16) {    // remaining outlier groups, 16 per MMA
-        uint32_t ent[4], val[4];
+    if (RS == 2 && e_begin[RS - 1] < e_end[RS - 1]) outlier_mma(RS - 1, pre_ent, pre_val);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int e = e0 + 2 * tig + (q & 1) + (q >> 1) * 8;
-            ent[q] = no_entry;
-            val[q] = 0;
-            if (e < e_end) { ent[q] = __ldg(p.entries + e); val[q] = __ldg(p.ovals + e); }
+    for (int r = 0; r < RS; ++r)
+        for (int e0 = e_begin[r] + 16; e0 < e_end[r]; e0 += 16) {    // remaining outlier groups, 16 per MMA
+            load_group(r, e0);
+            outlier_mma(r, pre_ent, pre_val);
         }
-        outlier_mma(ent, val);
-    }
 
 #pragma unroll
-    for (int nt = 0; nt < MT; ++nt) part[nt][warp][lane] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
+    for (int nt = 0; nt < NT; ++nt) part[nt][warp][lane] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
     __syncthreads();
-    if (tid < 128 * MT) {
+    if (tid < 128 * NT) {
         float s = bias_v;
         for (int w = 0; w < nwarps; ++w) s += reinterpret_cast<const float *>(&part[rT][w][rL])[rj];
         if (out_m < p.m && out_n < p.n_rows) {
@@ -320,14 +362,22 @@ template <int MT>
 int launch_gemv_strip(const GemvParams &p, bool vec, cudaStream_t st) {
     const int max_warps = MT == 1 ? GS_MAX_WARPS : GS_WARPS2;
     int nwarps = p.n_chunks < max_warps ? p.n_chunks : max_warps;
-    if (nwarps < 4 * MT) nwarps = 4 * MT;  // the reduction needs 128 threads per MMA tile
+    const bool fast = vec && (p.k_tiles & 3) == 0 && p.bs_shift >= 6;   // whole chunks, blocks of whole tiles
+    const int64_t strips = ceil_div_i64(p.n_rows, 16);
+    // Strip pairs pay where a warp has little of K to spread its set-up over (at most one 256-column chunk: 12288 x 4096
+    // 15.7 -> 14.6 us at one bf16 row, 18.1 -> 16.3 at eight; 22016 x 4096 24.4 -> 22.4 and 28.7 -> 25.4) and, for
+    // bf16, whose conversion they halve, over many waves of CTAs (57344 x 8192 96 -> 93, 110 -> 104; with fp16 rows
+    // 95 -> 96).  They lose where half the CTAs fill the SMs once and a little (10240 x 8192: 23 -> 26) or not at all
+    // (4096 x 4096: 6.0 -> 8.6).
+    const bool two = MT == 1 && fast && strips >= 4 * 148 &&
+                     (p.n_chunks <= GS_MAX_WARPS || (p.dtype == ATLAS_DTYPE_BF16 && strips >= 16 * 148));
+    if (nwarps < 4 * MT * (two ? 2 : 1)) nwarps = 4 * MT * (two ? 2 : 1);  // the reduction needs 128 threads per MMA tile
     // one or two rows of bf16 activations are converted once per CTA into shared memory (measured at 1 / 2 / 4 / 8
     // rows: 3.7 / 3.5 / 3.1 / 2.6 TB/s staged against 3.4 / 3.3 / 3.3 / 3.1 converted per step)
     const size_t stage_bytes = (size_t)p.m * ((size_t)p.n_cols * 2 + 16);
-    const bool fast = vec && (p.k_tiles & 3) == 0 && p.bs_shift >= 6;   // whole chunks, blocks of whole tiles
     const bool stage = MT == 1 && p.dtype == ATLAS_DTYPE_BF16 && vec && p.m <= 2 && stage_bytes <= (size_t)GS_STAGE_MAX_BYTES;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((p.n_rows + 15) / 16), 1, 1);
+    cfg.gridDim = dim3((unsigned)(two ? (strips + 1) / 2 : strips), 1, 1);
     cfg.blockDim = dim3((unsigned)(nwarps * 32), 1, 1);
     cfg.dynamicSmemBytes = stage ? stage_bytes : 0;
     cfg.stream = st;
@@ -337,16 +387,21 @@ int launch_gemv_strip(const GemvParams &p, bool vec, cudaStream_t st) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (stage) {
-        auto kern = fast ? gemv_strip_kernel<true, true, 1, true, true> : gemv_strip_kernel<true, true, 1, true, false>;
-        static thread_local int configured_dev[2] = {-1, -1};   // more than the default dynamic shared memory: opt in once
+        auto kern = two ? gemv_strip_kernel<true, true, 1, true, true, 2>
+                        : (fast ? gemv_strip_kernel<true, true, 1, true, true> : gemv_strip_kernel<true, true, 1, true, false>);
+        static thread_local int configured_dev[3] = {-1, -1, -1};   // more than the default dynamic shared memory: opt in once
         int dev = 0;
         cudaGetDevice(&dev);
-        if (configured_dev[fast] != dev) {
+        if (configured_dev[two ? 2 : (int)fast] != dev) {
             int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_STAGE_MAX_BYTES),
                                 "cudaFuncSetAttribute(gemv smem)");
             if (rc) return rc;
-            configured_dev[fast] = dev;
+            configured_dev[two ? 2 : (int)fast] = dev;
         }
+        return check_cuda(cudaLaunchKernelEx(&cfg, kern, p), "gemv_strip_kernel launch");
+    }
+    if (two) {
+        auto kern = p.dtype == ATLAS_DTYPE_BF16 ? gemv_strip_kernel<true, true, 1, false, true, 2> : gemv_strip_kernel<false, true, 1, false, true, 2>;
         return check_cuda(cudaLaunchKernelEx(&cfg, kern, p), "gemv_strip_kernel launch");
     }
     if (fast) {
