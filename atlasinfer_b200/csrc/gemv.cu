@@ -358,19 +358,33 @@ __global__ void __launch_bounds__((MT == 1 ? GS_MAX_WARPS : GS_WARPS2) * 32, 2) 
 
 constexpr int GS_STAGE_MAX_BYTES = 48 * 1024;   // staged fp16 activations per CTA, at most (two CTAs per SM)
 
+// Whether a CTA serves two strips.  Pairs halve the CTAs, so the last wave must not be much emptier than the others; they
+// save the set-up of a warp, which counts while a warp has at most one and a half chunks of K, and half of the conversion
+// of bf16 rows, which counts a little longer; with fewer than 12 chunks the small CTAs of single strips fill the SMs
+// better.  Time of single strips over pairs at 1 and 8 rows, fp16 and bf16 (rows x K, waves of pairs):
+//   22016 x 4096, 2.3: 1.06 1.05 1.08 1.14     18432 x 6144, 1.9: 1.08 1.08 1.11 1.14     9472 x 4096, 1.0: 1.08 1.13 1.14 1.21
+//   18432 x 3072, 1.9: 1.13 1.12 1.12 1.16     12288 x 5120, 1.3: 0.91 0.90 0.97 0.97    14336 x 7168, 1.5: 0.94 0.98 0.97 1.01
+//   57344 x 8192, 6.1: 0.98 1.00 1.02 1.06     24576 x 7168, 2.6: 0.99 0.99 1.01 1.05    16384 x 11008, 1.7: 0.98 1.04 0.97 1.04
+//   12288 x 2048, 1.3: 0.90 0.93 0.92 0.97      9472 x 2048, 1.0: 0.88 0.90 0.91 0.97
+bool strip_pairs_pay(int64_t pairs, int n_chunks, bool bf16) {
+    static thread_local int dev_cached = -1, sms = 148;
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev != dev_cached) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 148;
+        dev_cached = dev;
+    }
+    const int64_t places = 2 * sms, waves = ceil_div_i64(pairs, places);
+    const int64_t percent = 100 * pairs / (waves * places);   // of the places of all waves that have a CTA
+    return n_chunks >= 12 && n_chunks <= (bf16 ? 32 : 24) && (percent >= 85 || (waves >= 3 && percent >= 75));
+}
+
 template <int MT>
 int launch_gemv_strip(const GemvParams &p, bool vec, cudaStream_t st) {
     const int max_warps = MT == 1 ? GS_MAX_WARPS : GS_WARPS2;
     int nwarps = p.n_chunks < max_warps ? p.n_chunks : max_warps;
     const bool fast = vec && (p.k_tiles & 3) == 0 && p.bs_shift >= 6;   // whole chunks, blocks of whole tiles
     const int64_t strips = ceil_div_i64(p.n_rows, 16);
-    // Strip pairs pay where a warp has little of K to spread its set-up over (at most one 256-column chunk: 12288 x 4096
-    // 15.7 -> 14.6 us at one bf16 row, 18.1 -> 16.3 at eight; 22016 x 4096 24.4 -> 22.4 and 28.7 -> 25.4) and, for
-    // bf16, whose conversion they halve, over many waves of CTAs (57344 x 8192 96 -> 93, 110 -> 104; with fp16 rows
-    // 95 -> 96).  They lose where half the CTAs fill the SMs once and a little (10240 x 8192: 23 -> 26) or not at all
-    // (4096 x 4096: 6.0 -> 8.6).
-    const bool two = MT == 1 && fast && strips >= 4 * 148 &&
-                     (p.n_chunks <= GS_MAX_WARPS || (p.dtype == ATLAS_DTYPE_BF16 && strips >= 16 * 148));
+    const bool two = MT == 1 && fast && strip_pairs_pay((strips + 1) / 2, p.n_chunks, p.dtype == ATLAS_DTYPE_BF16);
     if (nwarps < 4 * MT * (two ? 2 : 1)) nwarps = 4 * MT * (two ? 2 : 1);  // the reduction needs 128 threads per MMA tile
     // one or two rows of bf16 activations are converted once per CTA into shared memory (measured at 1 / 2 / 4 / 8
     // rows: 3.7 / 3.5 / 3.1 / 2.6 TB/s staged against 3.4 / 3.3 / 3.3 / 3.1 converted per step)

@@ -72,8 +72,8 @@ def test_back_to_back_launches(cuda_device):
     aw.check_status(cuda_device)
 
 
-# strips served in pairs (many strips): an odd number of strips, ragged rows, one chunk of K for eight warps
-@pytest.mark.parametrize("n,k,bs", [(9473, 256, 128), (9472 + 16, 512, 64), (12288, 1024, 256)])
+# strips in pairs (the pairs fill the SMs, 12 chunks of K or more): an odd number of strips, ragged rows; and single ones
+@pytest.mark.parametrize("n,k,bs", [(9441, 4096, 64), (9460, 3072, 128), (9441, 4352, 256), (9473, 256, 128)])
 def test_strip_pairs(n, k, bs, cuda_device):
     _check(n, k, (1, 2, 3, 8), cuda_device, bs=bs, force="gemv")
     _check(n, k, (1,), cuda_device, bs=bs, thr=1.0, force="gemv")
