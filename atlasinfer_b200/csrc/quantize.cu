@@ -563,6 +563,10 @@ __global__ void __launch_bounds__(QT_THREADS, 5) quantize_fast_kernel(QuantParam
                 if (cnt < BS) sc = max(f2h_bits(h2f_bits((uint16_t)maxabs) * (1.0f / 127.0f)), eps_h);
                 if (t == 0) s_scale[b] = sc;
                 const float rsc = __frcp_rn(h2f_bits(sc));
+                // A NaN quotient is code 0.  It takes an infinity or a NaN among the values kept, which makes the scale
+                // infinite or NaN and every other quotient of the block 0 or NaN: such a block selects zero bytes
+                // instead of the low bytes of its (min/max-cleaned) sums, which costs the others nothing.
+                const uint32_t low_bytes = sc < 0x7c00u ? 0x4420u : 0x4444u;
                 uint8_t *db = s_dense;
                 const int e0 = b * BS + 2 * t;
                 const __half2 lim = __float2half2_rn(127.f), nlim = __float2half2_rn(-127.f), magic = __float2half2_rn(1536.f);
@@ -573,7 +577,7 @@ __global__ void __launch_bounds__(QT_THREADS, 5) quantize_fast_kernel(QuantParam
                     q = __hmax2(__hmin2(q, lim), nlim);
                     q = __hadd2(q, magic);
                     const uint32_t bits = *reinterpret_cast<uint32_t *>(&q);
-                    *reinterpret_cast<uint16_t *>(db + dense_byte(e0 + j * 8)) = (uint16_t)__byte_perm(bits, 0u, 0x4420);
+                    *reinterpret_cast<uint16_t *>(db + dense_byte(e0 + j * 8)) = (uint16_t)__byte_perm(bits, 0u, low_bytes);
                 }
                 if (any_out) {
 #pragma unroll

@@ -301,3 +301,34 @@ def test_quantize_fast_kernel_branches(bs, offset, sigma, thr, cuda_device):
         w[n // 2:n // 2 + 2 * bs] = offset   # constant blocks
         q = ab.quantize_tensor(w.to(cuda_device), bs, thr)
         assert_streams_equal(q, O.quantize(w, bs, thr), what=f"n {n} bs {bs} offset {offset} sigma {sigma} thr {thr}: ")
+
+
+# An infinity or a NaN among a block's values makes its scale infinite or NaN and all its codes 0.  (Non-finite weights
+# are outside the bit-exact contract: beside an infinity the finite values of a block become outliers here, and a NaN
+# scale has another sign bit than the oracle's; positions, codes and finite scales are compared.)
+@pytest.mark.parametrize("bs", [32, 64, 128, 256])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_quantize_non_finite_codes_are_zero(bs, value, cuda_device):
+    w = config_weights(40, 1024, bs)
+    hit = torch.tensor([0, 7, 20, 20, 20 * 1024 // bs])                      # blocks; two values in block 20
+    w.view(-1)[hit * bs + torch.tensor([5, 3, 0, 1, bs - 1])] = value
+    q = ab.quantize_tensor(w.to(cuda_device), bs, 3.0)
+    o = O.quantize(w, bs, 3.0)
+    codes = torch.full((w.numel(),), 99, dtype=torch.int8)
+    keep = torch.ones(w.numel(), dtype=torch.bool)
+    keep[q.outlier_indices.cpu()] = False
+    codes[keep] = q.fp8_data.cpu()
+    want = torch.full((w.numel(),), 99, dtype=torch.int8)
+    keep_o = torch.ones(w.numel(), dtype=torch.bool)
+    keep_o[o.outlier_indices] = False
+    want[keep_o] = o.fp8_data
+    bad = torch.zeros(w.numel() // bs, dtype=torch.bool)
+    bad[hit] = True
+    codes, want, keep = (t.view(-1, bs) for t in (codes, want, keep))
+    assert torch.equal(codes[~bad], want[~bad])
+    assert bool((codes[bad][keep[bad]] == 0).all()) and bool((want[bad] == 0).all())
+    assert bool(keep.view(-1)[~torch.isfinite(w.view(-1))].all())            # the non-finite values themselves are kept
+    if value != value:
+        assert torch.equal(codes, want) and torch.equal(q.outlier_indices.cpu(), o.outlier_indices)
+    sc, so = q.scale_factors.cpu(), o.scale_factors
+    assert torch.equal(torch.isnan(sc), torch.isnan(so)) and torch.equal(bits(sc[~torch.isnan(sc)]), bits(so[~torch.isnan(so)]))
