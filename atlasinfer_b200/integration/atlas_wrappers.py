@@ -55,10 +55,11 @@ def status_word(dev: torch.device) -> torch.Tensor:
     index = dev.index
     if index is None:
         index = torch.cuda.current_device()
-    t = _status_words.get(index)
+    key = (dev.type, index)   # (the word of a CPU device must not pass for a GPU's)
+    t = _status_words.get(key)
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=dev)
-        _status_words[index] = t
+        _status_words[key] = t
     return t
 
 

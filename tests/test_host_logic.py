@@ -144,3 +144,22 @@ def test_shard_rows_equals_quantizing_the_shard():
     assert sum(len(sharding.layers_for_rank(10, 4, r)) for r in range(4)) == 10
     with pytest.raises(ValueError):
         sharding.shard_rows(whole, 10, 100)
+
+
+def test_status_word_of_a_cpu_device_is_not_the_gpus(monkeypatch):
+    # the kernels write the word through the pointer they are given: a host tensor must never be handed out for a GPU
+    made = []
+
+    def zeros(*size, dtype=None, device=None):
+        made.append(torch.device(device))
+        return types.SimpleNamespace(device=torch.device(device))
+
+    monkeypatch.setattr(atlas_wrappers, "_status_words", {})
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(atlas_wrappers.torch, "zeros", zeros)
+    assert atlas_wrappers.status_word(torch.device("cpu")).device.type == "cpu"
+    word = atlas_wrappers.status_word(torch.device("cuda", 0))
+    assert word.device == torch.device("cuda", 0)
+    assert atlas_wrappers.status_word(torch.device("cuda")) is word
+    assert atlas_wrappers.status_word(torch.device("cuda", 1)) is not word
+    assert atlas_wrappers.status_word(torch.device("cpu")).device.type == "cpu"
