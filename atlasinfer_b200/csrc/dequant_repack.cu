@@ -50,7 +50,9 @@ struct Span {
 };
 
 // Stages the span [span0, span1): mask, prefix counts and codes.  Nothing outside codes[0, n_codes) and oidx[0, n_out)
-// is read.
+// is read, whatever oidx holds; if it is not ascending (a damaged file) the values are arbitrary, but hi >= lo keeps the
+// staged length within the span and, as every bit of the mask stands for an index in [lo, hi), the outliers read within
+// [lo, hi) too.
 __device__ __forceinline__ void stage_span(Span &s, const int8_t *codes, int64_t n_codes, const int64_t *oidx,
                                            int64_t n_out, int64_t span0, int64_t span1) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -60,7 +62,7 @@ __device__ __forceinline__ void stage_span(Span &s, const int8_t *codes, int64_t
         if (lane == 0) (warp == 0 ? s.lo : s.hi) = r;
     }
     __syncthreads();
-    const int64_t lo = s.lo, hi = s.hi;
+    const int64_t lo = s.lo, hi = max(lo, s.hi);
     for (int64_t i = lo + tid; i < hi; i += DQ_THREADS) {
         const int64_t p = __ldg(oidx + i) - span0;
         if (p >= 0 && p < DQ_SPAN) atomicOr(&s.mask[p >> 5], 1u << (p & 31));
@@ -291,9 +293,22 @@ __global__ void __launch_bounds__(DQ_THREADS) repack_kernel(const __grid_constan
         const int total = (int)(sh.strip.row_at[16] - first);
         if (t.row_ptr && tid < 17 && strip * 16 + tid <= t.n_rows && (tid < 16 || strip * 16 + 16 == t.n_rows))
             t.row_ptr[strip * 16 + tid] = (int32_t)sh.strip.row_at[tid];
-        if (total <= RP_STRIP_CAP) {
-            for (int i = tid; i < total; i += DQ_THREADS) sh.strip.col[i] = (uint32_t)(__ldg(t.oidx + first + i) % t.n_cols);
-            __syncthreads();
+        // The ranks below are a permutation, and what the linear kernels index with the entries lies in the strip, only if
+        // the strip's positions ascend and lie in the rows that the searches gave them.  A strip of which that is not true
+        // (a damaged file) gets an empty list.  (A row's first column replaces a 64-bit remainder, so the check is free.)
+        int bad = tid < 16 && sh.strip.row_at[tid + 1] < sh.strip.row_at[tid];
+        for (int i = tid; i < total; i += DQ_THREADS) {
+            int row = 0;
+#pragma unroll
+            for (int r = 1; r < 16; ++r) row += sh.strip.row_at[r] - first <= i;
+            const int64_t at = __ldg(t.oidx + first + i), col = at - (strip * 16 + row) * t.n_cols;
+            bad |= col < 0 || col >= t.n_cols || (i > 0 && __ldg(t.oidx + first + i - 1) >= at);
+            if (i < RP_STRIP_CAP) sh.strip.col[i] = (uint32_t)col;
+        }
+        if (__syncthreads_or(bad)) {
+            const int n_chunks = (int)(t.n_cols >> 6);
+            for (int c = tid; c <= n_chunks; c += DQ_THREADS) t.chunk_ptr[strip * (n_chunks + 1) + c] = (int32_t)(t.entry_base + first);
+        } else if (total <= RP_STRIP_CAP) {
             write_strip(t, strip, sh.strip, [&](int i) { return (int64_t)sh.strip.col[i]; });
         } else {
             write_strip(t, strip, sh.strip, [&](int i) { return __ldg(t.oidx + first + i) % t.n_cols; });
