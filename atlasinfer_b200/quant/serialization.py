@@ -105,16 +105,32 @@ def _load_array(path: str, meta: dict, device) -> torch.Tensor:
     return t.to(device)
 
 
+def _check_record(path: str, name: str, q: QuantizedTensor) -> None:
+    """Refuse streams that do not belong together: the kernels find an element's code by counting the outliers before it."""
+    numel, bs = q.original_shape.numel(), q.block_size
+    blocks = -(-numel // bs) if bs > 0 else -1
+    idx = q.outlier_indices
+    if (q.scale_factors.numel() != blocks or q.fp16_outliers.numel() != idx.numel()
+            or q.fp8_data.numel() + idx.numel() != blocks * bs):
+        raise ValueError(f"{path}: record {name!r}: stream lengths do not fit shape {tuple(q.original_shape)} and block size {bs}")
+    if idx.numel() and not (0 <= int(idx[0]) and int(idx[-1]) < blocks * bs and bool((idx[1:] > idx[:-1]).all())):
+        raise ValueError(f"{path}: record {name!r}: outlier indices do not ascend inside the tensor")
+
+
 def load_quantized_state(path: str, device="cpu", names=None) -> Dict[str, Tuple[QuantizedTensor, Optional[torch.Tensor]]]:
-    """Read records written by ``save_quantized_state``: name -> (QuantizedTensor, bias or None) on ``device``."""
+    """Read records written by ``save_quantized_state``: name -> (QuantizedTensor, bias or None) on ``device``.
+
+    ``ValueError`` for a record whose streams do not belong together (a damaged file)."""
     header = read_header(path)
     out = {}
     for name, entry in header["records"].items():
         if names is not None and name not in names:
             continue
         arr = entry["arrays"]
-        q = QuantizedTensor(*(_load_array(path, arr[f], device) for f, _ in _FIELDS),
+        q = QuantizedTensor(*(_load_array(path, arr[f], "cpu") for f, _ in _FIELDS),
                             torch.Size(entry["shape"]), int(entry["block_size"]))
+        _check_record(path, name, q)
+        q = q.to(torch.device(device))
         bias = _load_array(path, arr["bias"], device) if "bias" in arr else None
         out[name] = (q, bias)
     return out

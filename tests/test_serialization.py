@@ -1,5 +1,6 @@
 """On-disk format of QuantizedTensor records (runs without a GPU)."""
 import numpy as np
+import pytest
 import torch
 import torch.nn as nn
 
@@ -78,3 +79,27 @@ def test_model_level_save_and_load(tmp_path):
         if bias is not None:
             assert torch.equal(bits(mod.bias), bits(bias))
     assert not any(isinstance(m, nn.Linear) for m in fresh.modules())
+
+
+@pytest.mark.parametrize("damage", ["swapped", "repeated", "negative", "beyond", "short_scales", "short_codes", "short_values"])
+def test_damaged_streams_are_refused(tmp_path, damage):
+    q = _q(16, 256, 8, bs=64)
+    idx = q.outlier_indices.clone()
+    assert idx.numel() > 4
+    if damage == "swapped":
+        idx[1], idx[2] = int(idx[2]), int(idx[1])
+    elif damage == "repeated":
+        idx[2] = idx[1]
+    elif damage == "negative":
+        idx[0] = -1
+    elif damage == "beyond":
+        idx[-1] = 16 * 256
+    bad = q._replace(outlier_indices=idx)
+    if damage.startswith("short"):
+        field = {"scales": "scale_factors", "codes": "fp8_data", "values": "fp16_outliers"}[damage[6:]]
+        bad = q._replace(**{field: getattr(q, field)[:-1]})
+    path = str(tmp_path / "w.atlq")
+    ab.save_quantized_state(path, {"good": q, "bad": bad})
+    with pytest.raises(ValueError, match="bad"):
+        ab.load_quantized_state(path)
+    assert_streams_equal(ab.load_quantized_state(path, names=["good"])["good"][0], q)
