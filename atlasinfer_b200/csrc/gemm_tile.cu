@@ -28,8 +28,10 @@
 // at 128 rows 66 -> 27; 12288 x 4096 at 128 rows 29 -> 31.  Issue slots are 40 % used; the rest is the chain of a k-tile
 // through one A tile (rebuild, fence, MMA, commit), of which four are in flight per SM.
 //
-// Every mbarrier wait is bounded; when one runs out the CTA sets the caller's status word, waits (bounded) for its own
-// copies, takes part in the cluster barriers, frees its TMEM and returns.
+// Every mbarrier wait is bounded; when one runs out the CTA sets the caller's status word.  The two producers and the
+// MMA thread end with a bounded wait for what they have issued themselves (on the normal path it has arrived long before
+// the epilogue), so that the CTA takes part in the cluster barriers, frees its TMEM and returns with nothing in flight,
+// whichever warp gave up and however far the producers were.
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -150,8 +152,8 @@ tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
                 mbar_arrive_expect_tx(bar, SM::X_BYTES);
                 tma_load_2d(base + SM::OFF_X + (kt % XS) * SM::X_BYTES, &x_map, (kt_begin + kt) * TL_BK, 0, bar);
             }
-            if (kt < KT)
-                for (int i = max(0, kt - XS); i < kt; ++i) mbar_wait<100>(p.x_bf16 ? x_land(i % XS) : x_full(i % XS), (uint32_t)((i / XS) & 1));
+            // whatever happens to the other warps from here on, no copy of this CTA is left in flight
+            for (int i = max(0, kt - XS); i < kt; ++i) mbar_wait<100>(p.x_bf16 ? x_land(i % XS) : x_full(i % XS), (uint32_t)((i / XS) & 1));
         }
     } else if (warp == 3) {
         // ------------------------------ bf16 -> fp16 in place ------------------------------
@@ -192,14 +194,14 @@ tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
                     bulk_load_1d(base + SM::OFF_S + slot * TL_S_BYTES,
                                  p.scales_t + ((size_t)blockIdx.x * p.blocks_per_row + (kt_begin + kt) / p.bs_tiles) * 128, TL_S_BYTES, full_c(slot));
             }
-            if (kt < KT)
-                for (int i = max(0, kt - CS); i < kt; ++i) mbar_wait<100>(full_c(i % CS), (uint32_t)((i / CS) & 1));
+            for (int i = max(0, kt - CS); i < kt; ++i) mbar_wait<100>(full_c(i % CS), (uint32_t)((i / CS) & 1));
         }
     } else if (warp == 1) {
         // ------------------------------ MMA ------------------------------
         if (lane == 0) {
             const uint64_t da0 = make_smem_desc(base + SM::OFF_A), db0 = make_smem_desc(base + SM::OFF_X);
             bool ok = true;
+            int issued = 0;
             for (int kt = 0; kt < KT && ok; ++kt) {
                 ok = mbar_wait(x_full(kt % XS), (uint32_t)((kt / XS) & 1)) && mbar_wait(ready_bar(kt), (uint32_t)((kt >> 1) & 1));
                 if (!ok || ((kt & 7) == 7 && *s_abort)) { ok = false; break; }
@@ -210,8 +212,11 @@ tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
                 for (int k = 0; k < 4; ++k)
                     umma_f16_ss(tmem_base, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), tl_idesc<BN>(), (kt | k) != 0);
                 umma_commit(done_bar(kt));   // frees the A tile and the activation slot
+                issued = kt + 1;
             }
             if (!ok) *s_abort = 1;
+            // nor an MMA: tensor memory is freed below also when a dequantizer has given up
+            if (issued > 0) mbar_wait<20>(done_bar(issued - 1), done_par(issued - 1));
         }
     } else {
         // ------------------------------ dequantizers ------------------------------
