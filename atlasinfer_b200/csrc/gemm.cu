@@ -33,7 +33,8 @@
 //   warps 3-18  epilogue: tcgen05.ld of their TMEM lane quarter (four warps per quarter, a quarter of
 //               the columns each), + bias, convert, transpose through shared memory, 16-byte stores
 // Every mbarrier wait is bounded; if one runs out the CTA sets the caller's status word,
-// skips the rest of its work, frees its TMEM and returns.
+// skips the rest of its work, gives its own copies a millisecond to land, frees its TMEM
+// and returns.
 //
 // bf16 activations are first converted to fp16 into the workspace, 16 bytes per thread (the MMA takes both operands as
 // fp16; |x| > 65504 saturates).  Two bytes at a time that kernel cost 5 % of a 2048-token linear (965 -> 1020 TFLOP/s at
@@ -327,6 +328,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
             }
             if (!ok) *s_abort = 1;
             umma_commit(accfull_bar);  // arrives when every MMA issued so far is complete
+            if (!ok) mbar_wait<20>(accfull_bar, 0);   // (the dequantizers may have stopped waiting for it)
         }
     } else {
         // ------------------------------ dequantizers, then epilogue ------------------------------
@@ -568,8 +570,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    if (tid == 0 && *s_abort && p.error_flag) atomicExch(p.error_flag, 1);
+    if (*s_abort) {
+        // a wait ran out: copies may still be on their way into this CTA's shared memory; give them time to land
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+        if (tid == 0 && p.error_flag) atomicExch(p.error_flag, 1);
+    }
     if (warp == 1) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
     }
 }
