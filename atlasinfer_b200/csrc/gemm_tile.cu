@@ -28,10 +28,9 @@
 // at 128 rows 66 -> 27; 12288 x 4096 at 128 rows 29 -> 31.  Issue slots are 40 % used; the rest is the chain of a k-tile
 // through one A tile (rebuild, fence, MMA, commit), of which four are in flight per SM.
 //
-// Every mbarrier wait is bounded; when one runs out the CTA sets the caller's status word.  The two producers and the
-// MMA thread end with a bounded wait for what they have issued themselves (on the normal path it has arrived long before
-// the epilogue), so that the CTA takes part in the cluster barriers, frees its TMEM and returns with nothing in flight,
-// whichever warp gave up and however far the producers were.
+// Every mbarrier wait is bounded; when one runs out the CTA sets the caller's status word, the producers and the MMA
+// thread wait (bounded) for what they have issued, and the CTA takes part in the cluster barriers, frees its TMEM and
+// returns with nothing in flight.  (The same waits on the normal path as well cost 0.3 us a launch.)
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -140,20 +139,19 @@ tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
     __syncthreads();
     tcgen05_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    int issued = 0;   // k-tiles that this thread (either producer, the MMA thread) has asked for
 
     if (warp == 0) {
         // ------------------------------ activations ------------------------------
         asm volatile("griddepcontrol.wait;" ::: "memory");   // x comes from earlier kernels of the stream
         if (lane == 0) {
-            int kt = 0;
-            for (; kt < KT && !*s_abort; ++kt) {
+            for (int kt = 0; kt < KT && !*s_abort; ++kt) {
                 if (kt >= XS && !mbar_wait<20>(done_bar(kt - XS), done_par(kt - XS))) { *s_abort = 1; break; }
                 const uint32_t bar = p.x_bf16 ? x_land(kt % XS) : x_full(kt % XS);
                 mbar_arrive_expect_tx(bar, SM::X_BYTES);
                 tma_load_2d(base + SM::OFF_X + (kt % XS) * SM::X_BYTES, &x_map, (kt_begin + kt) * TL_BK, 0, bar);
+                issued = kt + 1;
             }
-            // whatever happens to the other warps from here on, no copy of this CTA is left in flight
-            for (int i = max(0, kt - XS); i < kt; ++i) mbar_wait<100>(p.x_bf16 ? x_land(i % XS) : x_full(i % XS), (uint32_t)((i / XS) & 1));
         }
     } else if (warp == 3) {
         // ------------------------------ bf16 -> fp16 in place ------------------------------
@@ -183,8 +181,7 @@ tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
         // ------------------------------ codes and scales ------------------------------
         if (lane == 0) {
             const int64_t crow0 = (int64_t)blockIdx.x * p.k_tiles + kt_begin;   // code tiles are runs of 128 rows of the map
-            int kt = 0;
-            for (; kt < KT; ++kt) {
+            for (int kt = 0; kt < KT; ++kt) {
                 const int slot = kt % CS, round = kt / CS;
                 if (round > 0 && !mbar_wait<40>(empty_c(slot), (uint32_t)((round - 1) & 1))) { *s_abort = 1; break; }
                 if (*s_abort) break;
@@ -193,15 +190,14 @@ tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
                 if (p.bs_tiles)
                     bulk_load_1d(base + SM::OFF_S + slot * TL_S_BYTES,
                                  p.scales_t + ((size_t)blockIdx.x * p.blocks_per_row + (kt_begin + kt) / p.bs_tiles) * 128, TL_S_BYTES, full_c(slot));
+                issued = kt + 1;
             }
-            for (int i = max(0, kt - CS); i < kt; ++i) mbar_wait<100>(full_c(i % CS), (uint32_t)((i / CS) & 1));
         }
     } else if (warp == 1) {
         // ------------------------------ MMA ------------------------------
         if (lane == 0) {
             const uint64_t da0 = make_smem_desc(base + SM::OFF_A), db0 = make_smem_desc(base + SM::OFF_X);
             bool ok = true;
-            int issued = 0;
             for (int kt = 0; kt < KT && ok; ++kt) {
                 ok = mbar_wait(x_full(kt % XS), (uint32_t)((kt / XS) & 1)) && mbar_wait(ready_bar(kt), (uint32_t)((kt >> 1) & 1));
                 if (!ok || ((kt & 7) == 7 && *s_abort)) { ok = false; break; }
@@ -215,8 +211,6 @@ tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
                 issued = kt + 1;
             }
             if (!ok) *s_abort = 1;
-            // nor an MMA: tensor memory is freed below also when a dequantizer has given up
-            if (issued > 0) mbar_wait<20>(done_bar(issued - 1), done_par(issued - 1));
         }
     } else {
         // ------------------------------ dequantizers ------------------------------
@@ -319,6 +313,15 @@ tile_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
     }
 
     __syncthreads();
+    if (*s_abort) {
+        // a wait ran out somewhere: no copy may land, and no MMA run, once this CTA has gone, however far their issuers were
+        if (tid == 0)
+            for (int i = max(0, issued - XS); i < issued; ++i) mbar_wait<100>(p.x_bf16 ? x_land(i % XS) : x_full(i % XS), (uint32_t)((i / XS) & 1));
+        if (tid == 2 * 32)
+            for (int i = max(0, issued - CS); i < issued; ++i) mbar_wait<100>(full_c(i % CS), (uint32_t)((i / CS) & 1));
+        if (tid == 1 * 32 && issued > 0) mbar_wait<100>(done_bar(issued - 1), done_par(issued - 1));
+        __syncthreads();
+    }
     tcgen05_fence_after();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(SM::TMEM_COLS) : "memory");
