@@ -52,14 +52,12 @@ _status_words = {}
 
 def status_word(dev: torch.device) -> torch.Tensor:
     """The device int32 kernels set non-zero when a bounded wait ran out (one per device)."""
-    index = dev.index
-    if index is None:
-        index = torch.cuda.current_device()
-    key = (dev.type, index)   # (the word of a CPU device must not pass for a GPU's)
-    t = _status_words.get(key)
+    t = _status_words.get(dev)   # (a CPU device is a key of its own: its word must not pass for a GPU's)
     if t is None:
+        if dev.type == "cuda" and dev.index is None:
+            return status_word(torch.device("cuda", torch.cuda.current_device()))
         t = torch.zeros(1, dtype=torch.int32, device=dev)
-        _status_words[key] = t
+        _status_words[dev] = t
     return t
 
 
