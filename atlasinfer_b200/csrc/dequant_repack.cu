@@ -233,7 +233,7 @@ union RepackShared {
 
 // entries of [lo, hi) (offsets into the strip's list, one row, ascending columns) with column < key
 template <class ColAt>
-__device__ __forceinline__ int count_below(const ColAt &col_at, int lo, int hi, int64_t key) {
+__device__ __forceinline__ int count_below(const ColAt &col_at, int lo, int hi, uint32_t key) {
     const int base = lo;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
@@ -254,17 +254,17 @@ __device__ __forceinline__ void write_strip(const RepackTensor &t, int64_t strip
         int row = 0;
 #pragma unroll
         for (int r = 1; r < 16; ++r) row += s.row_at[r] - first <= i;
-        const int64_t col = col_at(i);
+        const uint32_t col = col_at(i);
         int rank = 0;
         for (int r = 0; r < 16; ++r)   // rows above: columns up to and with this one; this row and below: columns before it
-            rank += count_below(col_at, (int)(s.row_at[r] - first), (int)(s.row_at[r + 1] - first), col + (r < row ? 1 : 0));
-        t.entries[first + rank] = (uint32_t)row << 24 | (uint32_t)col;
+            rank += count_below(col_at, (int)(s.row_at[r] - first), (int)(s.row_at[r + 1] - first), col + (r < row ? 1u : 0u));
+        t.entries[first + rank] = (uint32_t)row << 24 | col;
         t.vals_sorted[first + rank] = __ldg(t.ovals + first + i);
     }
     for (int c = threadIdx.x; c <= n_chunks; c += DQ_THREADS) {
         int count = 0;
         for (int r = 0; r < 16; ++r)
-            count += count_below(col_at, (int)(s.row_at[r] - first), (int)(s.row_at[r + 1] - first), (int64_t)c * 64);
+            count += count_below(col_at, (int)(s.row_at[r] - first), (int)(s.row_at[r + 1] - first), (uint32_t)c * 64u);
         t.chunk_ptr[strip * (n_chunks + 1) + c] = (int32_t)(t.entry_base + first + count);
     }
 }
@@ -294,24 +294,28 @@ __global__ void __launch_bounds__(DQ_THREADS) repack_kernel(const __grid_constan
         if (t.row_ptr && tid < 17 && strip * 16 + tid <= t.n_rows && (tid < 16 || strip * 16 + 16 == t.n_rows))
             t.row_ptr[strip * 16 + tid] = (int32_t)sh.strip.row_at[tid];
         // The ranks below are a permutation, and what the linear kernels index with the entries lies in the strip, only if
-        // the strip's positions ascend and lie in the rows that the searches gave them.  A strip of which that is not true
-        // (a damaged file) gets an empty list.  (A row's first column replaces a 64-bit remainder, so the check is free.)
-        int bad = tid < 16 && sh.strip.row_at[tid + 1] < sh.strip.row_at[tid];
+        // the strip's positions ascend and its rows begin where the searches say.  A strip of which that is not true (a
+        // damaged file) gets an empty list.
+        const int64_t strip0 = strip * 16 * t.n_cols, strip1 = min(strip * 16 + 16, t.n_rows) * t.n_cols;
+        const uint32_t n_cols = (uint32_t)t.n_cols;   // (a strip has at most 2^28 positions)
+        int bad = 0;
+        if (tid < 17) {
+            const int64_t at = sh.strip.row_at[tid], end = sh.strip.row_at[16], key = min(strip0 + tid * t.n_cols, strip1);
+            bad = at < first || at > end || (tid < 16 && sh.strip.row_at[tid + 1] < at);
+            if (!bad) bad = (at > first && __ldg(t.oidx + at - 1) >= key) || (at < end && __ldg(t.oidx + at) < key);
+        }
         for (int i = tid; i < total; i += DQ_THREADS) {
-            int row = 0;
-#pragma unroll
-            for (int r = 1; r < 16; ++r) row += sh.strip.row_at[r] - first <= i;
-            const int64_t at = __ldg(t.oidx + first + i), col = at - (strip * 16 + row) * t.n_cols;
-            bad |= col < 0 || col >= t.n_cols || (i > 0 && __ldg(t.oidx + first + i - 1) >= at);
-            if (i < RP_STRIP_CAP) sh.strip.col[i] = (uint32_t)col;
+            const int64_t *at = t.oidx + first + i;
+            bad |= i > 0 && __ldg(at - 1) >= __ldg(at);
+            if (i < RP_STRIP_CAP) sh.strip.col[i] = (uint32_t)(__ldg(at) - strip0) % n_cols;
         }
         if (__syncthreads_or(bad)) {
-            const int n_chunks = (int)(t.n_cols >> 6);
+            const int n_chunks = (int)(n_cols >> 6);
             for (int c = tid; c <= n_chunks; c += DQ_THREADS) t.chunk_ptr[strip * (n_chunks + 1) + c] = (int32_t)(t.entry_base + first);
         } else if (total <= RP_STRIP_CAP) {
-            write_strip(t, strip, sh.strip, [&](int i) { return (int64_t)sh.strip.col[i]; });
+            write_strip(t, strip, sh.strip, [&](int i) { return sh.strip.col[i]; });
         } else {
-            write_strip(t, strip, sh.strip, [&](int i) { return __ldg(t.oidx + first + i) % t.n_cols; });
+            write_strip(t, strip, sh.strip, [&](int i) { return (uint32_t)(__ldg(t.oidx + first + i) - strip0) % n_cols; });
         }
         return;
     }
