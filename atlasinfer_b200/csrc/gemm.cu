@@ -757,8 +757,8 @@ cudaLaunchConfig_t pdl_config(dim3 grid, dim3 block, size_t smem, cudaStream_t s
     return cfg;
 }
 
-// tokens per tile for a batch of m rows (up to 128 rows that are not gathered go to the kernel in gemm_tile.cu)
-int gemm_bn_for(int64_t m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 256); }
+// tokens per tile for a batch of m rows
+int gemm_bn_for(int64_t m) { return m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256)); }
 
 // K slices (one CTA per SM, `tiles` output tiles).
 // Decode-sized tiles: the count that minimises waves x (k-tiles per CTA + the fixed cost of a CTA, about 12 k-tiles'
@@ -768,6 +768,7 @@ int gemm_bn_for(int64_t m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 256); }
 // otherwise: 4096 x 11008 at 301 tokens is 64 tiles.
 int gemm_splits_for(int64_t m, int64_t n_rows, int64_t n_cols, int sms) {
     const int bn = gemm_bn_for(m);
+    if (bn == 128) return 1;   // (few row tiles at 65 to 128 rows: the kernel in gemm_tile.cu slices K)
     const int64_t tiles = ceil_div_i64(n_rows, GM_BM) * ceil_div_i64(m, bn);
     const int k_tiles = (int)(n_cols / 64);
     int best = 1;
@@ -782,6 +783,37 @@ int gemm_splits_for(int64_t m, int64_t n_rows, int64_t n_cols, int sms) {
     return best;
 }
 
+// bf16 rows of decode-sized token tiles are converted in the kernel when the weight is small: one more kernel in the chain
+// then costs more than the conversion's share of the producer warp over the few stages of a CTA
+bool gemm_converts(int64_t m, int64_t n_rows, int64_t n_cols) { return m <= 64 && n_rows * n_cols <= ((int64_t)32 << 20); }
+
+// About how long this file's kernels take for at most 128 rows, in us; fitted to the same shapes as the model of
+// plan_tile.  Where this kernel is the faster one: few row tiles with a long K, of which it can cut 16 slices (1024 x 8192,
+// 32 bf16 rows: 10.9 us, the kernel in gemm_tile.cu 13.7), and one full wave of its CTAs at 65 to 128 rows, which needs no
+// clusters and no sum over shared memory (12288 x 4096, 128 fp16 rows: 29.5 us, there 30.9).
+double gemm_us(int64_t m, int64_t n_rows, int64_t n_cols, bool bf16, bool can_convert, bool aligned, int sms) {
+    const int64_t tiles = ceil_div_i64(n_rows, GM_BM);
+    const int splits = gemm_splits_for(m, n_rows, n_cols, sms);
+    const double waves = (double)ceil_div_i64(tiles * splits, sms), kt = (double)ceil_div_i64(n_cols / 64, splits);
+    // output rows on no 16-byte boundary are stored by elements, in this kernel or, with K slices, in the second one
+    const double ragged = aligned || splits > 1 ? 0. : .045 * (double)m;
+    const double copy = bf16 ? copy_us(m, n_cols / 64) : 0.;
+    if (m > 64) return waves * (.375 * kt + 6. + ragged) - 3.3 + (bf16 ? .5 + copy : 0.);
+    double per_kt = .39, per_wave = 3.3 + ragged, once = .45;
+    if (can_convert && gemm_converts(m, n_rows, n_cols)) {
+        per_kt += m <= 32 ? .105 : .25;
+        per_wave -= m <= 32 ? .3 : .9;
+    } else if (bf16) {
+        once += 1. + copy;
+    }
+    if (splits > 1) once += .3 + 3e-6 * splits * (double)m * (double)n_rows + (aligned ? 0. : 9e-6 * (double)m * (double)n_rows);   // the second kernel
+    double us = waves * (per_kt * kt + per_wave) + once;
+    if (splits == 16) us *= 1.12;
+    // (nearly all SMs in one wave of short slices: the second kernel and the next launch's first CTAs get in the way)
+    if (splits >= 4 && tiles * splits <= sms && tiles * splits > sms * 92 / 100) us *= 1.3;
+    return us;
+}
+
 int gemm_sm_count() {
     static thread_local int dev_cached = -1, sms = 0;
     int dev = 0;
@@ -791,6 +823,34 @@ int gemm_sm_count() {
         dev_cached = dev;
     }
     return sms;
+}
+
+// Up to 128 rows: whichever of the two kernels the models expect to be faster, and how.  `shape` decides everything, so the
+// answers for the last shapes a thread has asked about are kept: evaluating the models takes 0.3 us of a call whose other
+// host work is 5 (60.3 -> 61.5 us for the six linears of a small layer's 128-token prompt).
+struct Shape {
+    int64_t m, n_rows, n_cols;
+    int sms, flags;   // 1: bf16, 2: a tensor map can take the rows, 4: output rows on 16-byte boundaries
+};
+struct Route {
+    bool tile;
+    TilePlan plan;
+};
+Route route_for(const Shape &shape) {
+    struct Entry { Shape shape; Route route; };
+    constexpr int KEPT = 64;
+    static thread_local Entry kept[KEPT] = {};
+    const uint64_t h = ((uint64_t)shape.m * 0x9e3779b97f4a7c15ull) ^ ((uint64_t)shape.n_rows * 0xc2b2ae3d27d4eb4full) ^
+                       ((uint64_t)shape.n_cols * 0x165667b19e3779f9ull) ^ ((uint64_t)shape.flags << 60);
+    Entry &e = kept[(h >> 58) % KEPT];
+    if (e.shape.m != shape.m || e.shape.n_rows != shape.n_rows || e.shape.n_cols != shape.n_cols || e.shape.sms != shape.sms ||
+        e.shape.flags != shape.flags) {
+        const bool bf16 = shape.flags & 1, tma_ok = shape.flags & 2, aligned = shape.flags & 4;
+        e.route.plan = plan_tile(shape.m, shape.n_rows, (int)(shape.n_cols / GM_BK), bf16 && tma_ok, bf16, shape.sms);
+        e.route.tile = e.route.plan.us <= gemm_us(shape.m, shape.n_rows, shape.n_cols, bf16, bf16 && tma_ok, aligned, shape.sms);
+        e.shape = shape;
+    }
+    return e.route;
 }
 
 template <int BN>
@@ -871,8 +931,17 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
     if (rc) return rc;
     if (m == 0) return ATLAS_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    // (the gathered form's arrival protocol lives in the kernels below)
-    const bool tile = !gather && m <= TILE_MAX_TOKENS;
+    // Rows the tensor map can take as they are: 16-byte aligned, fp16 -- or bf16 for decode-sized token tiles,
+    // which the kernel converts in shared memory.  Anything else is copied to a dense fp16 buffer first.
+    const bool tma_ok = ((uintptr_t)x & 15) == 0 && (ldx % 8) == 0;
+    const bool bf16 = dtype == ATLAS_DTYPE_BF16;
+    // (the gathered form's arrival protocol lives in the kernels of this file)
+    Route route = {};
+    if (!gather && m <= TILE_MAX_TOKENS) {
+        const bool aligned = n_rows % 8 == 0 && ldy % 8 == 0 && ((uintptr_t)y & 15) == 0;
+        route = route_for(Shape{m, n_rows, n_cols, gemm_sm_count(), (bf16 ? 1 : 0) | (tma_ok ? 2 : 0) | (aligned ? 4 : 0)});
+    }
+    const bool tile = route.tile;
     const int bn = tile ? tile_tokens_for(m) : gemm_bn_for(m);
 
     // operand B must be fp16 with rows on 16-byte boundaries for the tensor map
@@ -880,15 +949,8 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
     int64_t ldb = ldx;
     const size_t xcopy = ((size_t)m * (size_t)n_cols * 2 + 255) & ~(size_t)255;
     const unsigned int *wait_flags = gather ? gather->wait_flags : nullptr;
-    // Rows the tensor map can take as they are: 16-byte aligned, fp16 -- or bf16 for decode-sized token tiles,
-    // which the kernel converts in shared memory.  Anything else is copied to a dense fp16 buffer first.
-    const bool tma_ok = ((uintptr_t)x & 15) == 0 && (ldx % 8) == 0;
-    // (in the kernel when the weight is small: one more kernel in the chain then costs more than the conversion by one
-    // warp over the few stages of a CTA.  16 rows of 4096 x 4096: 11.2 us with the copy, 10.5 without; 64 rows: 14.0
-    // and 16.0, but 9.6 and 9.4 at 2048 x 2048)
-    const bool small_weight = n_rows * n_cols <= ((int64_t)(tile && bn == 64 ? 8 : 32) << 20);
-    const bool in_kernel_bf16 = dtype == ATLAS_DTYPE_BF16 && bn <= 64 && tma_ok && small_weight;
-    const bool direct = tma_ok && (dtype == ATLAS_DTYPE_F16 || in_kernel_bf16);
+    const bool in_kernel_bf16 = bf16 && tma_ok && (tile ? route.plan.convert : gemm_converts(m, n_rows, n_cols));
+    const bool direct = tma_ok && (!bf16 || in_kernel_bf16);
     // a gathered input is waited for by whichever kernel reads x first: the copy kernel, or the linear kernel itself
     const bool wait_in_copy = wait_flags && !direct;
     if (!direct) {
@@ -946,8 +1008,9 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
         t.bs_tiles = block_size % GM_BK == 0 ? block_size / GM_BK : 0;
         t.out_bf16 = dtype == ATLAS_DTYPE_BF16;
         t.x_bf16 = in_kernel_bf16;
+        t.splits = route.plan.splits;
         t.error_flag = status;
-        return launch_tile(x_map, c_map, t, gemm_sm_count(), st);
+        return launch_tile(x_map, c_map, t, st);
     }
     GemmParams p;
     p.tiles = tiles;
@@ -978,6 +1041,7 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
     switch (bn) {
         case 32: rc = launch_gemm<32>(x_map, c_map, p, st); break;
         case 64: rc = launch_gemm<64>(x_map, c_map, p, st); break;
+        case 128: rc = launch_gemm<128>(x_map, c_map, p, st); break;
         default: rc = launch_gemm<256>(x_map, c_map, p, st); break;
     }
     if (rc) return rc;

@@ -25,12 +25,12 @@
 //
 // Measured (us, launch chain, against gemm.cu's kernel that served these sizes before): 57344 x 8192 at 32 rows 201 -> 156,
 // 64 rows 207 -> 163; 8192 x 28672 at 32 rows 95 -> 76; 22016 x 4096 at 32 rows 52 -> 37, 128 rows 58 -> 48; 4096 x 11008
-// at 128 rows 66 -> 27; 12288 x 4096 at 128 rows 29 -> 31.  Issue slots are 40 % used; the rest is the chain of a k-tile
+// at 128 rows 66 -> 27 (where gemm.cu's kernel is the faster one, route_for in gemm.cu leaves it the call).  Issue slots are 40 % used; the rest is the chain of a k-tile
 // through one A tile (rebuild, fence, MMA, commit), of which four are in flight per SM.
 //
 // Every mbarrier wait is bounded; when one runs out the CTA sets the caller's status word, the producers and the MMA
 // thread wait (bounded) for what they have issued, and the CTA takes part in the cluster barriers, frees its TMEM and
-// returns with nothing in flight.  (The same waits on the normal path as well cost 0.3 us a launch.)
+// returns with nothing in flight.
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -392,27 +392,101 @@ int launch_tile_bn(const CUtensorMap &x_map, const CUtensorMap &c_map, const Til
     return check_cuda(cudaLaunchKernelEx(&cfg, tile_kernel<BN>, x_map, c_map, p), "tile_kernel launch");
 }
 
-// K slices of a tile (at most the portable cluster size): the count that minimises waves x (k-tiles per CTA + the fixed
-// cost of a CTA in k-tiles), with two CTAs per SM.  Clusters of 3, 5, 6 or 7 do not fill the SMs of a GPC, which leaves
-// about a tenth of the places empty: 96 tiles x 3 slices took 29 us where 96 x 2 took 22 (12288 x 4096, 16 tokens).
-int tile_splits_for(int64_t n_rows, int k_tiles, int sms) {
-    const int64_t tiles = ceil_div_i64(n_rows, TL_BM);
-    int best = 1;
-    int64_t best_cost = 0;
-    for (int s = 1; s <= 8 && s <= k_tiles; ++s) {
-        const int64_t places = (s & (s - 1)) == 0 ? 2 * sms : 2 * sms * 9 / 10;
-        const int64_t cost = ceil_div_i64(tiles * s, places) * (ceil_div_i64(k_tiles, s) + 8);
-        if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
+// Clusters of s CTAs that are resident at once, two CTAs per SM.  A cluster lies within one GPC, so the sizes that do not
+// divide a GPC's places leave some empty, and one cluster too many costs a whole second wave (K 2048 at 32 rows in four
+// slices: 71 row tiles 11.1 us, 72 tiles 16.4).  The occupancy query counts one CTA per SM for this kernel.  Two CTAs of a
+// cluster share an SM, so an even s takes the count of s / 2; an odd one lies between its neighbours.  Measured by stepping
+// the number of tiles on one B200: 92, 71, 56, 45, 37, 33 clusters of 3 .. 8; this gives 92, 71, 53, 45, 36, 33.  (Four
+// CTAs on two SMs lose a little of their count to placements on three.)
+struct Clusters {
+    int dev = -1;
+    int resident[9];
+};
+const int *resident_clusters(int sms) {
+    static thread_local Clusters cache;
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev == cache.dev) return cache.resident;
+    int raw[9];
+    bool ok = cudaFuncSetAttribute(tile_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TileSmem<128>::TOTAL) == cudaSuccess;
+    for (int s = 1; s <= 8 && ok; ++s) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 1;
+        attr.val.clusterDim.y = (unsigned)s;
+        attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(512, (unsigned)s, 1);
+        cfg.blockDim = dim3(TL_THREADS);
+        cfg.dynamicSmemBytes = TileSmem<128>::TOTAL;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        ok = cudaOccupancyMaxActiveClusters(&raw[s], tile_kernel<128>, &cfg) == cudaSuccess && raw[s] > 0;
     }
-    return best;
+    if (!ok) cudaGetLastError();   // (the launch that follows reports what is wrong)
+    int *n = cache.resident;
+    for (int s = 1; s <= 8; ++s) n[s] = !ok ? (s <= 2 ? 2 * sms / s : 2 * sms * 8 / (10 * s)) : (raw[1] > sms ? raw[s] : (s == 1 ? 2 * raw[1] : raw[s / 2]));
+    if (ok && raw[1] <= sms) {
+        n[4] = raw[2] * 24 / 25;
+        for (int s = 3; s <= 7; s += 2) n[s] = (n[s - 1] * (s - 1) + n[s + 1] * (s + 1)) * 48 / (100 * s);
+    }
+    for (int s = 1; s <= 8; ++s) n[s] = n[s] > 1 ? n[s] : 1;
+    cache.dev = ok ? dev : -1;
+    return cache.resident;
+}
+
+// us per k-tile and per CTA, for a CTA that has an SM to itself and for one of two that share it, by token tile.  Fitted
+// to 3760 shapes (1 to 448 row tiles, K 1024 to 28672, 17 to 128 rows, fp16 and bf16, each with 1 to 8 slices): what is
+// chosen by it takes 1.3 % longer than the best choice of kernel and slices, geometric mean.
+struct TileCost { int tokens; double alone_kt, alone, shared_kt, shared, convert_kt; };
+constexpr TileCost TILE_COST[] = {{16, .38, 3.1, .58, 4.4, .12}, {32, .405, 3.3, .60, 4.75, .16}, {64, .495, 3.2, .625, 5.7, .335},
+                                  {96, .47, 5.3, .61, 6.55, 0.}, {128, .485, 5.95, .68, 7.4, 0.}};
+
+double tile_us(const TileCost &c, int64_t tiles, int k_tiles, int s, bool convert, const int *resident, int sms) {
+    const int64_t ctas = tiles * s, places = (int64_t)resident[s] * s;
+    const int64_t full = ctas / places, rest = ctas % places;
+    const double kt = (double)ceil_div_i64(k_tiles, s), extra = convert ? c.convert_kt : 0.;
+    // f: how much of the last wave runs two to an SM.  CTAs of one slice spread over the SMs before they share.  Those of
+    // a cluster share while others stand empty, the more the fuller the chip is; clusters of two and four fit beside
+    // each other best; the longer they run the more it shows (the next launch has less of its work under this one's).
+    const double at = (double)rest / sms;
+    double f = s == 1 ? (at > 1. ? 1. : 0.) : (at - .213) / (s == 2 || s == 4 ? 1.5 : 1.);
+    if (s > 1 && kt > 16.) f *= 1. + (kt - 16.) / 80.;
+    f = f < 0. ? 0. : (f > 1. ? 1. : f);
+    const double sum = s > 2 ? 1.8e-5 * c.tokens * c.tokens * (s - 2) : 0.;   // the sum over the slices' tiles
+    const double shared = (c.shared_kt + extra) * kt + c.shared + sum, alone = (c.alone_kt + extra) * kt + c.alone;
+    // (without clusters a place is taken again as soon as one CTA ends, under the work of the other CTA of the SM)
+    const double us = (double)full * (s == 1 ? shared - c.shared : shared) + (rest ? f * shared + (1. - f) * alone : 0.);
+    // (clusters of seven never share their SMs evenly; clusters of a further wave wait for all the places they need)
+    return s == 7 || (s > 1 && full > 0) ? 1.04 * us : us;
 }
 
 }  // namespace
 
 int tile_tokens_for(int64_t m) { return m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 96 ? 96 : 128))); }
 
-int launch_tile(const CUtensorMap &x_map, const CUtensorMap &c_map, TileParams &p, int sms, cudaStream_t st) {
-    p.splits = tile_splits_for(p.n_rows, p.k_tiles, sms);
+// The slices (at most the portable cluster size) that take the least time by the model above.  What it corrects against
+// counting waves of 2 x 148 CTAs: 74 row tiles in four slices do not fit one wave (9472 x 2048, 32 fp16 rows: 16.7 us, in
+// two slices 11.0); many short CTAs share SMs (4096 x 1024, 64 fp16 rows: in eight slices 8.7 us, in four 6.9); one warp
+// converts bf16 slower than the rest of a CTA works (1024 x 8192, 64 rows: 19.4 us, with a copy kernel in front 13.4).
+TilePlan plan_tile(int64_t m, int64_t n_rows, int k_tiles, bool can_convert, bool needs_copy, int sms) {
+    const int bn = tile_tokens_for(m);
+    const TileCost *c = TILE_COST;
+    while (c->tokens != bn) ++c;
+    const int *resident = resident_clusters(sms);
+    const int64_t tiles = ceil_div_i64(n_rows, TL_BM);
+    TilePlan best = {1, false, 1e300};
+    for (int s = 1; s <= 8 && s <= k_tiles; ++s) {
+        if (can_convert && bn <= 64) {
+            const double us = tile_us(*c, tiles, k_tiles, s, true, resident, sms);
+            if (us < best.us) best = {s, true, us};
+        }
+        const double us = tile_us(*c, tiles, k_tiles, s, false, resident, sms) + (needs_copy ? copy_us(m, k_tiles) : 0.);
+        if (us < best.us) best = {s, false, us};
+    }
+    return best;
+}
+
+int launch_tile(const CUtensorMap &x_map, const CUtensorMap &c_map, const TileParams &p, cudaStream_t st) {
     switch (tile_tokens_for(p.m)) {
         case 16: return launch_tile_bn<16>(x_map, c_map, p, st);
         case 32: return launch_tile_bn<32>(x_map, c_map, p, st);

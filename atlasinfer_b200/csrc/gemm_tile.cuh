@@ -30,8 +30,21 @@ struct TileParams {
 // Rows of x the kernel takes, and tokens per tile for m of them.
 constexpr int TILE_MAX_TOKENS = 128;
 int tile_tokens_for(int64_t m);
+
+// How the kernel would run a shape, and about how long it would take.
+struct TilePlan {
+    int splits;      // K slices
+    bool convert;    // bf16 rows are converted in the kernel, not by a copy kernel in front of it
+    double us;
+};
+// A copy kernel in front of either kernel: one more launch in the chain, and its traffic.
+inline double copy_us(int64_t m, int64_t k_tiles) { return 1. + 5.1e-5 * (double)m * (double)k_tiles; }
+// can_convert: the rows are bf16 and a tensor map can take them as they are; needs_copy: a copy kernel makes them dense
+// fp16 unless the kernel converts.
+TilePlan plan_tile(int64_t m, int64_t n_rows, int k_tiles, bool can_convert, bool needs_copy, int sms);
+
 // x_map: boxes of 64 columns x tile_tokens_for(m) rows, 128-byte swizzle; c_map: the code tiles as 64-byte rows, boxes
 // of 128 rows, 64-byte swizzle.
-int launch_tile(const CUtensorMap &x_map, const CUtensorMap &c_map, TileParams &p, int sms, cudaStream_t st);
+int launch_tile(const CUtensorMap &x_map, const CUtensorMap &c_map, const TileParams &p, cudaStream_t st);
 
 }  // namespace atlas

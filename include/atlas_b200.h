@@ -200,10 +200,12 @@ ATLAS_API int atlas_repack_many(int count, const AtlasRepackItem *items, void *s
  * atlas_qlinear_gemm: larger batches (any m >= 1 accepted).  Code tiles and
  * activations come in by TMA and go through tcgen05.mma with fp32 accumulators
  * in tensor memory.  Up to 128 rows: the weights are rebuilt into shared memory
- * (token tiles of 16 to 128), K is sliced over the CTAs of a cluster, which add
- * their fp32 tiles in slice order.  More rows: the weights are rebuilt straight
- * into tensor memory (token tiles of 256); where that leaves much of the chip
- * idle K is sliced and a second kernel adds the partial tiles in slice order.
+ * (token tiles of 16 to 128) and K is sliced over the CTAs of a cluster, which
+ * add their fp32 tiles in slice order, or they are rebuilt straight into tensor
+ * memory (token tiles of 32 to 128) and K is sliced over up to 16 CTAs whose
+ * partial tiles a second kernel adds in slice order: whichever a model of the
+ * two takes to be faster for the shape.  More rows: the latter, with token tiles
+ * of 256 and slices only where the tiles leave much of the chip idle.
  * Deterministic either way.
  * `workspace` must hold atlas_qlinear_gemm_workspace_bytes(m, n_rows, n_cols)
  * bytes, 256-byte aligned.

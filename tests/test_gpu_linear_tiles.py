@@ -47,6 +47,41 @@ def test_tile_kernel_unaligned_rows(cuda_device):
     _check(200, 512, (17, 64, 100), cuda_device, strided=True)
 
 
+# up to 128 rows that the prompt kernel takes: a long K under few row tiles (16 K slices; an odd number of k-tiles, ragged
+# rows, blocks smaller than and not commensurable with a k-tile), and one wave of 128-token tiles
+@pytest.mark.parametrize("n,k,bs,thr,ms", [(1024, 8192, 128, 3.0, (17, 33, 64)), (130, 16448, 64, 3.0, (17, 32, 40)),
+                                           (512, 12288, 96, 3.0, (32, 64)), (256, 16384, 32, 1.0, (20, 50)),
+                                           (12288, 1088, 64, 3.0, (65, 128)), (9464, 1024, 32, 1.5, (97,))])
+def test_prompt_kernel_takes_over(n, k, bs, thr, ms, cuda_device):
+    _check(n, k, ms, cuda_device, bs=bs, thr=thr)
+    if n <= 130:
+        _check(n, k, ms[:1], cuda_device, bs=bs, thr=thr, strided=True)
+
+
+# the same kernel with the gather of its output, one rank: one to many K slices, ragged rows, more than 16 outliers of a
+# strip in a stage, every block form
+@pytest.mark.parametrize("n,k,bs,thr", [(200, 8256, 64, 3.0), (1000, 2048, 32, 3.0), (128, 6144, 96, 1.0), (64, 64, 64, 3.0)])
+def test_gathered_gemm_edges(n, k, bs, thr, cuda_device):
+    from atlasinfer_b200 import peer
+    o = O.quantize(config_weights(n, k, n + k), bs, thr)
+    lay = aw.build_kernel_layout(ab.QuantizedTensor(*o).to(cuda_device))
+    w = O.dequantize(o)
+    gen = torch.Generator().manual_seed(n)
+    b = (torch.randn(n, generator=gen) * 0.02).half()
+    arena = peer.PeerArena(1 << 20, cuda_device, world=1, rank=0, exchange=False)
+    try:
+        for dtype in (torch.float16, torch.bfloat16):
+            g = peer.GatheredLinear(arena, lay, 64, dtype, bias=b.to(cuda_device), kernel="gemm")
+            for m in (1, 32, 33, 64):
+                x = torch.randn(m, k, generator=gen).to(dtype)
+                y = g(x.to(cuda_device), wait=True).clone()
+                aw.check_status(cuda_device)
+                err = rel_max_err(y, O.linear(x, w, b), report=f"gathered {n}x{k} bs={bs} m={m}")
+                assert err < LINEAR_TOL, f"{n}x{k} bs={bs} m={m} {dtype}: {err}"
+    finally:
+        arena.close()
+
+
 # prompts whose few row tiles are cut along K: second kernel, 8 features at a time or one
 @pytest.mark.parametrize("n,k", [(128, 4096), (257, 2048), (1024, 8192)])
 def test_prompt_k_slices(n, k, cuda_device):
