@@ -6,7 +6,6 @@ sm_100a GPU is usable, calls raise -- there is no CPU or PyTorch fallback.
 from __future__ import annotations
 
 import ctypes
-import glob
 import importlib.util
 import os
 from typing import Optional
@@ -134,13 +133,15 @@ def native():
     """The host-path module (``csrc/native.cpp``), loaded on first use; raises with build instructions if it is missing."""
     global _native
     if _native is None:
+        from .build import NATIVE_NAME, native_path
+
         load()
-        path = [p for p in glob.glob(os.path.join(_PKG, "lib", "_atlas_native.*.so"))]
-        if not path:
+        path = native_path()   # (a module built for another torch or interpreter has another name)
+        if not os.path.exists(path):
             raise RuntimeError(
-                "atlasinfer_b200: the module _atlas_native is missing. Build it with "
+                f"atlasinfer_b200: {path} is missing. Build it with "
                 "`python -m atlasinfer_b200.build`; there is no fallback path.")
-        spec = importlib.util.spec_from_file_location("_atlas_native", path[0])
+        spec = importlib.util.spec_from_file_location(NATIVE_NAME, path)
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
         _native = mod

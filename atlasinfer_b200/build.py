@@ -46,7 +46,15 @@ def _inputs():
 
 NATIVE_NAME = "_atlas_native"
 NATIVE_SRC = os.path.join(CSRC, "native.cpp")
-NATIVE_PATH = os.path.join(LIB_DIR, NATIVE_NAME + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def native_path() -> str:
+    """Where the host path belongs: its name carries the torch version and the interpreter it was compiled for, since
+    it is tied to the C++ interfaces of both."""
+    import torch
+
+    abi = "" if torch.compiled_with_cxx11_abi() else "-oldabi"
+    return os.path.join(LIB_DIR, f"{NATIVE_NAME}-torch{torch.__version__}{abi}" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
 def _stale(target: str, sources) -> bool:
@@ -59,8 +67,9 @@ def _stale(target: str, sources) -> bool:
 def build_native(force: bool = False, verbose: bool = False) -> str:
     """Compile the host path (``csrc/native.cpp``, against torch's headers) if it is missing or old; return its path."""
     header = os.path.join(ROOT, "include", "atlas_b200.h")
-    if not force and not _stale(NATIVE_PATH, [NATIVE_SRC, header]):
-        return NATIVE_PATH
+    target = native_path()
+    if not force and not _stale(target, [NATIVE_SRC, header]):
+        return target
     import torch
     from torch.utils import cpp_extension
 
@@ -71,14 +80,14 @@ def build_native(force: bool = False, verbose: bool = False) -> str:
     cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else (shutil.which("g++") or "c++")
     cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-DTORCH_EXTENSION_NAME={NATIVE_NAME}",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{d}" for d in dirs), NATIVE_SRC,
-           "-o", NATIVE_PATH, f"-L{LIB_DIR}", "-l:libatlas_b200.so", "-Wl,-rpath,$ORIGIN", f"-L{torch_lib}",
+           "-o", target, f"-L{LIB_DIR}", "-l:libatlas_b200.so", "-Wl,-rpath,$ORIGIN", f"-L{torch_lib}",
            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
     if verbose:
         print(res.stdout + res.stderr)
-    return NATIVE_PATH
+    return target
 
 
 def is_stale() -> bool:

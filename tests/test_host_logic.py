@@ -1,4 +1,5 @@
 """Host-side mirror of the reference's Python surface (runs without a GPU)."""
+import os
 import sys
 import types
 
@@ -163,3 +164,19 @@ def test_status_word_of_a_cpu_device_is_not_the_gpus(monkeypatch):
     assert atlas_wrappers.status_word(torch.device("cuda")) is word
     assert atlas_wrappers.status_word(torch.device("cuda", 1)) is not word
     assert atlas_wrappers.status_word(torch.device("cpu")).device.type == "cpu"
+
+
+def test_native_module_of_another_torch_or_interpreter_is_not_taken(tmp_path, monkeypatch):
+    from atlasinfer_b200 import _capi, build
+    own = build.native_path()
+    monkeypatch.setattr(_capi, "_native", None)
+    monkeypatch.setattr(_capi, "_PKG", str(tmp_path))
+    monkeypatch.setattr(build, "LIB_DIR", str(tmp_path / "lib"))
+    (tmp_path / "lib").mkdir()
+    (tmp_path / "lib" / "_atlas_native.cpython-39-x86_64-linux-gnu.so").write_bytes(b"")
+    monkeypatch.setattr(_capi, "load", lambda: None)
+    with pytest.raises(RuntimeError, match="python -m atlasinfer_b200.build"):
+        _capi.native()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    other = build.native_path()
+    assert os.path.basename(other) != os.path.basename(own) and build._stale(other, [])
