@@ -1,4 +1,4 @@
-"""The dequantizer and the kernel layout at the edges of their 8192-element spans, byte for byte."""
+"""The dequantizer and the kernel layout at the edges of their 16384-element spans, byte for byte."""
 import numpy as np
 import pytest
 import torch
@@ -25,7 +25,7 @@ def _streams(numel, bs, share, seed):
     return O.OracleQuantized(codes, vals, idx, scales, torch.Size([numel]), bs)
 
 
-@pytest.mark.parametrize("numel", [1, 7, 8, 9, 8191, 8192, 8193, 16384 + 5, 100003])
+@pytest.mark.parametrize("numel", [1, 7, 8, 9, 8191, 8192, 8193, 16383, 16384, 16385, 16384 + 5, 32767, 32768, 32769, 100003])
 @pytest.mark.parametrize("bs,share", [(128, 0.003), (64, 0.3), (100, 0.01), (7, 0.02), (32, 0.0), (32, 1.0)])
 def test_dequantize_span_edges(numel, bs, share, cuda_device):
     o = _streams(numel, bs, share, numel + bs)
@@ -73,9 +73,11 @@ def _assert_layout(lay, want, row_ptr=True):
             assert np.array_equal(g.cpu().numpy().astype(np.int64), np.asarray(w).astype(np.int64)), name
 
 
-# one-unit rows, rows and columns on neither 16 nor 128, more than RP_STRIP_CAP outliers in a strip, many scale blocks
+# one-unit rows, rows and columns on neither 16 nor 128, more than RP_STRIP_CAP outliers in a strip, many scale blocks,
+# one and two whole spans, a span and one row more
 @pytest.mark.parametrize("n,k,bs,thr", [(1, 64, 64, 3.0), (16, 64, 16, 3.0), (129, 192, 64, 3.0), (300, 1088, 32, 3.0),
-                                        (200, 4096, 128, 1.0), (128, 8192, 128, 0.5), (77, 11008, 256, 3.0)])
+                                        (200, 4096, 128, 1.0), (128, 8192, 128, 0.5), (77, 11008, 256, 3.0),
+                                        (4, 4096, 128, 3.0), (8, 4096, 64, 1.0), (257, 64, 64, 3.0), (1, 16448, 64, 1.0)])
 def test_repack_matches_streams(n, k, bs, thr, cuda_device):
     w = config_weights(n, k, n + k)
     o = O.quantize(w, max(bs, 32), thr)._replace() if bs >= 32 else _streams(n * k, bs, 0.01, 3)._replace(original_shape=torch.Size([n, k]))
