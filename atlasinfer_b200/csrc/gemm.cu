@@ -1,5 +1,6 @@
-// Quantized linear for prompts: y[m][n] = sum_k x[m][k] * W[n][k] + bias[n], m > 128 (fewer rows: gemm_tile.cu), and
-// the decode-sized form whose output is gathered over the ranks of a node (m <= 64).
+// Quantized linear for prompts: y[m][n] = sum_k x[m][k] * W[n][k] + bias[n], m > 128; for fewer rows where it is the
+// faster kernel (route_for; else gemm_tile.cu); and the decode-sized form whose output is gathered over the ranks of a
+// node (m <= 64).
 //
 // Replaces the dequantize-then-F.linear of QuantizedLinear.forward
 // (integration/atlas_wrappers.py:56,67) for prompt-sized batches.  The fp16

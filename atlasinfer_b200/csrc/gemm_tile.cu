@@ -6,8 +6,9 @@
 //
 // One CTA computes 128 (output features) x BN (tokens) over a slice of K; the slices of a tile are the CTAs of one
 // cluster.  A pipeline step is one k-tile (64 columns of K).
-//   warp 0       activation producer: TMA of the BN x 64 tile (128-byte swizzle); bf16 rows are converted to fp16 in
-//                place, 16 bytes at a time (the swizzle only permutes 16-byte pieces)
+//   warp 0       activation producer: TMA of the BN x 64 tile (128-byte swizzle)
+//   warp 3       bf16 rows, where the tensor map delivers them: converted to fp16 in place, 16 bytes at a time (the
+//                swizzle only permutes 16-byte pieces)
 //   warp 2       code producer: TMA of the 8 KB code tile (64-byte swizzle) and 256 B of scales
 //   warps 4-11   dequantizers, thread = row: warp (q, ph) rebuilds rows 32q .. 32q+31 of every second k-tile as
 //                fp16(fp16(code) * scale) and stores them into a 16 KB K-major A tile in shared memory.  The outliers
@@ -25,8 +26,9 @@
 //
 // Measured (us, launch chain, against gemm.cu's kernel that served these sizes before): 57344 x 8192 at 32 rows 201 -> 156,
 // 64 rows 207 -> 163; 8192 x 28672 at 32 rows 95 -> 76; 22016 x 4096 at 32 rows 52 -> 37, 128 rows 58 -> 48; 4096 x 11008
-// at 128 rows 66 -> 27 (where gemm.cu's kernel is the faster one, route_for in gemm.cu leaves it the call).  Issue slots are 40 % used; the rest is the chain of a k-tile
-// through one A tile (rebuild, fence, MMA, commit), of which four are in flight per SM.
+// at 128 rows 66 -> 27 (where gemm.cu's kernel is the faster one, route_for in gemm.cu leaves it the call).  Issue slots are 45 % used (ncu, 22016 x 4096 at 32
+// rows); the rest is the chain of a k-tile through one A tile (rebuild, fence, MMA, commit), of which four are in flight
+// per SM.  Up to 16 rows (BN = 16) this is reached on request only: the per-strip kernel serves them.
 //
 // Every mbarrier wait is bounded; when one runs out the CTA sets the caller's status word, the producers and the MMA
 // thread wait (bounded) for what they have issued, and the CTA takes part in the cluster barriers, frees its TMEM and

@@ -366,6 +366,8 @@ constexpr int GS_STAGE_MAX_BYTES = 48 * 1024;   // staged fp16 activations per C
 //   18432 x 3072, 1.9: 1.13 1.12 1.12 1.16     12288 x 5120, 1.3: 0.91 0.90 0.97 0.97    14336 x 7168, 1.5: 0.94 0.98 0.97 1.01
 //   57344 x 8192, 6.1: 0.98 1.00 1.02 1.06     24576 x 7168, 2.6: 0.99 0.99 1.01 1.05    16384 x 11008, 1.7: 0.98 1.04 0.97 1.04
 //   12288 x 2048, 1.3: 0.90 0.93 0.92 0.97      9472 x 2048, 1.0: 0.88 0.90 0.91 0.97
+// What the rule gives away: 12288 x 4096, 1.3: 1.04 1.03 1.05 1.11 (its 64 % of two waves is refused with its neighbours
+// 11008 x 4096, 1.2: 0.94 0.95 0.94 1.00, 12288 x 3072, 1.3: 0.88 0.90 0.95 0.96 and 12288 x 6144, 1.3: 0.95 0.90 0.97 0.97).
 bool strip_pairs_pay(int64_t pairs, int n_chunks, bool bf16) {
     static thread_local int dev_cached = -1, sms = 148;
     int dev = 0;

@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(QT_THREADS) quantize_kernel(QuantParams p) {
 
 // ---------------------------------------------------------------------------------------------
 // Fast variant for block sizes 32 / 64 / 128 / 256.  Same results as quantize_kernel above, bit for bit, at a quarter of
-// its instructions: 121 us for 11008 x 4096 in blocks of 128 (165 with guard bands around the roundings and byte-wise
-// compaction), 46 % of the issue slots used, the rest mostly the barriers around the look-back.
+// its instructions: 121 us for 11008 x 4096 in blocks of 128 back to back, 128 with L2 flushed before (165 back to back with
+// guard bands around the roundings and byte-wise compaction), 46 % of the issue slots used, the rest mostly the barriers around the look-back.
 //
 // Four threads work on a block; thread t plays ATen's SIMD lanes 2t and 2t + 1, whose elements are neighbours, so the
 // values stay packed two to a register and most steps cost one instruction per pair.  What replaces the IEEE divisions
@@ -344,9 +344,16 @@ __global__ void __launch_bounds__(QT_THREADS) quantize_kernel(QuantParams p) {
 //     exceed T * den.  A tie (only possible for subnormal thresholds) goes to the even neighbour: if thr is odd, |d| =
 //     T * den is an outlier too.
 //   * d = fp16(x - mean) is one fp16 subtraction.
-//   * standard deviation.  fp32 sum of squares minus the squared sum, if the mean takes less than a fifth of it away (worst
-//     case error 2.5e-6 relative, else a second pass about the mean); only if rounding it to fp16 could go either way
-//     within 4e-6 is it recomputed in fp64 (about 1 % of blocks).
+//   * standard deviation.  fp32 sum of squares minus the squared sum, if the mean takes less than a fifth of it away, else a
+//     second pass about the mean; only if rounding it to fp16 could go either way within 4e-6 is it recomputed in fp64
+//     (about 1 % of blocks).  The bound, with u = 2^-24, Q the sum of squares, M = Q - F^2 / n the second moment and blocks
+//     of 256, the longest sums: Q carries 31 additions of a thread and 3 across threads, 34 u Q.  F carries 7 + 3 in a lane
+//     and 7 over the lanes, 17 u sum|x| <= 17 u sqrt(n Q), and |F| <= sqrt(0.2 n Q) here, so F^2 / n is off by
+//     2 * 0.45 * 17 u Q = 15 u Q.  With Q <= 1.25 M that is 62 u of M, 31 u of its root, and 4 u for the product, the root
+//     and the rounding of M: 35 u = 2.1e-6.  The second pass adds 64 times (66 u with the shuffles, 2 u for the squared
+//     differences), 34 u of the root, and 4 u as above: 2.3e-6; the mean it is taken about enters only through r1^2 / n,
+//     which is small because values that round in F make the block spread by a thirtieth of the largest at least.  (The
+//     largest error in an emulation over 4.8 M blocks of six kinds, offsets and wide exponents among them: 6.5e-7.)
 // The dense codes of a tile go to shared memory once; the compaction is driven by the output: a thread finds where its 16
 // bytes of the code stream start in the tile, takes them with one unaligned read, and squeezes out the places of outliers.
 struct FastConsts {

@@ -22,8 +22,10 @@ from .. import _capi
 from ..quant.adaptive_quantizer import QuantizedTensor
 
 # rows of x up to which the per-strip streaming kernel is used (16 rows per pass over the weight); above it the tcgen05
-# kernels.  At 16 rows the two are within 10 % of each other either way (4096 x 4096 9.1 against 10.8 us, 10240 x 8192
-# 37 against 32).  The persistent streaming kernel takes up to STREAM_MAX_ROWS rows in one pass; it is what the
+# kernels.  At 16 fp16 rows the per-strip kernel is ahead on small weights (1024 x 1024 3.3 against 4.6 us, 4096 x 4096
+# 8.3 against 10.6), even on 12288 x 4096 (21.5, 22.4) and 57344 x 8192 (151, 151) and behind where its strips end in a
+# poorly filled wave or K is long (10240 x 8192 36.8 against 30.8, 8192 x 28672 81.5 against 72.1); at 9 rows it is behind
+# in three of twelve shapes, by 6 % at most.  The persistent streaming kernel takes up to STREAM_MAX_ROWS rows in one pass; it is what the
 # column-parallel linear with the fused gather runs on and can be asked for with force="stream".
 GEMV_MAX_ROWS = 16
 STREAM_MAX_ROWS = 32
