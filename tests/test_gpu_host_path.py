@@ -89,3 +89,33 @@ def test_one_tensor_of_a_batch_overflows_its_outlier_buffer(cuda_device):
     assert qs[1].fp16_outliers.numel() > dense.numel() // 32 + 1024
     for q, w in zip(qs, ws):
         assert_streams_equal(q, O.quantize(w))
+
+
+@pytest.mark.parametrize("m", [1, 24, 100, 160])
+def test_first_call_of_a_thread_may_be_captured(m, cuda_device):
+    # what a thread looks up once per device (attributes, occupancy, the kernels' choice) must not need a call before
+    # the capture; the layout and the kernels' code are there already, as in a program that captures its second pass
+    lay = aw.build_kernel_layout(ab.quantize_tensor(config_weights(1024, 2048, 9).to(cuda_device)))
+    x = torch.randn(m, 2048, device=cuda_device).to(torch.bfloat16)
+    want = aw.quantized_linear_forward(x, lay, None)
+    torch.cuda.synchronize()
+    got, errors = [], []
+
+    def work():
+        try:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.stream(torch.cuda.Stream(cuda_device)):
+                with torch.cuda.graph(graph):
+                    y = aw.quantized_linear_forward(x, lay, None)
+                graph.replay()
+                torch.cuda.current_stream().synchronize()
+            got.append(y.clone())
+            torch.cuda.synchronize()
+        except BaseException as e:   # noqa: BLE001 - reported by the main thread
+            errors.append(e)
+
+    thread = threading.Thread(target=work)
+    thread.start()
+    thread.join()
+    assert not errors, errors[0]
+    assert torch.equal(bits(got[0]), bits(want))
