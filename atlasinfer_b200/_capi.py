@@ -22,6 +22,7 @@ DTYPE_F16, DTYPE_BF16 = 0, 1
 EXPORTS = (
     "atlas_version", "atlas_last_error", "atlas_status_string",
     "atlas_quantize_workspace_bytes", "atlas_quantize", "atlas_quantize_noalloc", "atlas_dequantize",
+    "atlas_quantize_many_workspace_bytes", "atlas_quantize_many", "atlas_copy_many",
     "atlas_tiles_bytes", "atlas_repack", "atlas_repack_many", "atlas_qlinear_gemv",
     "atlas_qlinear_stream_workspace_bytes", "atlas_qlinear_stream", "atlas_qlinear_stream_gather",
     "atlas_peer_wait", "atlas_peer_push", "atlas_peer_alloc", "atlas_peer_free", "atlas_peer_export", "atlas_peer_import",
@@ -40,6 +41,19 @@ class PeerGather(ctypes.Structure):
                 ("y_dst", ctypes.c_void_p * MAX_PEERS), ("flags_dst", ctypes.c_void_p * MAX_PEERS),
                 ("state", ctypes.c_void_p), ("wait_flags", ctypes.c_void_p), ("poll_limit", ctypes.c_int64)]
 
+
+class QuantizeItem(ctypes.Structure):
+    """``AtlasQuantizeItem`` of include/atlas_b200.h."""
+
+    _fields_ = [("w", ctypes.c_void_p), ("numel", ctypes.c_int64), ("codes", ctypes.c_void_p),
+                ("outlier_vals", ctypes.c_void_p), ("outlier_idx", ctypes.c_void_p), ("outlier_capacity", ctypes.c_int64),
+                ("scales", ctypes.c_void_p), ("counts", ctypes.c_void_p)]
+
+
+class CopyItem(ctypes.Structure):
+    """``AtlasCopyItem`` of include/atlas_b200.h."""
+
+    _fields_ = [("dst", ctypes.c_void_p), ("src", ctypes.c_void_p), ("bytes", ctypes.c_int64)]
 
 
 class RepackItem(ctypes.Structure):
@@ -85,6 +99,12 @@ def load() -> ctypes.CDLL:
     L.atlas_quantize.argtypes = [vp, i64, i32, f64, vp, vp, vp, i64, vp, vp, vp, sz, vp]
     L.atlas_quantize_noalloc.restype = i32
     L.atlas_quantize_noalloc.argtypes = [vp, i64, i32, f64, vp, vp, vp, i64, vp, vp, vp]
+    L.atlas_quantize_many_workspace_bytes.restype = sz
+    L.atlas_quantize_many_workspace_bytes.argtypes = [i32, ctypes.POINTER(QuantizeItem), i32]
+    L.atlas_quantize_many.restype = i32
+    L.atlas_quantize_many.argtypes = [i32, ctypes.POINTER(QuantizeItem), i32, f64, vp, sz, vp]
+    L.atlas_copy_many.restype = i32
+    L.atlas_copy_many.argtypes = [i32, ctypes.POINTER(CopyItem), vp]
     L.atlas_dequantize.restype = i32
     L.atlas_dequantize.argtypes = [vp, i64, vp, vp, i64, vp, i64, i32, vp, vp]
     L.atlas_tiles_bytes.restype = sz

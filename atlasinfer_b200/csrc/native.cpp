@@ -62,58 +62,86 @@ at::Tensor linear(const at::Tensor &x, const at::Tensor &tiles, const at::Tensor
     return y;
 }
 
+// What a tensor's streams are written to: codes and scales of their final length (codes: nearly), the outliers roomy.
 struct Job {
-    at::Tensor codes, scales, workspace, ovals, oidx;
-    int64_t capacity = 0, padded = 0;
+    at::Tensor codes, scales;
+    int64_t capacity, padded;
+    AtlasQuantizeItem item;
 };
 
-Job launch_quantize(const at::Tensor &flat, int64_t bs, double z, int64_t *counts, int64_t capacity, void *stream) {
+Job make_job(const at::Tensor &flat, int64_t bs, int64_t capacity, void *ovals, void *oidx, int64_t *counts) {
     Job j;
-    const int64_t numel = flat.numel(), blocks = (numel + bs - 1) / bs;
+    const int64_t blocks = (flat.numel() + bs - 1) / bs;
     j.padded = blocks * bs;
     j.capacity = capacity;
-    const size_t ws = atlas_quantize_workspace_bytes(numel, (int)bs);
-    const auto opt = flat.options();
-    j.codes = at::empty({j.padded}, opt.dtype(at::kChar));
-    j.scales = at::empty({blocks}, opt.dtype(at::kHalf));
-    j.workspace = at::empty({(int64_t)ws}, opt.dtype(at::kByte));
-    j.ovals = at::empty({capacity}, opt.dtype(at::kHalf));
-    j.oidx = at::empty({capacity}, opt.dtype(at::kLong));
-    check(atlas_quantize(flat.data_ptr(), numel, (int)bs, z, (int8_t *)j.codes.data_ptr(), j.ovals.data_ptr(), (int64_t *)j.oidx.data_ptr(),
-                         capacity, j.scales.data_ptr(), counts, j.workspace.data_ptr(), ws, stream), "atlas_quantize");
+    j.codes = at::empty({j.padded}, flat.options().dtype(at::kChar));
+    j.scales = at::empty({blocks}, flat.options().dtype(at::kHalf));
+    j.item = {flat.data_ptr(), flat.numel(), (int8_t *)j.codes.data_ptr(), ovals, (int64_t *)oidx, capacity, j.scales.data_ptr(), counts};
     return j;
 }
 
-// The four streams of every flat fp16 tensor (all on one device): all kernels are enqueued first, the stream lengths of
-// all of them come back in one device-to-host copy.
+int64_t up16(int64_t v) { return (v + 15) / 16 * 16; }
+
+// The four streams of every flat fp16 tensor (all on one device): one launch (block sizes of the fast kernel; up to 16
+// tensors), one device-to-host copy for the stream lengths of all, one launch that takes the outliers to buffers of their
+// own length.
 std::vector<std::array<at::Tensor, 4>> quantize_many(const std::vector<at::Tensor> &flats, int64_t bs, double z) {
     const c10::cuda::CUDAGuard guard(flats[0].device());
     void *stream = at::cuda::getCurrentCUDAStream(flats[0].get_device()).stream();
-    at::Tensor counts = at::empty({(int64_t)flats.size(), 4}, flats[0].options().dtype(at::kLong));
-    int64_t *dev_counts = counts.data_ptr<int64_t>();
-    std::vector<Job> jobs;
-    for (size_t i = 0; i < flats.size(); ++i) {
+    const auto bytes_opt = flats[0].options().dtype(at::kByte);
+    const size_t n = flats.size();
+    std::vector<int64_t> capacity(n);
+    int64_t workspace_bytes = 0, outlier_bytes = 0;
+    for (size_t i = 0; i < n; ++i) {
         // |z| > t bounds the outliers of a block by (block_size - 1) / t^2, but weight-like data has well under
         // 1 %: start with 1/32 of the tensor and retry with full capacity in the rare case that is short
         const int64_t padded = (flats[i].numel() + bs - 1) / bs * bs;
-        jobs.push_back(launch_quantize(flats[i], bs, z, dev_counts + 4 * i, std::min(padded, padded / 32 + 1024), stream));
+        capacity[i] = std::min(padded, padded / 32 + 1024);
+        workspace_bytes += atlas_quantize_workspace_bytes(flats[i].numel(), (int)bs);
+        outlier_bytes += up16(capacity[i] * 8) + up16(capacity[i] * 2);
     }
-    at::Tensor host = counts.cpu();   // the one synchronisation
+    // counts, and behind them the workspace: cleared together
+    at::Tensor scratch = at::empty({(int64_t)n * 32 + workspace_bytes}, bytes_opt);
+    at::Tensor outliers = at::empty({outlier_bytes}, bytes_opt);
+    int64_t *counts = (int64_t *)scratch.data_ptr();
+    std::vector<Job> jobs;
+    std::vector<AtlasQuantizeItem> items;
+    char *at_byte = (char *)outliers.data_ptr();
+    for (size_t i = 0; i < n; ++i) {
+        jobs.push_back(make_job(flats[i], bs, capacity[i], at_byte + up16(capacity[i] * 8), at_byte, counts + 4 * i));
+        at_byte += up16(capacity[i] * 8) + up16(capacity[i] * 2);
+        items.push_back(jobs[i].item);
+    }
+    check(atlas_quantize_many((int)n, items.data(), (int)bs, z, counts + 4 * n, (size_t)workspace_bytes, stream), "atlas_quantize");
+    const at::Tensor host = scratch.narrow(0, 0, (int64_t)n * 32).cpu();   // the one synchronisation
+    const int64_t *c = (const int64_t *)host.data_ptr();
     std::vector<std::array<at::Tensor, 4>> out;
-    for (size_t i = 0; i < flats.size(); ++i) {
-        const int64_t *c = host.data_ptr<int64_t>() + 4 * i;
-        int64_t n_codes = c[0], n_out = c[1], timed_out = c[2];
+    std::vector<AtlasCopyItem> copies;
+    std::vector<at::Tensor> held;   // buffers of a second attempt, until the copies are enqueued
+    for (size_t i = 0; i < n; ++i) {
+        int64_t n_codes = c[4 * i], n_out = c[4 * i + 1], timed_out = c[4 * i + 2];
         Job &j = jobs[i];
         if (!timed_out && n_out > j.capacity) {   // rare: more outliers than the first buffer holds
-            j = launch_quantize(flats[i], bs, z, dev_counts + 4 * i, j.padded, stream);
-            const at::Tensor again = counts.cpu();
-            c = again.data_ptr<int64_t>() + 4 * i;
-            n_codes = c[0], n_out = c[1], timed_out = c[2];
+            const size_t ws = atlas_quantize_workspace_bytes(flats[i].numel(), (int)bs);
+            const at::Tensor again = at::empty({32 + (int64_t)ws}, bytes_opt), roomy = at::empty({j.padded * 10}, bytes_opt);
+            held.push_back(roomy);
+            int64_t *own = (int64_t *)again.data_ptr();
+            j = make_job(flats[i], bs, j.padded, (char *)roomy.data_ptr() + j.padded * 8, roomy.data_ptr(), own);
+            check(atlas_quantize_many(1, &j.item, (int)bs, z, own + 4, ws, stream), "atlas_quantize");
+            const at::Tensor second = again.narrow(0, 0, 32).cpu();
+            const int64_t *s = (const int64_t *)second.data_ptr();
+            n_codes = s[0], n_out = s[1], timed_out = s[2];
         }
         if (timed_out) check(ATLAS_ERR_TIMEOUT, "atlas_quantize: device-side wait timed out");
-        // codes: a view (the buffer is 0.3 % longer than the stream); outliers: copied out of their roomy buffers
-        out.push_back({j.codes.narrow(0, 0, n_codes), j.ovals.narrow(0, 0, n_out).clone(), j.oidx.narrow(0, 0, n_out).clone(), j.scales});
+        // codes: a view (the buffer is 0.3 % longer than the stream)
+        const at::Tensor ovals = at::empty({n_out}, flats[i].options().dtype(at::kHalf)), oidx = at::empty({n_out}, flats[i].options().dtype(at::kLong));
+        if (n_out) {
+            copies.push_back({ovals.data_ptr(), j.item.outlier_vals, n_out * 2});
+            copies.push_back({oidx.data_ptr(), j.item.outlier_idx, n_out * 8});
+        }
+        out.push_back({j.codes.narrow(0, 0, n_codes), ovals, oidx, j.scales});
     }
+    check(atlas_copy_many((int)copies.size(), copies.data(), stream), "atlas_copy_many");
     return out;
 }
 

@@ -370,10 +370,37 @@ __device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned l
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Outliers of all tiles before `tile` (whole warp).  All resident CTAs finish a tile at about the same time and find only
-// counts, no prefixes, among each other's, so the walk back covers 256 tiles per round trip.  A status word holds all
-// that is passed on, so relaxed accesses do.
-__device__ __forceinline__ long long look_back(const unsigned long long *status, int64_t tile, int lane, int64_t *counts) {
+// One tensor of a launch.
+struct QuantItem {
+    const uint16_t *x;
+    int8_t *codes;
+    uint16_t *ovals;
+    int64_t *oidx;
+    uint16_t *scales;
+    int64_t *counts;
+    int64_t numel, padded, ocap;
+    int64_t first_tile;   // of this tensor, among the tiles of the launch
+    int in_aligned;       // x is 16-byte aligned
+    int out_aligned;      // codes is 16-byte aligned
+};
+constexpr int QF_MAX_ITEMS = 16;
+struct QuantBatch {
+    QuantItem item[QF_MAX_ITEMS];
+    int n;
+    unsigned int num_tiles;
+    unsigned int *tile_counter;
+    unsigned long long *status;   // one word per tile
+};
+
+constexpr int QF_WORKERS = 8;                        // warps that work on elements: 1024 of a tile each
+constexpr int QF_THREADS = (QF_WORKERS + 1) * 32;    // and one for the tile numbers and the look-back
+constexpr int QF_CTAS = 4;                           // per SM: 56 registers
+constexpr int QF_BUFS = 3;                           // tiles a CTA holds codes of
+static_assert(QF_WORKERS * 1024 == QT_TILE && QT_WORDS == QF_WORKERS * 32, "a warp's elements are its 32 mask words");
+
+// Outliers of the launch's tiles [first, tile) (whole warp).  A status word holds all that is passed on, so relaxed
+// accesses do; a round trip covers 256 tiles.
+__device__ __forceinline__ long long look_back(const unsigned long long *status, int64_t first, int64_t tile, int lane, int64_t *counts) {
     long long prefix = 0;
     int64_t look = tile - 1;
     for (int spins = 0; spins <= QT_SPIN_LIMIT; ++spins) {
@@ -381,18 +408,18 @@ __device__ __forceinline__ long long look_back(const unsigned long long *status,
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int64_t idx = look - k * 32 - lane;
-            v[k] = idx >= 0 ? ld_relaxed_u64(status + idx) : ST_PREFIX;   // tiles before the first count as prefix 0
+            v[k] = idx >= first ? ld_relaxed_u64(status + idx) : ST_PREFIX;   // tiles before the tensor's first count as prefix 0
         }
         int taken = 0;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             if (taken != k) continue;
             const unsigned pm = __ballot_sync(0xffffffffu, (v[k] >> 62) == 2), none = __ballot_sync(0xffffffffu, (v[k] >> 62) == 0);
-            const int first = pm ? __ffs(pm) - 1 : 31;
-            if (none & (0xffffffffu >> (31 - first))) continue;          // not there yet
-            unsigned int contrib = lane < first || (!pm && lane == first) ? (unsigned int)(v[k] & ST_VALUE) : 0u;   // a tile's own count
+            const int first_pm = pm ? __ffs(pm) - 1 : 31;
+            if (none & (0xffffffffu >> (31 - first_pm))) continue;       // not there yet
+            unsigned int contrib = lane < first_pm || (!pm && lane == first_pm) ? (unsigned int)(v[k] & ST_VALUE) : 0u;   // a tile's own count
             prefix += (long long)__reduce_add_sync(0xffffffffu, contrib);
-            if (pm) return prefix + (long long)(__shfl_sync(0xffffffffu, v[k], first) & ST_VALUE);
+            if (pm) return prefix + (long long)(__shfl_sync(0xffffffffu, v[k], first_pm) & ST_VALUE);
             ++taken;
         }
         look -= taken * 32;
@@ -402,330 +429,485 @@ __device__ __forceinline__ long long look_back(const unsigned long long *status,
     return prefix;
 }
 
-// Byte offset of element e's code in the dense tile: 16-byte pieces permuted so that the eight blocks a warp works on
-// fall on different banks.
-__device__ __forceinline__ int dense_byte(int e) { return e ^ (((e >> 7) & 7) << 4); }
+// Byte offset of element e's code in the dense tile: 32-byte pieces permuted so that the four 128-element runs a
+// half-warp stores to fall on different banks.
+__device__ __forceinline__ int dense_byte(int e) { return e ^ (((e >> 7) & 3) << 5); }
+
+// Two fp32 values in one register pair: one instruction works on both.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float2 h2f2(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2 *>(&v)); }
+
+// Values held packed are converted anew in every pass: the compiler must not keep 32 floats for the next one.
+__device__ __forceinline__ void forget(uint4 (&x)[4]) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) asm volatile("" : "+r"(x[c].x), "+r"(x[c].y), "+r"(x[c].z), "+r"(x[c].w));
+}
+
+struct FastShared {
+    __align__(16) uint8_t dense[QF_BUFS][QT_TILE + 128];
+    __align__(16) float fold[QF_WORKERS][256];       // accumulators of a warp, on their way to the threads that add them
+    __align__(16) uint32_t mask[QF_BUFS][QT_WORDS + 4];   // bit e & 31 of word e >> 5: element e is an outlier
+    uint32_t word_before[QF_BUFS][QT_WORDS];         // outliers before the word, counted in its warp's elements
+    uint32_t warp_total[QF_BUFS][QF_WORKERS];
+    uint32_t warp_base[QF_BUFS][QF_WORKERS + 1];     // outliers of the tile before the warp's elements; the last: of the tile
+    long long prefix[2];                             // outliers of the tensor before the tile
+    unsigned int tile[4];
+    int item[4];
+};
+
+// The 32 elements (four runs of eight) of this thread in a tile; zeros beyond the tensor's end.
+template <class At>
+__device__ __forceinline__ void load_elements(const QuantItem &q, int64_t tile_base, const At &at, uint4 (&x)[4]) {
+    const uint16_t *src = q.x + tile_base;
+    const int real = (int)min((int64_t)QT_TILE, q.numel - tile_base);
+    if (q.in_aligned && real == QT_TILE) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(x[c].x), "=r"(x[c].y), "=r"(x[c].z), "=r"(x[c].w) : "l"(src + at(c)));
+        return;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int e = at(c);
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            w[i] = e + 2 * i < real ? __ldg(src + e + 2 * i) : 0u;
+            if (e + 2 * i + 1 < real) w[i] |= (uint32_t)__ldg(src + e + 2 * i + 1) << 16;
+        }
+        x[c] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// Second moment of a block about its mean as fp32 has it, the first moment about that taken out again, so that the
+// rounding of the mean itself only enters to second order (whole warp; x0 ... x3: the thread's runs of the block, the
+// first four, two or one of them for blocks of 128 and more, 64 and 32).  Rare, so it is a call: inlined, its registers
+// would spill the others'.
+template <int BS>
+__device__ __noinline__ float moment_about(uint4 x0, uint4 x1, uint4 x2, uint4 x3, float mean) {
+    constexpr int NW = BS < 128 ? BS / 8 : 16, GROUP = BS == 256 ? 8 : 4;
+    const uint32_t xw[16] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w, x2.x, x2.y, x2.z, x2.w, x3.x, x3.y, x3.z, x3.w};
+    float r1 = 0.f, m2 = 0.f;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        const float2 f = h2f2(xw[w]);
+        const float d0 = f.x - mean, d1 = f.y - mean;
+        r1 += d0 + d1;
+        m2 = fmaf(d0, d0, fmaf(d1, d1, m2));
+    }
+#pragma unroll
+    for (int o = 1; o < GROUP; o <<= 1) {
+        m2 += __shfl_xor_sync(0xffffffffu, m2, o);
+        r1 += __shfl_xor_sync(0xffffffffu, r1, o);
+    }
+    return fmaxf(fmaf(-r1, r1 * (1.f / (float)BS), m2), 0.f);
+}
+
+// fp16 standard deviation of a block from fp64 moments (as above).
+template <int BS>
+__device__ __noinline__ uint16_t std_in_fp64(uint4 x0, uint4 x1, uint4 x2, uint4 x3) {
+    constexpr int NW = BS < 128 ? BS / 8 : 16, GROUP = BS == 256 ? 8 : 4;
+    const uint32_t xw[16] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w, x2.x, x2.y, x2.z, x2.w, x3.x, x3.y, x3.z, x3.w};
+    double dsum = 0.0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) { const float2 f = h2f2(xw[w]); dsum += (double)f.x + (double)f.y; }
+#pragma unroll
+    for (int o = 1; o < GROUP; o <<= 1) dsum += __shfl_xor_sync(0xffffffffu, dsum, o);
+    const double mean = dsum / (double)BS;
+    double m2 = 0.0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        const float2 f = h2f2(xw[w]);
+        const double d0 = (double)f.x - mean, d1 = (double)f.y - mean;
+        m2 = fma(d0, d0, fma(d1, d1, m2));
+    }
+#pragma unroll
+    for (int o = 1; o < GROUP; o <<= 1) m2 += __shfl_xor_sync(0xffffffffu, m2, o);
+    return f2h_bits(__double2float_rn(sqrt(m2 / (double)(BS - 1))));
+}
 
 template <int BS>
-__global__ void __launch_bounds__(QT_THREADS, 5) quantize_fast_kernel(QuantParams p, FastConsts fc) {
-    constexpr int NP = BS / 8;                // pairs per thread
-    constexpr int TILE_BLOCKS = QT_TILE / BS;
-    // blocks are padded by 16 bytes so that the eight blocks a warp works on at a time fall on different banks
-    constexpr int XSTRIDE = BS * 2 + 16;      // bytes
-    __shared__ __align__(16) uint8_t s_xb[TILE_BLOCKS * XSTRIDE];
-    __shared__ __align__(16) uint8_t s_dense[QT_TILE + 128];
-    auto xref = [&](int e) -> uint16_t & {
-        return *reinterpret_cast<uint16_t *>(s_xb + (e / BS) * XSTRIDE + (e % BS) * 2);
-    };
-    __shared__ uint32_t s_mask[QT_WORDS + 1];
-    __shared__ uint32_t s_wordpre[QT_WORDS];
-    __shared__ uint16_t s_scale[TILE_BLOCKS];
-    __shared__ uint32_t s_warp_tot[QT_THREADS / 32];
-    __shared__ long long s_tile_prefix;
-    __shared__ int s_tile_total;
-    __shared__ unsigned int s_tile;
+__global__ void __launch_bounds__(QF_THREADS, QF_CTAS) quantize_fast_kernel(const __grid_constant__ QuantBatch p, FastConsts fc) {
+    constexpr int NB = BS < 128 ? 128 / BS : 1;   // blocks a thread has a part of
+    constexpr int CK = 4 / NB;                    // its runs of eight in each
+    __shared__ FastShared s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr unsigned ALL = 0xffffffffu, NO_TILE = 0xffffffffu;
 
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int warp = tid >> 5;
-    const uint16_t eps_h = f2h_bits(1e-6f);
-    const float eps_f = h2f_bits(eps_h);
-    if (tid == 0) s_mask[QT_WORDS] = 0u;
-
-    for (;;) {
-        __syncthreads();  // previous tile's shared state is no longer read
-        if (tid == 0) s_tile = atomicAdd(p.tile_counter, 1u);
+    if (warp == QF_WORKERS) {
+        // ---- the warp that numbers the tiles and looks back -------------------------------------------
+        const int64_t item_first = lane < p.n ? p.item[lane].first_tile : INT64_MAX;
+        auto fetch = [&](int slot) {
+            unsigned int t = 0;
+            if (lane == 0) t = atomicAdd(p.tile_counter, 1u);
+            t = __shfl_sync(ALL, t, 0);
+            const int it = __popc(__ballot_sync(ALL, item_first <= (int64_t)t)) - 1;
+            if (lane == 0) {
+                s.tile[slot] = t < p.num_tiles ? t : NO_TILE;
+                s.item[slot] = it;
+            }
+        };
+        if (lane < QF_BUFS) s.mask[lane][QT_WORDS] = 0u;
+        fetch(0);
         __syncthreads();
-        const int64_t tile = s_tile;
-        if (tile >= p.num_tiles) break;
-        const int64_t tile_base = tile * QT_TILE;
-        const int tile_elems = (int)min((int64_t)QT_TILE, p.padded - tile_base);
-        const int tile_real = (int)max((int64_t)0, min((int64_t)tile_elems, p.numel - tile_base));
-        const int tile_blocks = tile_elems / BS;
-
-        // ---- stage the tile (zero padding included) -------------------------------
-        if (p.in_aligned) {
-            const uint4 *src = reinterpret_cast<const uint4 *>(p.x + tile_base);
-#pragma unroll
-            for (int i = 0; i < QT_TILE / 8 / QT_THREADS; ++i) {
-                const int v = tid + i * QT_THREADS, e0 = v * 8;
-                if (e0 + 8 <= tile_real) {
-                    *reinterpret_cast<uint4 *>(s_xb + (e0 / BS) * XSTRIDE + (e0 % BS) * 2) = __ldg(src + v);
-                } else if (e0 < tile_elems) {
-                    for (int e = e0; e < e0 + 8; ++e) xref(e) = (e < tile_real) ? p.x[tile_base + e] : (uint16_t)0;
+        unsigned int prev = NO_TILE;
+        int prev_item = 0;
+        long long prev_total = 0;
+        for (int i = 0, buf = 0;; ++i, buf = buf == QF_BUFS - 1 ? 0 : buf + 1) {
+            const unsigned int cur = s.tile[i & 3];
+            const int cur_item = s.item[i & 3];
+            if (cur != NO_TILE) fetch((i + 1) & 3);
+            if (prev != NO_TILE) {
+                const QuantItem &q = p.item[prev_item];
+                long long prefix = 0;
+                if (prev != q.first_tile) {
+                    prefix = look_back(p.status, q.first_tile, prev, lane, q.counts);
+                    if (lane == 0) st_relaxed_u64(p.status + prev, ST_PREFIX | (unsigned long long)(prefix + prev_total));
+                }
+                if (lane == 0) {
+                    s.prefix[(i - 1) & 1] = prefix;
+                    if (((int64_t)prev - q.first_tile + 1) * QT_TILE >= q.padded) {   // the tensor's last tile
+                        q.counts[0] = q.padded - (prefix + prev_total);
+                        q.counts[1] = prefix + prev_total;
+                    }
                 }
             }
-        } else {
-            for (int e = tid; e < tile_elems; e += QT_THREADS)
-                xref(e) = (e < tile_real) ? p.x[tile_base + e] : (uint16_t)0;
+            __syncthreads();
+            if (cur == NO_TILE) break;
+            const uint32_t own = lane < QF_WORKERS ? s.warp_total[buf][lane] : 0u;
+            uint32_t inc = own;
+#pragma unroll
+            for (int o = 1; o < QF_WORKERS; o <<= 1) {
+                const uint32_t n = __shfl_up_sync(ALL, inc, o);
+                if (lane >= o) inc += n;
+            }
+            prev_total = __shfl_sync(ALL, inc, QF_WORKERS - 1);
+            if (lane < QF_WORKERS) s.warp_base[buf][lane] = inc - own;
+            if (lane == QF_WORKERS) s.warp_base[buf][lane] = (uint32_t)prev_total;
+            if (lane == 0)
+                st_relaxed_u64(p.status + cur, (cur == p.item[cur_item].first_tile ? ST_PREFIX : ST_AGG) | (unsigned long long)prev_total);
+            prev = cur;
+            prev_item = cur_item;
         }
-        s_mask[tid] = 0u;   // QT_WORDS == QT_THREADS
-        __syncthreads();
+        return;
+    }
 
-        // ---- statistics and codes of whole blocks, 4 threads per block ----------
-        {
-            const int t = tid & 3;
-            const unsigned gmask = 0xfu << (lane & 28);
-            for (int b = tid >> 2; b < tile_blocks; b += QT_THREADS / 4) {
-                const uint32_t *xb = reinterpret_cast<const uint32_t *>(s_xb + b * XSTRIDE) + t;
-                // (read from shared memory again in every pass: keeping 32 floats costs the fifth CTA of an SM)
-                auto pair = [&](int j) { return __half22float2(*reinterpret_cast<const __half2 *>(xb + j * 4)); };
-                // fp32 sum in ATen's order, and the sum of squares
-                float lo4[4] = {0.f, 0.f, 0.f, 0.f}, hi4[4] = {0.f, 0.f, 0.f, 0.f}, sq = 0.f, sq_hi = 0.f;
+    // ---- workers -------------------------------------------------------------------------------------
+    const int t = lane & 3, grp = lane >> 2;
+    const int run0 = warp * 1024 + grp * (BS < 128 ? BS : 128) + t * 8;
+    auto at = [&](int c) { return run0 + (c / CK) * 8 * BS + (c % CK) * 32; };   // first element of run c in the tile
+    const uint16_t eps_h = f2h_bits(1e-6f);
+    const float eps_f = h2f_bits(eps_h);
+    const unsigned gmask = BS == 256 ? 0xffu << (lane & 24) : 0xfu << (lane & 28);   // the threads of a block
+    float *fold = s.fold[warp];
+
+    __syncthreads();
+    uint4 x[4];
+    unsigned int cur = s.tile[0], prev = NO_TILE;
+    int cur_item = s.item[0], prev_item = 0;
+    if (cur != NO_TILE) load_elements(p.item[cur_item], ((int64_t)cur - p.item[cur_item].first_tile) * QT_TILE, at, x);
+
+    for (int i = 0, buf = 0, prev_buf = 0;; ++i, prev_buf = buf, buf = buf == QF_BUFS - 1 ? 0 : buf + 1) {
+        // ---- statistics, codes and outlier mask of this thread's elements ---------------------------
+        if (cur != NO_TILE) {
+            const QuantItem &q = p.item[cur_item];
+            const int64_t tile_base = ((int64_t)cur - q.first_tile) * QT_TILE;
+            const int tile_elems = (int)min((int64_t)QT_TILE, q.padded - tile_base);
+            uint16_t *scales = q.scales + tile_base / BS;
+            uint32_t mask16[2] = {0u, 0u};   // outlier bits of runs 0, 1 and 2, 3
 #pragma unroll
-                for (int j = 0; j < NP; ++j) {
-                    const float2 f = pair(j);
-                    lo4[j & 3] = __fadd_rn(lo4[j & 3], f.x);
-                    hi4[j & 3] = __fadd_rn(hi4[j & 3], f.y);
-                    sq = fmaf(f.x, f.x, sq);
-                    sq_hi = fmaf(f.y, f.y, sq_hi);
+            for (int b = 0; b < NB; ++b) {
+                const uint32_t *xw = reinterpret_cast<const uint32_t *>(x) + b * CK * 4;
+                // fp32 sum in ATen's order, and the sum of squares.  This thread holds accumulator t of all eight lanes.
+                uint64_t a[4], sq2[2];
+#pragma unroll
+                for (int w = 0; w < CK * 4; ++w) {
+                    const float2 f = h2f2(xw[w]);
+                    const uint64_t f2 = pack2(f.x, f.y);
+                    a[w & 3] = w < 4 ? f2 : add2(a[w & 3], f2);
+                    sq2[w & 1] = w < 2 ? mul2(f2, f2) : fma2(f2, f2, sq2[w & 1]);
                 }
-                asm volatile("" ::: "memory");
-                const float lo_sum = __fadd_rn(__fadd_rn(__fadd_rn(lo4[0], lo4[1]), lo4[2]), lo4[3]);
-                const float hi_sum = __fadd_rn(__fadd_rn(__fadd_rn(hi4[0], hi4[1]), hi4[2]), hi4[3]);
-                float fin = 0.f;
+                forget(x);
+                float *slot = fold + grp * 32 + (t ^ (grp & 3)) * 8;   // permuted against bank conflicts
+                auto store_fold = [&]() {
+                    const float2 a0 = unpack2(a[0]), a1 = unpack2(a[1]), a2 = unpack2(a[2]), a3 = unpack2(a[3]);
+                    *reinterpret_cast<float4 *>(slot + (grp & 1) * 4) = make_float4(a0.x, a0.y, a1.x, a1.y);
+                    *reinterpret_cast<float4 *>(slot + (~grp & 1) * 4) = make_float4(a2.x, a2.y, a3.x, a3.y);
+                };
+                __syncwarp();
+                store_fold();
+                __syncwarp();
+                if (BS == 256) {
+                    // the block's second half goes on from the first half's accumulators
+                    const int pg = grp & 6;
+                    const float *ps = fold + pg * 32 + (t ^ (pg & 3)) * 8;
+                    const float4 p0 = *reinterpret_cast<const float4 *>(ps), p1 = *reinterpret_cast<const float4 *>(ps + 4);
+                    a[0] = pack2(p0.x, p0.y); a[1] = pack2(p0.z, p0.w); a[2] = pack2(p1.x, p1.y); a[3] = pack2(p1.z, p1.w);
 #pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    fin = __fadd_rn(fin, __shfl_sync(gmask, lo_sum, s, 4));
-                    fin = __fadd_rn(fin, __shfl_sync(gmask, hi_sum, s, 4));
+                    for (int w = 0; w < CK * 4; ++w) {
+                        const float2 f = h2f2(xw[w]);
+                        a[w & 3] = add2(a[w & 3], pack2(f.x, f.y));
+                    }
+                    __syncwarp();
+                    if (grp & 1) store_fold();
+                    __syncwarp();
+                }
+                float fin;
+                {
+                    // this thread adds lanes 2t and 2t + 1: accumulators in order, then the lanes in order
+                    const int g = BS == 256 ? grp | 1 : grp;
+                    const float *src = fold + g * 32 + ((t >> 1) ^ (g & 1)) * 4 + (t & 1) * 2;
+                    uint64_t l = *reinterpret_cast<const uint64_t *>(src + (0 ^ (g & 3)) * 8);
+#pragma unroll
+                    for (int j = 1; j < 4; ++j) l = add2(l, *reinterpret_cast<const uint64_t *>(src + (j ^ (g & 3)) * 8));
+                    const float2 lv = unpack2(l);
+                    fin = __fadd_rn(__fadd_rn(0.f, lv.x), lv.y);
+#pragma unroll
+                    for (int j = 1; j < 4; ++j) fin = __fadd_rn(__fadd_rn(__shfl_sync(ALL, fin, j - 1, 4), lv.x), lv.y);
+                    fin = __shfl_sync(ALL, fin, 3, 4);
                 }
                 const float mean32 = fin * (1.f / (float)BS);   // a power of two: exact
                 const uint16_t mean_h = f2h_bits(mean32);
-                sq += sq_hi;
-                sq += __shfl_xor_sync(gmask, sq, 1, 4);
-                sq += __shfl_xor_sync(gmask, sq, 2, 4);
-                float m2f = fmaf(-fin, mean32, sq);
-                if (!(sq <= 1.25f * m2f)) {   // (the same decision in all four threads)
-                    // about mean32, with the first moment about it taken out again, so that the rounding of mean32
-                    // itself only enters to second order
-                    float r1 = 0.f;
-                    m2f = 0.f;
-#pragma unroll 1
-                    for (int j = 0; j < NP; ++j) {
-                        const float2 f = pair(j);
-                        const float d0 = f.x - mean32, d1 = f.y - mean32;
-                        r1 += d0 + d1;
-                        m2f = fmaf(d0, d0, fmaf(d1, d1, m2f));
-                    }
+                constexpr int GROUP = BS == 256 ? 8 : 4;
+                const float2 sv = unpack2(add2(sq2[0], sq2[1]));
+                float sq = sv.x + sv.y;
 #pragma unroll
-                    for (int o = 1; o < 4; o <<= 1) {
-                        m2f += __shfl_xor_sync(gmask, m2f, o, 4);
-                        r1 += __shfl_xor_sync(gmask, r1, o, 4);
-                    }
-                    m2f = fmaxf(fmaf(-r1, r1 * (1.f / (float)BS), m2f), 0.f);
+                for (int o = 1; o < GROUP; o <<= 1) sq += __shfl_xor_sync(ALL, sq, o);
+                float m2f = fmaf(-fin, mean32, sq);
+                forget(x);
+                const bool about_mean = !(sq <= 1.25f * m2f);   // (the same decision in all threads of a block)
+                if (__any_sync(ALL, about_mean)) {
+                    const float m2 = moment_about<BS>(x[b * CK], x[b * CK + (CK > 1)], x[b * CK + (CK > 2) * 2], x[b * CK + (CK > 2) * 3], mean32);
+                    if (about_mean) m2f = m2;
                 }
+                forget(x);
                 float std32;
                 asm("sqrt.approx.f32 %0, %1;" : "=f"(std32) : "f"(m2f * (1.f / (float)(BS - 1))));
                 uint16_t std_h = f2h_bits(std32 * (1.f - 4e-6f));
-                if (std_h != f2h_bits(std32 * (1.f + 4e-6f))) {
-                    // the fp16 rounding is within reach of the fp32 error: redo it in fp64
-                    double dsum = 0.0;
-#pragma unroll 1
-                    for (int j = 0; j < NP; ++j) { const float2 f = pair(j); dsum += (double)f.x + (double)f.y; }
-#pragma unroll
-                    for (int o = 1; o < 4; o <<= 1) dsum += __shfl_xor_sync(gmask, dsum, o, 4);
-                    const double mean_d = dsum / (double)BS;
-                    double m2 = 0.0;
-#pragma unroll 1
-                    for (int j = 0; j < NP; ++j) {
-                        const float2 f = pair(j);
-                        const double d0 = (double)f.x - mean_d, d1 = (double)f.y - mean_d;
-                        m2 = fma(d0, d0, fma(d1, d1, m2));
-                    }
-#pragma unroll
-                    for (int o = 1; o < 4; o <<= 1) m2 += __shfl_xor_sync(gmask, m2, o, 4);
-                    std_h = f2h_bits(__double2float_rn(sqrt(m2 / (double)(BS - 1))));
+                const bool unsure = std_h != f2h_bits(std32 * (1.f + 4e-6f));   // the fp16 rounding is within reach of the fp32 error
+                if (__any_sync(ALL, unsure)) {
+                    const uint16_t exact = std_in_fp64<BS>(x[b * CK], x[b * CK + (CK > 1)], x[b * CK + (CK > 2) * 2], x[b * CK + (CK > 2) * 3]);
+                    if (unsure) std_h = exact;
                 }
+                forget(x);
                 const float den_f = h2f_bits(f2h_bits(__fadd_rn(h2f_bits(std_h), eps_f)));
                 // the largest |d| that is not an outlier
                 const float bound = fc.T * den_f;
                 uint16_t cut = __half_as_ushort(__float2half_rd(bound));
                 if (fc.tie_out && h2f_bits(cut) == bound) --cut;
                 const __half2 cut2 = __half2half2(__ushort_as_half(cut)), mean2 = __half2half2(__ushort_as_half(mean_h));
-                // z test, outlier mask (low half: even elements, high half: odd ones), absmax of the rest
-                constexpr int NM = (NP + 15) / 16;
-                uint32_t omask[NM], maxabs = 0u;
+                // z test, outlier bits (low half: even elements, high half: odd ones), absmax of the rest
+                uint32_t bits2[2] = {0u, 0u}, maxabs = 0u;
 #pragma unroll
-                for (int i = 0; i < NM; ++i) omask[i] = 0u;
-#pragma unroll
-                for (int j = 0; j < NP; ++j) {
-                    const uint32_t x2 = xb[j * 4];
-                    const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&x2), mean2);
+                for (int w = 0; w < CK * 4; ++w) {
+                    const int c = b * CK + (w >> 2);   // run
+                    const __half2 d = __hsub2(*reinterpret_cast<const __half2 *>(&xw[w]), mean2);
                     const uint32_t out = __hgt2_mask(__habs2(d), cut2);
-                    omask[j >> 4] |= out & (0x00010001u << (j & 15));
-                    maxabs = __vmaxu2(maxabs, x2 & 0x7fff7fffu & ~out);   // fp16 magnitude bits order like the values
+                    bits2[c >> 1] |= out & (0x00020001u << ((c & 1) * 8 + (w & 3) * 2));
+                    maxabs = __vmaxu2(maxabs, xw[w] & 0x7fff7fffu & ~out);   // fp16 magnitude bits order like the values
                 }
-                asm volatile("" ::: "memory");
-                int cnt = 0;
-#pragma unroll
-                for (int i = 0; i < NM; ++i) cnt += __popc(omask[i]);
-                const bool any_out = cnt != 0;
-#pragma unroll
-                for (int o = 1; o < 4; o <<= 1) {
-                    cnt += __shfl_xor_sync(gmask, cnt, o, 4);
-                    maxabs = __vmaxu2(maxabs, __shfl_xor_sync(gmask, maxabs, o, 4));
+                bool kept;
+                if (CK == 4) {
+                    const uint32_t m0 = (bits2[0] | bits2[0] >> 16) & 0xffffu, m1 = (bits2[1] | bits2[1] >> 16) & 0xffffu;
+                    kept = (m0 & m1) != 0xffffu;
+                    mask16[0] = m0;
+                    mask16[1] = m1;
+                } else {
+                    const int h = (b * CK) >> 1, sh = ((b * CK) & 1) * 8;
+                    constexpr uint32_t full = CK == 2 ? 0xffffu : 0xffu;
+                    const uint32_t m = (bits2[h] | bits2[h] >> 16) & (full << sh);
+                    kept = m != full << sh;
+                    mask16[h] |= m;
                 }
+                const bool any_kept = (__ballot_sync(ALL, kept) & gmask) != 0u;
+#pragma unroll
+                for (int o = 1; o < GROUP; o <<= 1) maxabs = __vmaxu2(maxabs, __shfl_xor_sync(ALL, maxabs, o));
                 maxabs = max(maxabs & 0xffffu, maxabs >> 16);
                 uint16_t sc = 0x3c00u;  // 1.0 when the block has no non-outliers
-                if (cnt < BS) sc = max(f2h_bits(h2f_bits((uint16_t)maxabs) * (1.0f / 127.0f)), eps_h);
-                if (t == 0) s_scale[b] = sc;
+                if (any_kept) sc = max(f2h_bits(h2f_bits((uint16_t)maxabs) * (1.0f / 127.0f)), eps_h);
+                if (t == 0 && (BS < 256 || !(grp & 1)) && at(b * CK) < tile_elems) scales[at(b * CK) / BS] = sc;
                 const float rsc = __frcp_rn(h2f_bits(sc));
-                // A NaN quotient is code 0.  It takes an infinity or a NaN among the values kept, which makes the scale
-                // infinite or NaN and every other quotient of the block 0 or NaN: such a block selects zero bytes
-                // instead of the low bytes of its (min/max-cleaned) sums, which costs the others nothing.
-                const uint32_t low_bytes = sc < 0x7c00u ? 0x4420u : 0x4444u;
-                uint8_t *db = s_dense;
-                const int e0 = b * BS + 2 * t;
-                const __half2 lim = __float2half2_rn(127.f), nlim = __float2half2_rn(-127.f), magic = __float2half2_rn(1536.f);
+                const uint64_t rsc2 = pack2(rsc, rsc);
+                const __half2 magic = __float2half2_rn(1536.f);
+                uint8_t *db = s.dense[buf];
+                // A kept value is at most 127 (1 + 2^-11) scales, 127.06, which the sum rounds to 127, unless the scale
+                // is subnormal (its rounding is coarser) or not finite: such blocks take the second form.
+                if (!__any_sync(ALL, (uint16_t)(sc - 0x400u) >= 0x7800u)) {
 #pragma unroll
-                for (int j = 0; j < NP; ++j) {
-                    const float2 f = pair(j);
-                    __half2 q = __floats2half2_rn(f.x * rsc, f.y * rsc);
-                    q = __hmax2(__hmin2(q, lim), nlim);
-                    q = __hadd2(q, magic);
-                    const uint32_t bits = *reinterpret_cast<uint32_t *>(&q);
-                    *reinterpret_cast<uint16_t *>(db + dense_byte(e0 + j * 8)) = (uint16_t)__byte_perm(bits, 0u, low_bytes);
-                }
-                if (any_out) {
+                    for (int k = 0; k < CK; ++k) {
+                        uint32_t h[4];
 #pragma unroll
-                    for (int i = 0; i < NM; ++i)
-                        for (uint32_t m = omask[i]; m; m &= m - 1) {
-                            const int bit = __ffs(m) - 1;
-                            const int pos = e0 + ((bit & 15) + i * 16) * 8 + (bit >> 4);
-                            atomicOr(&s_mask[pos >> 5], 1u << (pos & 31));
+                        for (int w = 0; w < 4; ++w) {
+                            const float2 f = h2f2(xw[k * 4 + w]);
+                            const float2 qf = unpack2(mul2(pack2(f.x, f.y), rsc2));
+                            const __half2 v = __hadd2(__floats2half2_rn(qf.x, qf.y), magic);
+                            h[w] = *reinterpret_cast<const uint32_t *>(&v);
                         }
+                        *reinterpret_cast<uint2 *>(db + dense_byte(at(b * CK + k))) =
+                            make_uint2(__byte_perm(h[0], h[1], 0x6420), __byte_perm(h[2], h[3], 0x6420));
+                    }
+                } else {
+                    // A NaN quotient is code 0.  It takes an infinity or a NaN among the values kept, which makes the scale
+                    // infinite or NaN and every other quotient of the block 0 or NaN: such a block gets zero bytes.
+                    const uint32_t finite = sc < 0x7c00u ? 0xffffffffu : 0u;
+                    const __half2 lim = __float2half2_rn(127.f), nlim = __float2half2_rn(-127.f);
+#pragma unroll
+                    for (int k = 0; k < CK; ++k) {
+                        uint32_t h[4];
+#pragma unroll
+                        for (int w = 0; w < 4; ++w) {
+                            const float2 f = h2f2(xw[k * 4 + w]);
+                            __half2 v = __floats2half2_rn(f.x * rsc, f.y * rsc);
+                            v = __hadd2(__hmax2(__hmin2(v, lim), nlim), magic);
+                            h[w] = *reinterpret_cast<const uint32_t *>(&v);
+                        }
+                        *reinterpret_cast<uint2 *>(db + dense_byte(at(b * CK + k))) =
+                            make_uint2(__byte_perm(h[0], h[1], 0x6420) & finite, __byte_perm(h[2], h[3], 0x6420) & finite);
+                    }
                 }
             }
-        }
-        __syncthreads();
-
-        // ---- exclusive scan of outliers per mask word --------------------------------
-        {
-            const uint32_t c = __popc(s_mask[tid]);  // QT_WORDS == QT_THREADS
-            uint32_t inc = c;
+            uint8_t *mb = reinterpret_cast<uint8_t *>(s.mask[buf]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)   // (blocks beyond the end of the tensor have no outliers)
+                mb[at(c) >> 3] = at(c) < tile_elems ? (uint8_t)(mask16[c >> 1] >> ((c & 1) * 8)) : (uint8_t)0;
+            __syncwarp();
+            const uint32_t own = __popc(s.mask[buf][tid]);
+            uint32_t inc = own;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                uint32_t n = __shfl_up_sync(0xffffffffu, inc, o);
+                const uint32_t n = __shfl_up_sync(ALL, inc, o);
                 if (lane >= o) inc += n;
             }
-            if (lane == 31) s_warp_tot[warp] = inc;
-            __syncthreads();
-            uint32_t wbase = 0;
-            for (int w = 0; w < warp; ++w) wbase += s_warp_tot[w];
-            s_wordpre[tid] = wbase + inc - c;
-            if (tid == QT_THREADS - 1) s_tile_total = (int)(wbase + inc);
+            s.word_before[buf][tid] = inc - own;
+            if (lane == 31) s.warp_total[buf][warp] = inc;
         }
         __syncthreads();
+        const unsigned int next = cur != NO_TILE ? s.tile[(i + 1) & 3] : NO_TILE;
+        const int next_item = next != NO_TILE ? s.item[(i + 1) & 3] : 0;
+        // the next tile's elements travel while the previous one is written out
+        if (next != NO_TILE) load_elements(p.item[next_item], ((int64_t)next - p.item[next_item].first_tile) * QT_TILE, at, x);
 
-        // ---- decoupled look-back over tiles (warp 0) -------------------------------------
-        if (warp == 0) {
-            const unsigned long long agg = (unsigned long long)s_tile_total;
-            long long prefix = 0;
-            if (tile == 0) {
-                if (lane == 0) st_relaxed_u64(p.status, ST_PREFIX | agg);
-            } else {
-                if (lane == 0) st_relaxed_u64(p.status + tile, ST_AGG | agg);
-                prefix = look_back(p.status, tile, lane, p.counts);
-                if (lane == 0) st_relaxed_u64(p.status + tile, ST_PREFIX | (unsigned long long)(prefix + (long long)agg));
-            }
-            if (lane == 0) {
-                s_tile_prefix = prefix;
-                if (tile == p.num_tiles - 1) {
-                    const long long total_out = prefix + (long long)agg;
-                    p.counts[0] = p.padded - total_out;
-                    p.counts[1] = total_out;
+        // ---- the previous tile, whose place in the streams is known by now -------------------------------
+        if (prev != NO_TILE) {
+            const QuantItem &q = p.item[prev_item];
+            const int64_t tile_base = ((int64_t)prev - q.first_tile) * QT_TILE;
+            const int tile_elems = (int)min((int64_t)QT_TILE, q.padded - tile_base);
+            const uint32_t *mask = s.mask[prev_buf], *base = s.warp_base[prev_buf], *word_before = s.word_before[prev_buf];
+            const uint8_t *dense = s.dense[prev_buf];
+            auto before = [&](int w) { return (int)(word_before[w] + base[w >> 5]); };
+            const long long tile_prefix = s.prefix[(i - 1) & 1];
+            const int64_t code_base = tile_base - tile_prefix;  // where this tile's codes start
+            const int shift = q.out_aligned ? (int)(code_base & 15) : 0;
+            // outliers, one mask word per thread; their values are read again
+            {
+                uint32_t word = mask[tid];
+                long long pos = tile_prefix + before(tid);
+                while (word) {
+                    const int64_t e = tile_base + tid * 32 + __ffs(word) - 1;
+                    word &= word - 1;
+                    if (pos < q.ocap) {
+                        q.ovals[pos] = e < q.numel ? __ldg(q.x + e) : (uint16_t)0;
+                        q.oidx[pos] = e;
+                    }
+                    ++pos;
                 }
             }
-        }
-        __syncthreads();
-
-        // ---- with the prefix: outliers straight out, one mask word per thread ------------------------
-        const long long tile_prefix = s_tile_prefix;
-        const int64_t code_base = tile_base - tile_prefix;  // where this tile's codes start
-        const int shift = p.out_aligned ? (int)(code_base & 15) : 0;
-        {
-            uint32_t word = s_mask[tid];   // QT_WORDS == QT_THREADS
-            long long pos = tile_prefix + s_wordpre[tid];
-            while (word) {
-                const int e = tid * 32 + __ffs(word) - 1;
-                word &= word - 1;
-                if (pos < p.ocap) {
-                    p.ovals[pos] = xref(e);
-                    p.oidx[pos] = tile_base + e;
-                }
-                ++pos;
-            }
-        }
-
-        // ---- the compacted codes, 16 bytes to an aligned global address per thread and step ------------------------
-        {
-            const int total = tile_elems - s_tile_total;  // code bytes of this tile
+            // the compacted codes, 16 bytes to an aligned global address per thread and step
+            const int total = tile_elems - (int)base[QF_WORKERS];  // code bytes of this tile
             const int end = shift + total;
-            int8_t *gdst = p.codes + (code_base - shift);  // 16-byte aligned when out_aligned
+            int8_t *gdst = q.codes + (code_base - shift);  // 16-byte aligned when out_aligned
             const int nchunks = (end + 15) >> 4;
-            const uint32_t *s32 = reinterpret_cast<const uint32_t *>(s_dense);
-            for (int c = tid; c < nchunks; c += QT_THREADS) {
+            const uint32_t *s32 = reinterpret_cast<const uint32_t *>(dense);
+            for (int c = tid; c < nchunks; c += QF_WORKERS * 32) {
                 const int lo = c << 4, a = max(lo, shift), z = min(lo + 16, end);
                 const int o0 = a - shift;                    // first code of the piece, counted in the tile
                 int w = o0 >> 5;                             // the mask word it lies in
-                while (w < QT_WORDS - 1 && (w + 1) * 32 - (int)s_wordpre[w + 1] <= o0) ++w;
-                const int skip = o0 - (w * 32 - (int)s_wordpre[w]);   // codes of that word in front of it
-                const uint32_t word = s_mask[w];
+                while (w < QT_WORDS - 1 && (w + 1) * 32 - before(w + 1) <= o0) ++w;
+                const int skip = o0 - (w * 32 - before(w));  // codes of that word in front of it
+                const uint32_t word = mask[w];
                 int in_word = skip;
                 if (word) {                                  // position of code number `skip` among the word's codes
-                    for (int i = 0; i < 32; ++i) {
-                        const int next = skip + __popc(word & (0xffffffffu >> (31 - min(in_word, 31))));
-                        if (next == in_word) break;
-                        in_word = next;
+                    for (int k = 0; k < 32; ++k) {
+                        const int next_at = skip + __popc(word & (0xffffffffu >> (31 - min(in_word, 31))));
+                        if (next_at == in_word) break;
+                        in_word = next_at;
                     }
                 }
                 const int pos = w * 32 + in_word;
                 // 20 dense codes from there and their outlier bits
-                uint32_t m = __funnelshift_r(s_mask[pos >> 5], s_mask[min((pos >> 5) + 1, QT_WORDS)], pos & 31) & 0xfffffu;
+                uint32_t m = __funnelshift_r(mask[pos >> 5], mask[min((pos >> 5) + 1, QT_WORDS)], pos & 31) & 0xfffffu;
                 uint32_t v[5];
                 {
                     const int wi = pos >> 2, r = (pos & 3) * 8;
                     uint32_t raw[6];
 #pragma unroll
-                    for (int i = 0; i < 6; ++i) raw[i] = s32[(wi + i) ^ ((((wi + i) >> 5) & 7) << 2)];
+                    for (int k = 0; k < 6; ++k) raw[k] = s32[(wi + k) ^ ((((wi + k) >> 5) & 3) << 3)];
 #pragma unroll
-                    for (int i = 0; i < 5; ++i) v[i] = __funnelshift_r(raw[i], raw[i + 1], r);
+                    for (int k = 0; k < 5; ++k) v[k] = __funnelshift_r(raw[k], raw[k + 1], r);
                 }
                 if (__popc(m) <= 4) {
                     while (m & 0xffffu) {                    // squeeze out the first outlier's place
                         const int j = __ffs(m) - 1, jw = j >> 2;
                         const uint32_t low = (1u << (8 * (j & 3))) - 1u;
 #pragma unroll
-                        for (int i = 0; i < 5; ++i) {
-                            const uint32_t down = __funnelshift_r(v[i], i < 4 ? v[i < 4 ? i + 1 : 4] : 0u, 8);
-                            v[i] = i < jw ? v[i] : (i == jw ? ((v[i] & low) | (down & ~low)) : down);
+                        for (int k = 0; k < 5; ++k) {
+                            const uint32_t down = __funnelshift_r(v[k], k < 4 ? v[k < 4 ? k + 1 : 4] : 0u, 8);
+                            v[k] = k < jw ? v[k] : (k == jw ? ((v[k] & low) | (down & ~low)) : down);
                         }
                         m = (m >> 1) & ~((1u << j) - 1u);
                     }
                 } else {                                     // dense outliers: code by code
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) v[i] = 0u;
-                    int q = pos;
+                    for (int k = 0; k < 4; ++k) v[k] = 0u;
+                    int at_e = pos;
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        if (a + i < z) {
-                            while ((s_mask[q >> 5] >> (q & 31)) & 1u) ++q;
-                            v[i >> 2] |= (uint32_t)s_dense[dense_byte(q)] << (8 * (i & 3));
-                            ++q;
+                    for (int k = 0; k < 16; ++k) {
+                        if (a + k < z) {
+                            while ((mask[at_e >> 5] >> (at_e & 31)) & 1u) ++at_e;
+                            v[k >> 2] |= (uint32_t)dense[dense_byte(at_e)] << (8 * (k & 3));
+                            ++at_e;
                         }
                     }
                 }
-                if (p.out_aligned && z - a == 16) {
+                if (q.out_aligned && z - a == 16) {
                     *reinterpret_cast<uint4 *>(gdst + lo) = make_uint4(v[0], v[1], v[2], v[3]);
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (a + i < z) gdst[a + i] = (int8_t)(v[i >> 2] >> (8 * (i & 3)));
+                    for (int k = 0; k < 16; ++k)
+                        if (a + k < z) gdst[a + k] = (int8_t)(v[k >> 2] >> (8 * (k & 3)));
                 }
             }
-            const int64_t block0 = tile_base / BS;
-            for (int b = tid; b < tile_blocks; b += QT_THREADS) p.scales[block0 + b] = s_scale[b];
         }
+        if (cur == NO_TILE) break;
+        prev = cur;
+        prev_item = cur_item;
+        cur = next;
+        cur_item = next_item;
     }
 }
 
@@ -743,6 +925,24 @@ FastConsts make_fast_consts(uint16_t thr_h) {
     else fc.T = 0.5f * (thr + __half2float(__ushort_as_half((uint16_t)(thr_h + 1))));
     if (!(thr_h & 0x8000u) && fc.T != INFINITY) fc.tie_out = thr_h & 1;
     return fc;
+}
+
+// ---- several copies in one launch ------------------------------------------------------------
+// A layer's fourteen outlier streams are 20 KB to 1 MB each: a copy's launch (4 us of host time) costs more than the copy.
+constexpr int CP_THREADS = 256;
+constexpr int CP_MAX_ITEMS = 32;
+struct CopyBatch {
+    AtlasCopyItem item[CP_MAX_ITEMS];
+    int n;
+};
+__global__ void __launch_bounds__(CP_THREADS) copy_many_kernel(const __grid_constant__ CopyBatch p) {
+    const AtlasCopyItem it = p.item[blockIdx.y];
+    const int64_t first = (int64_t)blockIdx.x * CP_THREADS + threadIdx.x, step = (int64_t)gridDim.x * CP_THREADS;
+    const bool vec = ((((uintptr_t)it.dst) | ((uintptr_t)it.src)) & 15) == 0;
+    const int64_t pieces = vec ? it.bytes >> 4 : 0;
+    for (int64_t i = first; i < pieces; i += step) reinterpret_cast<uint4 *>(it.dst)[i] = __ldg(reinterpret_cast<const uint4 *>(it.src) + i);
+    for (int64_t i = pieces * 16 + first; i < it.bytes; i += step)
+        reinterpret_cast<uint8_t *>(it.dst)[i] = __ldg(reinterpret_cast<const uint8_t *>(it.src) + i);
 }
 
 struct DeviceInfo {
@@ -785,72 +985,157 @@ size_t atlas_quantize_workspace_bytes(int64_t numel, int block_size) {
     return (size_t)(16 + 8 * tiles);
 }
 
-int atlas_quantize(const void *w, int64_t numel, int block_size, double z_threshold, int8_t *codes,
-                   void *outlier_vals, int64_t *outlier_idx, int64_t outlier_capacity, void *scales,
-                   int64_t *counts, void *workspace, size_t workspace_bytes, void *stream) {
+size_t atlas_quantize_many_workspace_bytes(int count, const AtlasQuantizeItem *items, int block_size) {
+    size_t bytes = 0;
+    for (int i = 0; items && i < count; ++i) bytes += atlas_quantize_workspace_bytes(items[i].numel, block_size);
+    return bytes;
+}
+
+int atlas_quantize_many(int count, const AtlasQuantizeItem *items, int block_size, double z_threshold,
+                        void *workspace, size_t workspace_bytes, void *stream) {
     using namespace atlas;
     clear_error();
-    ATLAS_RETURN_IF(numel < 0 || counts == nullptr || outlier_capacity < 0, ATLAS_ERR_BAD_ARGUMENT,
-                    "atlas_quantize: negative size or null counts");
+    ATLAS_RETURN_IF(count < 1 || !items, ATLAS_ERR_BAD_ARGUMENT, "atlas_quantize: no tensors");
+    for (int i = 0; i < count; ++i)
+        ATLAS_RETURN_IF(items[i].numel < 0 || items[i].counts == nullptr || items[i].outlier_capacity < 0, ATLAS_ERR_BAD_ARGUMENT,
+                        "atlas_quantize: negative size or null counts");
     ATLAS_RETURN_IF(block_size < 32 || block_size > 512 || block_size % 32 != 0, ATLAS_ERR_UNSUPPORTED,
                     "atlas_quantize: block_size %d is not a multiple of 32 in [32, 512]", block_size);
     int rc = check_device();
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    rc = check_cuda(cudaMemsetAsync(counts, 0, 4 * sizeof(int64_t), st), "memset(counts)");
-    if (rc) return rc;
-    if (numel == 0) return ATLAS_OK;
-    ATLAS_RETURN_IF(!w || !codes || !scales || !workspace ||
-                        (outlier_capacity > 0 && (!outlier_vals || !outlier_idx)),
-                    ATLAS_ERR_BAD_ARGUMENT, "atlas_quantize: null buffer");
-    const size_t need = atlas_quantize_workspace_bytes(numel, block_size);
-    ATLAS_RETURN_IF(workspace_bytes < need, ATLAS_ERR_CAPACITY,
-                    "atlas_quantize: workspace holds %zu bytes, %zu needed", workspace_bytes, need);
-    ATLAS_RETURN_IF(((uintptr_t)workspace & 15) != 0 || ((uintptr_t)w & 1) != 0 ||
-                        ((uintptr_t)outlier_idx & 7) != 0 || ((uintptr_t)counts & 7) != 0,
-                    ATLAS_ERR_BAD_ARGUMENT, "atlas_quantize: misaligned buffer");
-
-    QuantParams p;
-    p.x = (const uint16_t *)w;
-    p.numel = numel;
-    p.n_blocks = ceil_div_i64(numel, block_size);
-    p.padded = p.n_blocks * block_size;
-    p.tile = (QT_TILE / block_size) * block_size;
-    p.num_tiles = ceil_div_i64(p.padded, p.tile);
-    p.bs = block_size;
-    p.thr_h = __half_as_ushort(__float2half_rn((float)z_threshold));
-    p.codes = codes;
-    p.ovals = (uint16_t *)outlier_vals;
-    p.oidx = outlier_idx;
-    p.ocap = outlier_capacity;
-    p.scales = (uint16_t *)scales;
-    p.counts = counts;
-    p.tile_counter = (unsigned int *)workspace;
-    p.status = (unsigned long long *)((char *)workspace + 16);
-    p.in_aligned = ((uintptr_t)w & 15) == 0;
-    p.out_aligned = ((uintptr_t)codes & 15) == 0;
-
-    rc = check_cuda(cudaMemsetAsync(workspace, 0, need, st), "memset(workspace)");
-    if (rc) return rc;
+    size_t need = 0;   // (an empty tensor has no tiles)
+    bool counts_in_a_row = true;
+    for (int i = 0; i < count; ++i) {
+        const AtlasQuantizeItem &a = items[i];
+        if (i > 0) counts_in_a_row = counts_in_a_row && a.counts == items[i - 1].counts + 4;
+        if (a.numel == 0) continue;
+        ATLAS_RETURN_IF(!a.w || !a.codes || !a.scales || !workspace || (a.outlier_capacity > 0 && (!a.outlier_vals || !a.outlier_idx)),
+                        ATLAS_ERR_BAD_ARGUMENT, "atlas_quantize: null buffer");
+        need += atlas_quantize_workspace_bytes(a.numel, block_size);
+        ATLAS_RETURN_IF(workspace_bytes < need, ATLAS_ERR_CAPACITY,
+                        "atlas_quantize: workspace holds %zu bytes, %zu needed", workspace_bytes, need);
+        ATLAS_RETURN_IF(((uintptr_t)workspace & 15) != 0 || ((uintptr_t)a.w & 1) != 0 ||
+                            ((uintptr_t)a.outlier_idx & 7) != 0 || ((uintptr_t)a.counts & 7) != 0,
+                        ATLAS_ERR_BAD_ARGUMENT, "atlas_quantize: misaligned buffer");
+    }
+    const size_t counts_bytes = 4 * sizeof(int64_t);
+    if (counts_in_a_row && need && (char *)items[0].counts + count * counts_bytes == (char *)workspace) {
+        rc = check_cuda(cudaMemsetAsync(items[0].counts, 0, count * counts_bytes + need, st), "memset(counts, workspace)");
+        if (rc) return rc;
+    } else {
+        if (counts_in_a_row) {
+            rc = check_cuda(cudaMemsetAsync(items[0].counts, 0, count * counts_bytes, st), "memset(counts)");
+        } else {
+            for (int i = 0; i < count && !rc; ++i) rc = check_cuda(cudaMemsetAsync(items[i].counts, 0, counts_bytes, st), "memset(counts)");
+        }
+        if (rc) return rc;
+        if (need) rc = check_cuda(cudaMemsetAsync(workspace, 0, need, st), "memset(workspace)");
+        if (rc) return rc;
+    }
+    if (!need) return ATLAS_OK;
     DeviceInfo di;
     rc = device_info(di);
     if (rc) return rc;
+    const uint16_t thr_h = __half_as_ushort(__float2half_rn((float)z_threshold));
     const bool fast = block_size == 32 || block_size == 64 || block_size == 128 || block_size == 256;
-    const int per_sm = fast ? 5 : di.quant_ctas_per_sm;   // resident CTAs of the fast kernels
-    const int64_t max_ctas = (int64_t)di.sms * per_sm;
-    const int grid = (int)(p.num_tiles < max_ctas ? p.num_tiles : max_ctas);
-    if (fast) {
-        const FastConsts fc = make_fast_consts(p.thr_h);
-        switch (block_size) {
-            case 32: quantize_fast_kernel<32><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
-            case 64: quantize_fast_kernel<64><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
-            case 128: quantize_fast_kernel<128><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
-            default: quantize_fast_kernel<256><<<grid, QT_THREADS, 0, st>>>(p, fc); break;
+    const int64_t tile = (QT_TILE / block_size) * block_size;
+    char *ws = (char *)workspace;
+    if (!fast) {
+        for (int i = 0; i < count; ++i) {
+            const AtlasQuantizeItem &a = items[i];
+            if (a.numel == 0) continue;
+            QuantParams p;
+            p.x = (const uint16_t *)a.w;
+            p.numel = a.numel;
+            p.n_blocks = ceil_div_i64(a.numel, block_size);
+            p.padded = p.n_blocks * block_size;
+            p.tile = (int)tile;
+            p.num_tiles = ceil_div_i64(p.padded, tile);
+            p.bs = block_size;
+            p.thr_h = thr_h;
+            p.codes = a.codes;
+            p.ovals = (uint16_t *)a.outlier_vals;
+            p.oidx = a.outlier_idx;
+            p.ocap = a.outlier_capacity;
+            p.scales = (uint16_t *)a.scales;
+            p.counts = a.counts;
+            p.tile_counter = (unsigned int *)ws;
+            p.status = (unsigned long long *)(ws + 16);
+            p.in_aligned = ((uintptr_t)a.w & 15) == 0;
+            p.out_aligned = ((uintptr_t)a.codes & 15) == 0;
+            ws += atlas_quantize_workspace_bytes(a.numel, block_size);
+            const int64_t max_ctas = (int64_t)di.sms * di.quant_ctas_per_sm;
+            quantize_kernel<<<(int)(p.num_tiles < max_ctas ? p.num_tiles : max_ctas), QT_THREADS, 0, st>>>(p);
+            rc = check_cuda(cudaGetLastError(), "quantize_kernel launch");
+            if (rc) return rc;
         }
-        return check_cuda(cudaGetLastError(), "quantize_fast_kernel launch");
+        return ATLAS_OK;
     }
-    quantize_kernel<<<grid, QT_THREADS, 0, st>>>(p);
-    return check_cuda(cudaGetLastError(), "quantize_kernel launch");
+    const FastConsts fc = make_fast_consts(thr_h);
+    for (int i = 0; i < count;) {
+        QuantBatch b = {};
+        int64_t tiles = 0;
+        for (; i < count && b.n < QF_MAX_ITEMS; ++i) {
+            const AtlasQuantizeItem &a = items[i];
+            if (a.numel == 0) continue;
+            const int64_t padded = ceil_div_i64(a.numel, block_size) * block_size, own = ceil_div_i64(padded, tile);
+            if (b.n && tiles + own > 0x7fffffff) break;
+            b.item[b.n++] = {(const uint16_t *)a.w, a.codes, (uint16_t *)a.outlier_vals, a.outlier_idx, (uint16_t *)a.scales,
+                             a.counts, a.numel, padded, a.outlier_capacity, tiles, ((uintptr_t)a.w & 15) == 0, ((uintptr_t)a.codes & 15) == 0};
+            tiles += own;
+        }
+        if (b.n == 0) break;
+        ATLAS_RETURN_IF(tiles > 0x7fffffff, ATLAS_ERR_UNSUPPORTED, "atlas_quantize: tensor too large");
+        b.num_tiles = (unsigned int)tiles;
+        b.tile_counter = (unsigned int *)ws;
+        b.status = (unsigned long long *)(ws + 16);
+        ws += 16 + 8 * tiles;
+        const int64_t max_ctas = (int64_t)di.sms * QF_CTAS;
+        const int grid = (int)(tiles < max_ctas ? tiles : max_ctas);
+        switch (block_size) {
+            case 32: quantize_fast_kernel<32><<<grid, QF_THREADS, 0, st>>>(b, fc); break;
+            case 64: quantize_fast_kernel<64><<<grid, QF_THREADS, 0, st>>>(b, fc); break;
+            case 128: quantize_fast_kernel<128><<<grid, QF_THREADS, 0, st>>>(b, fc); break;
+            default: quantize_fast_kernel<256><<<grid, QF_THREADS, 0, st>>>(b, fc); break;
+        }
+        rc = check_cuda(cudaGetLastError(), "quantize_fast_kernel launch");
+        if (rc) return rc;
+    }
+    return ATLAS_OK;
+}
+
+int atlas_quantize(const void *w, int64_t numel, int block_size, double z_threshold, int8_t *codes,
+                   void *outlier_vals, int64_t *outlier_idx, int64_t outlier_capacity, void *scales,
+                   int64_t *counts, void *workspace, size_t workspace_bytes, void *stream) {
+    const AtlasQuantizeItem item = {w, numel, codes, outlier_vals, outlier_idx, outlier_capacity, scales, counts};
+    return atlas_quantize_many(1, &item, block_size, z_threshold, workspace, workspace_bytes, stream);
+}
+
+int atlas_copy_many(int count, const AtlasCopyItem *items, void *stream) {
+    using namespace atlas;
+    clear_error();
+    ATLAS_RETURN_IF(count < 0 || (count && !items), ATLAS_ERR_BAD_ARGUMENT, "atlas_copy_many: bad count");
+    for (int i = 0; i < count; ++i)
+        ATLAS_RETURN_IF(items[i].bytes < 0 || (items[i].bytes && (!items[i].dst || !items[i].src)), ATLAS_ERR_BAD_ARGUMENT,
+                        "atlas_copy_many: null buffer or negative length");
+    int rc = check_device();
+    if (rc) return rc;
+    for (int i = 0; i < count;) {
+        CopyBatch b = {};
+        int64_t longest = 0;
+        for (; i < count && b.n < CP_MAX_ITEMS; ++i) {
+            if (!items[i].bytes) continue;
+            b.item[b.n++] = items[i];
+            if (items[i].bytes > longest) longest = items[i].bytes;
+        }
+        if (b.n == 0) break;
+        const int64_t want = ceil_div_i64(longest, CP_THREADS * 16);
+        copy_many_kernel<<<dim3((unsigned)(want < 64 ? want : 64), (unsigned)b.n), CP_THREADS, 0, (cudaStream_t)stream>>>(b);
+        rc = check_cuda(cudaGetLastError(), "copy_many_kernel launch");
+        if (rc) return rc;
+    }
+    return ATLAS_OK;
 }
 
 }  // extern "C"

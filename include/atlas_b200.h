@@ -81,6 +81,34 @@ ATLAS_API int atlas_quantize(const void *w, int64_t numel, int block_size, doubl
                    int64_t outlier_capacity, void *scales, int64_t *counts,
                    void *workspace, size_t workspace_bytes, void *stream);
 
+/* Several tensors at a time, with one block size and threshold: what atlas_quantize does for each.  For block sizes
+ * 32 / 64 / 128 / 256 up to 16 tensors share one launch, so that the GPU does not run empty between them; others are
+ * launched one by one.  `counts` of an item is its own 4 x int64; items whose counts lie behind one another are cleared
+ * by one memset, and by the workspace's own if the workspace follows them.  workspace: 16-byte aligned,
+ * atlas_quantize_many_workspace_bytes(count, items, block_size) bytes. */
+typedef struct AtlasQuantizeItem {
+    const void *w;
+    int64_t numel;
+    int8_t *codes;
+    void *outlier_vals;
+    int64_t *outlier_idx;
+    int64_t outlier_capacity;
+    void *scales;
+    int64_t *counts;
+} AtlasQuantizeItem;
+ATLAS_API size_t atlas_quantize_many_workspace_bytes(int count, const AtlasQuantizeItem *items, int block_size);
+ATLAS_API int atlas_quantize_many(int count, const AtlasQuantizeItem *items, int block_size, double z_threshold,
+                                  void *workspace, size_t workspace_bytes, void *stream);
+
+/* `count` device-to-device copies of any length and alignment, 32 to a launch: the outlier streams of freshly quantized
+ * tensors go from their roomy buffers to buffers of their own length.  Sources and destinations must not overlap. */
+typedef struct AtlasCopyItem {
+    void *dst;
+    const void *src;
+    int64_t bytes;
+} AtlasCopyItem;
+ATLAS_API int atlas_copy_many(int count, const AtlasCopyItem *items, void *stream);
+
 /* ---- quantize for callers that cannot allocate -------------------------------
  * No counterpart in the reference.  Same computation and outputs as
  * atlas_quantize, but the look-back scratch lives in a device array inside the
