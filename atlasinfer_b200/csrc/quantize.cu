@@ -3,7 +3,7 @@
 // Replaces quantize_tensor (atlasinfer_core/quant/adaptive_quantizer.py:51-148).
 // The reference walks the blocks in a Python loop and concatenates four
 // streams; here a persistent grid takes tiles of 8192 elements in order
-// (dynamic tile ids), evaluates every block of a tile in shared memory, and
+// (dynamic tile ids), evaluates every block of a tile on chip, and
 // finds where the tile's compacted codes and outliers start in the output
 // through a decoupled look-back over per-tile outlier counts, so the input is
 // read once and every output byte is written once.
@@ -326,13 +326,20 @@ __global__ void __launch_bounds__(QT_THREADS) quantize_kernel(QuantParams p) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Fast variant for block sizes 32 / 64 / 128 / 256.  Same results as quantize_kernel above, bit for bit, at a quarter of
-// its instructions: 121 us for 11008 x 4096 in blocks of 128 back to back, 128 with L2 flushed before (165 back to back with
-// guard bands around the roundings and byte-wise compaction), 46 % of the issue slots used, the rest mostly the barriers around the look-back.
+// Fast variant for block sizes 32 / 64 / 128 / 256, up to 16 tensors per launch.  Same results as quantize_kernel above, bit
+// for bit.  11008 x 4096 in blocks of 128: 120 us, 54 M warp instructions, 43 % of the issue slots used; the seven weights of
+// a 7B-shaped layer in one launch instead of seven, with their outliers copied by one kernel instead of fourteen copies:
+// 777 -> 600 us through quantize_tensors.
 //
-// Four threads work on a block; thread t plays ATen's SIMD lanes 2t and 2t + 1, whose elements are neighbours, so the
-// values stay packed two to a register and most steps cost one instruction per pair.  What replaces the IEEE divisions
-// and the fp64 moment, and why the results are the same:
+// Eight warps of a CTA hold a tile's elements in registers, a ninth numbers the tiles and looks back.  A tile's codes and
+// outlier mask stay in shared memory while the next tile is worked on, and are written out after it: by then its place in
+// the streams is known, and the elements of the tile after that are on their way.  A tile so costs one CTA barrier.  What
+// the warps wait for is that barrier (8 of 20 cycles per instruction) and the loads (5 of 20).
+//
+// Four threads work on a block (eight on one of 256); thread t holds the 8-wide chunks t, t + 4, ..., that is ATen's
+// accumulator t of all eight SIMD lanes, so that a chunk is one 16-byte load; the accumulators change hands through 1 KB of
+// shared memory per warp.  Values stay packed two to a register and most steps cost one instruction per pair (fp32 pairs:
+// add, mul and fma.rn.f32x2).  What replaces the IEEE divisions and the fp64 moment, and why the results are the same:
 //   * code.  x and the scale have 11-bit significands, so a quotient x / scale is never the midpoint of two fp16 numbers
 //     (scale times a midpoint's odd 12-bit significand needs more than 11 bits) and is more than 2^-23 away from one,
 //     relatively: |a 2^k - m b| >= 1 with m < 2^12, b < 2^11.  x * (1 / scale), two roundings to fp32, is within 2^-23:
@@ -347,10 +354,10 @@ __global__ void __launch_bounds__(QT_THREADS) quantize_kernel(QuantParams p) {
 //   * standard deviation.  fp32 sum of squares minus the squared sum, if the mean takes less than a fifth of it away, else a
 //     second pass about the mean; only if rounding it to fp16 could go either way within 4e-6 is it recomputed in fp64
 //     (about 1 % of blocks).  The bound, with u = 2^-24, Q the sum of squares, M = Q - F^2 / n the second moment and blocks
-//     of 256, the longest sums: Q carries 31 additions of a thread and 3 across threads, 34 u Q.  F carries 7 + 3 in a lane
+//     of 256, the longest sums: Q carries at most 31 additions of a thread and 3 across threads, 34 u Q.  F carries 7 + 3 in a lane
 //     and 7 over the lanes, 17 u sum|x| <= 17 u sqrt(n Q), and |F| <= sqrt(0.2 n Q) here, so F^2 / n is off by
 //     2 * 0.45 * 17 u Q = 15 u Q.  With Q <= 1.25 M that is 62 u of M, 31 u of its root, and 4 u for the product, the root
-//     and the rounding of M: 35 u = 2.1e-6.  The second pass adds 64 times (66 u with the shuffles, 2 u for the squared
+//     and the rounding of M: 35 u = 2.1e-6.  The second pass adds at most 64 times (66 u with the shuffles, 2 u for the squared
 //     differences), 34 u of the root, and 4 u as above: 2.3e-6; the mean it is taken about enters only through r1^2 / n,
 //     which is small because values that round in F make the block spread by a thirtieth of the largest at least.  (The
 //     largest error in an emulation over 4.8 M blocks of six kinds, offsets and wide exponents among them: 6.5e-7.)
