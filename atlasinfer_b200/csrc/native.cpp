@@ -1,4 +1,4 @@
-// Host path of the quantized linear and of the quantizer: argument checks, allocations and launches in one native call.
+// Host path of the quantized linear, of its weight layouts and of the quantizer: argument checks, allocations and launches in one native call.
 //
 // A decode step of a small model is bound by the host, not the GPU: a linear takes 3 to 15 us on the device, and the
 // same checks, allocations and argument marshalling cost 15 us a call in Python.  Semantics and errors are those of the
@@ -7,7 +7,10 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
+
+#include <atomic>
 
 #include "atlas_b200.h"
 
@@ -23,6 +26,61 @@ void check(int status, const char *what) {
 }
 
 const void *ptr_or_null(const at::Tensor &t) { return t.numel() ? t.data_ptr() : nullptr; }
+
+// Stands for a layout that may still be written by the stream it was enqueued on.  The linear kernels read weights before
+// the stream's earlier work has completed (programmatic dependent launch), but no kernel of that stream starts before the
+// one that writes the layout has ended, since that one does not let others start early.  So only a use on another stream, or
+// in a capture, whose kernels run who knows where, has to wait; it waits on the host, once.
+class LayoutReady {
+   public:
+    LayoutReady() {
+        device_ = at::cuda::current_device();
+        stream_ = at::cuda::getCurrentCUDAStream(device_).stream();
+        C10_CUDA_CHECK(cudaEventCreateWithFlags(&event_, cudaEventDisableTiming));
+        C10_CUDA_CHECK(cudaEventRecord(event_, stream_));
+    }
+    ~LayoutReady() { cudaEventDestroy(event_); }
+    LayoutReady(const LayoutReady &) = delete;
+    // True once the layout is final.  False: not yet, but work enqueued on the current stream comes after it.
+    bool wait() {
+        if (done_.load(std::memory_order_acquire)) return true;
+        const cudaStream_t on = at::cuda::getCurrentCUDAStream(device_).stream();
+        // (none of these calls touches a capture of this or another thread)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(on, &capture);
+        bool done = false;
+        if (e == cudaSuccess && on == stream_ && capture == cudaStreamCaptureStatusNone) {
+            const cudaError_t q = cudaEventQuery(event_);
+            done = q == cudaSuccess;
+            if (q == cudaErrorNotReady) (void)cudaGetLastError();
+            else e = q;
+        } else if (e == cudaSuccess) {
+            e = cudaEventSynchronize(event_);
+            done = e == cudaSuccess;
+        }
+        const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
+        C10_CUDA_CHECK(e);
+        C10_CUDA_CHECK(back);
+        if (done) done_.store(true, std::memory_order_release);
+        return done;
+    }
+    void finish() {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaEventSynchronize(event_), back = cudaThreadExchangeStreamCaptureMode(&mode);
+        C10_CUDA_CHECK(e);
+        C10_CUDA_CHECK(back);
+        done_.store(true, std::memory_order_release);
+    }
+
+   private:
+    int device_;
+    cudaStream_t stream_;
+    cudaEvent_t event_ = nullptr;
+    std::atomic<bool> done_{false};
+};
 
 // x @ W^T + bias for a kernel layout; `gemv` chooses the per-strip kernel, else the tcgen05 kernels.
 at::Tensor linear(const at::Tensor &x, const at::Tensor &tiles, const at::Tensor &scales, const at::Tensor &chunk_ptr,
@@ -145,9 +203,78 @@ std::vector<std::array<at::Tensor, 4>> quantize_many(const std::vector<at::Tenso
     return out;
 }
 
+// The kernel layouts of `members` (codes, outlier values, outlier positions, scales, rows; one device, K and block size) as
+// the rows of one layout: tiles, scales, CSR row pointers (of a single tensor), chunk pointers, entries, values.  Enqueued,
+// not waited for.
+std::array<at::Tensor, 6> build_layout(const std::vector<std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, int64_t>> &members,
+                                       int64_t k, int64_t bs) {
+    const at::Tensor &first = std::get<0>(members[0]);
+    const c10::cuda::CUDAGuard guard(first.device());
+    const c10::cuda::CUDAStream stream = at::cuda::getCurrentCUDAStream(first.get_device());
+    int64_t rows_padded = 0, n_out = 0;
+    for (const auto &m : members) {
+        rows_padded += (std::get<4>(m) + 127) / 128 * 128;
+        n_out += std::get<2>(m).numel();
+    }
+    const int64_t chunks = k / 64 + 1;
+    const auto opt = first.options();
+    at::Tensor tiles = at::empty({rows_padded * k}, opt.dtype(at::kByte)), scales = at::empty({rows_padded * (k / bs)}, opt.dtype(at::kHalf));
+    at::Tensor row_ptr = at::empty({members.size() == 1 ? std::get<4>(members[0]) + 1 : 0}, opt.dtype(at::kInt));
+    at::Tensor chunk_ptr = at::empty({rows_padded / 16 * chunks}, opt.dtype(at::kInt));
+    at::Tensor entries = at::empty({n_out}, opt.dtype(at::kInt)), vals = at::empty({n_out}, opt.dtype(at::kHalf));
+    std::vector<AtlasRepackItem> items;
+    std::vector<at::Tensor> held;   // alive until the kernel is enqueued
+    int64_t row = 0, entry = 0;
+    for (const auto &m : members) {
+        const at::Tensor codes = std::get<0>(m).contiguous(), ovals = std::get<1>(m).contiguous(), oidx = std::get<2>(m).contiguous(),
+                         sc = std::get<3>(m).contiguous();
+        const int64_t n = std::get<4>(m);
+        AtlasRepackItem item = {};
+        item.codes = (const int8_t *)ptr_or_null(codes);
+        item.n_codes = codes.numel();
+        item.outlier_vals = ptr_or_null(ovals);
+        item.outlier_idx = (const int64_t *)ptr_or_null(oidx);
+        item.n_outliers = oidx.numel();
+        item.scales = sc.data_ptr();
+        item.n_rows = n;
+        item.n_cols = k;
+        item.block_size = bs;
+        item.tiles = (uint8_t *)tiles.data_ptr() + row * k;
+        item.scales_tiled = (char *)scales.data_ptr() + row * (k / bs) * 2;
+        item.outlier_row_ptr = members.size() == 1 ? (int32_t *)row_ptr.data_ptr() : nullptr;
+        item.outlier_chunk_ptr = (int32_t *)chunk_ptr.data_ptr() + row / 16 * chunks;
+        if (n_out) {
+            item.outlier_entries = (uint32_t *)entries.data_ptr() + entry;
+            item.outlier_vals_sorted = (char *)vals.data_ptr() + entry * 2;
+        }
+        item.entry_base = entry;
+        items.push_back(item);
+        // the streams may be freed, by another stream's owner too, before the kernel has read them
+        for (const at::Tensor &t : {codes, ovals, oidx, sc}) {
+            if (t.numel()) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
+            held.push_back(t);
+        }
+        row += (n + 127) / 128 * 128;
+        entry += oidx.numel();
+    }
+    check(atlas_repack_many((int)items.size(), items.data(), stream.stream()), "atlas_repack");
+    return {tiles, scales, row_ptr, chunk_ptr, entries, vals};
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    py::class_<LayoutReady, std::shared_ptr<LayoutReady>>(m, "LayoutReady")
+        .def(py::init<>())
+        .def("wait", &LayoutReady::wait, py::call_guard<py::gil_scoped_release>())
+        .def("__reduce__", [](LayoutReady &r) {   // copied or saved: what it stands for is final first, and nothing is left to wait for
+            {
+                py::gil_scoped_release release;
+                r.finish();
+            }
+            return py::make_tuple(py::type::of(py::none()), py::tuple());
+        });
+    m.def("build_layout", &build_layout, py::call_guard<py::gil_scoped_release>());
     m.def("quantize_many", &quantize_many, py::call_guard<py::gil_scoped_release>());
     m.def("linear", &linear, py::call_guard<py::gil_scoped_release>());
 }

@@ -47,6 +47,7 @@ class KernelLayout(NamedTuple):
     n_rows: int
     n_cols: int
     block_size: int
+    ready: object = None           # while the buffers may still be written: what a use on another stream waits for
 
 
 _status_words = {}
@@ -105,65 +106,46 @@ def kernel_layout_supported(shape, block_size: int) -> Optional[str]:
     return None
 
 
-def build_kernel_layout(q: QuantizedTensor) -> KernelLayout:
+def build_kernel_layout(q: QuantizedTensor, wait: bool = True) -> KernelLayout:
     """Expand the compacted code stream of ``q`` (on a CUDA device) into the kernel layout."""
-    return build_joined_layout([q])[0]
+    return build_joined_layout([q], wait)[0]
 
 
-def build_joined_layout(qs):
+def build_joined_layout(qs, wait: bool = True):
     """The kernel layouts of ``qs`` (one device, in_features and block size) as the rows of one layout, back to back.
 
     Returns ``(layout, row offsets)``.  Every member but the last is padded to whole 128-row tiles, as in
     ``concat_layouts``, but the members are expanded straight into the joined buffers by one launch.  The CSR row
-    pointers of the canonical streams are only written for a single tensor."""
+    pointers of the canonical streams are only written for a single tensor.
+
+    With ``wait`` the buffers are final on return.  Without, ``layout.ready`` stands for the work under way:
+    ``quantized_linear_forward`` may be called at once, any other use outside the current stream waits for it."""
     for q in qs:
         reason = kernel_layout_supported(q.original_shape, int(q.block_size))
         if reason is not None:
             raise NotImplementedError("QuantizedLinear: " + reason)
-    L = _capi.load()
     dev = qs[0].fp8_data.device
     k, bs = int(qs[0].original_shape[1]), int(qs[0].block_size)
     if any((int(q.original_shape[1]), int(q.block_size)) != (k, bs) for q in qs):
         raise ValueError("fused linears must share in_features and block size")
     rows = [int(q.original_shape[0]) for q in qs]
-    padded = [(n + 127) // 128 * 128 for n in rows]
-    n_pad, n_out = sum(padded), sum(q.outlier_indices.numel() for q in qs)
-    chunks = k // 64 + 1
-    with torch.cuda.device(dev):
-        tiles = torch.empty(n_pad * k, dtype=torch.uint8, device=dev)
-        scales_tiled = torch.empty(n_pad * (k // bs), dtype=torch.float16, device=dev)
-        row_ptr = torch.empty(rows[0] + 1 if len(qs) == 1 else 0, dtype=torch.int32, device=dev)
-        chunk_ptr = torch.empty((n_pad // 16) * chunks, dtype=torch.int32, device=dev)
-        entries = torch.empty(n_out, dtype=torch.int32, device=dev)
-        vals_sorted = torch.empty(n_out, dtype=torch.float16, device=dev)
-        items = (_capi.RepackItem * len(qs))()
-        offsets, held, row, entry = [], [], 0, 0
-        for item, q, n, n_p in zip(items, qs, rows, padded):
-            codes, oidx = q.fp8_data.contiguous(), q.outlier_indices.contiguous()
-            ovals, scales = q.fp16_outliers.contiguous(), q.scale_factors.contiguous()
-            held.append((codes, oidx, ovals, scales))   # alive until the kernel has read them
-            item.codes, item.n_codes = _capi.ptr(codes), codes.numel()
-            item.outlier_vals, item.outlier_idx, item.n_outliers = _capi.ptr(ovals), _capi.ptr(oidx), oidx.numel()
-            item.scales, item.n_rows, item.n_cols, item.block_size = scales.data_ptr(), n, k, bs
-            item.tiles = tiles.data_ptr() + row * k
-            item.scales_tiled = scales_tiled.data_ptr() + row * (k // bs) * 2
-            item.outlier_row_ptr = _capi.ptr(row_ptr)
-            item.outlier_chunk_ptr = chunk_ptr.data_ptr() + (row // 16) * chunks * 4
-            if n_out:
-                item.outlier_entries = entries.data_ptr() + entry * 4
-                item.outlier_vals_sorted = vals_sorted.data_ptr() + entry * 2
-            item.entry_base = entry
-            offsets.append(row)
-            row += n_p
-            entry += oidx.numel()
-        status = L.atlas_repack_many(len(qs), items, _capi.stream_ptr(dev))
-    _capi.check(status, "atlas_repack")
-    # the linear kernels read the weight-side buffers before the stream's earlier work has completed
-    # (programmatic dependent launch), so the layout must be final before any of them is launched
-    torch.cuda.current_stream(dev).synchronize()
+    native = _capi.native()
+    if torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream(dev).synchronize()   # raises: a layout must not live in a graph's memory
+    members = [(q.fp8_data, q.fp16_outliers, q.outlier_indices, q.scale_factors, n) for q, n in zip(qs, rows)]
+    buffers = native.build_layout(members, k, bs)
+    ready = None
+    if wait:
+        torch.cuda.current_stream(dev).synchronize()
+    else:
+        with torch.cuda.device(dev):
+            ready = native.LayoutReady()
+    offsets, row = [], 0
+    for n in rows:
+        offsets.append(row)
+        row += (n + 127) // 128 * 128
     source = qs[0] if len(qs) == 1 else tuple(qs)
-    return KernelLayout(source, tiles, scales_tiled, row_ptr, chunk_ptr, entries, vals_sorted,
-                        n_pad - padded[-1] + rows[-1], k, bs), offsets
+    return KernelLayout(source, *buffers, offsets[-1] + rows[-1], k, bs, ready), offsets
 
 
 def quantized_linear_forward(x: torch.Tensor, layout: KernelLayout, bias: Optional[torch.Tensor],
@@ -182,6 +164,8 @@ def quantized_linear_forward(x: torch.Tensor, layout: KernelLayout, bias: Option
         gemv_rows = _ANY_ROWS if force == "gemv" else 0
     else:
         raise ValueError(f"force={force!r}")
+    if layout.ready is not None:
+        layout.ready.wait()
     return _capi.native().linear(x, layout.tiles, layout.scales_tiled, layout.chunk_ptr, layout.entries, layout.vals_sorted,
                                  layout.n_rows, layout.n_cols, layout.block_size, bias, status_word(x.device), gemv_rows)
 
@@ -193,6 +177,8 @@ def _stream_forward(x: torch.Tensor, layout: KernelLayout, bias: Optional[torch.
     n, k = layout.n_rows, layout.n_cols
     if x.shape[-1] != k:
         raise RuntimeError(f"QuantizedLinear: input has {x.shape[-1]} features, weight expects {k}")
+    if layout.ready is not None:
+        layout.ready.wait()
     x2 = x.reshape(-1, k)
     if x2.stride(-1) != 1 or (x2.shape[0] > 1 and x2.stride(0) < k):
         x2 = x2.contiguous()
@@ -224,6 +210,8 @@ def concat_layouts(layouts) -> KernelLayout:
     k_tiles = first.n_cols // 64
     chunk_ptrs, base = [], 0
     for l in layouts:
+        if l.ready is not None:
+            l.ready.wait()
         chunk_ptrs.append(l.chunk_ptr + base)          # entry indices become positions in the joined list
         base += l.entries.numel()
     padded = [(l.n_rows + 127) // 128 * 128 for l in layouts]
@@ -247,7 +235,7 @@ def slice_layout(fused: KernelLayout, row_offset: int, n_rows: int, source, entr
     t0, s0, c0 = row_offset * k, row_offset * (k // bs), (row_offset // 16) * (k_tiles + 1)
     return KernelLayout(source, fused.tiles[t0:t0 + n_pad * k], fused.scales_tiled[s0:s0 + n_pad * (k // bs)],
                         fused.row_ptr, fused.chunk_ptr[c0:c0 + (n_pad // 16) * (k_tiles + 1)],
-                        fused.entries, fused.vals_sorted, n_rows, k, bs)
+                        fused.entries, fused.vals_sorted, n_rows, k, bs, fused.ready)
 
 
 class FusedLinearGroup:
@@ -291,7 +279,7 @@ class FusedLinearGroup:
                 self.offsets.append(off)
                 off += (lay.n_rows + 127) // 128 * 128
         else:
-            fused, self.offsets = build_joined_layout(sources)
+            fused, self.offsets = build_joined_layout(sources, wait=False)
         rows = [int(q.original_shape[0]) for q in sources]
         if any(mod.bias is not None for mod in self.members):
             b = torch.zeros(fused.n_rows, dtype=torch.float16, device=dev)
@@ -299,11 +287,15 @@ class FusedLinearGroup:
                 if mod.bias is not None:
                     b[o:o + n] = mod.bias.to(torch.float16)
             self.bias = b
+            if fused.ready is not None:   # the bias is part of what a use waits for
+                with torch.cuda.device(dev):
+                    fused = fused._replace(ready=_capi.native().LayoutReady())
         # the members now look at the joined buffers; their own copies are released
         for mod, q, n, o in zip(self.members, sources, rows, self.offsets):
             mod._kernel_layout = slice_layout(fused, o, n, q)
         self.layout = fused
-        torch.cuda.current_stream(dev).synchronize()
+        if fused.ready is None:
+            torch.cuda.current_stream(dev).synchronize()
 
     def member_forward(self, index: int, x: torch.Tensor) -> Optional[torch.Tensor]:
         """Member ``index``'s output for ``x``, or None if the group does not apply (the member computes alone)."""
@@ -311,6 +303,8 @@ class FusedLinearGroup:
             return None
         if self.layout is None or self.layout.tiles.device != x.device:
             self.build(x.device)
+        elif self.layout.ready is not None and self.layout.ready.wait():
+            self.layout = self.layout._replace(ready=None)
         c = self._cache
         if c is None or c[0] is not x or c[1] != x._version or index in c[3]:
             y_all = quantized_linear_forward(x, self.layout, self.bias)
@@ -368,7 +362,7 @@ class QuantizedLinear(nn.Module):
 
     def _layout_for(self, q: QuantizedTensor) -> KernelLayout:
         if not self._has_layout_for(q):
-            self._kernel_layout = build_kernel_layout(q)
+            self._kernel_layout = build_kernel_layout(q, wait=False)
         return self._kernel_layout
 
     def offload_canonical(self, device="cpu") -> None:
@@ -402,6 +396,8 @@ class QuantizedLinear(nn.Module):
         bias = self.bias
         if lay is not None and lay.source is q_tensor and x.is_cuda and lay.tiles.device == x.device and (
                 bias is None or bias.device == x.device):
+            if lay.ready is not None and lay.ready.wait():
+                self._kernel_layout = lay = lay._replace(ready=None)
             return quantized_linear_forward(x, lay, self._bias_for(bias))
         # the kernels need a GPU; CPU activations are staged through it and the result returned
         compute_device = x.device if x.device.type == "cuda" else _capi.require_cuda()
