@@ -3,25 +3,30 @@
 //
 // Replaces dequantize_tensor (atlasinfer_core/quant/adaptive_quantizer.py:156-251).
 // The reference keeps a running offset into the code stream and, per block,
-// masks the whole outlier index list (:194-196, O(blocks x outliers)).  Here the
-// sorted outlier index list is searched once per span of 16384 elements: the
-// number of outliers before the span both locates the span's outliers and
-// gives the span's offset into the compacted code stream (position minus
-// outliers before it), so every span is independent.
+// masks the whole outlier index list (:194-196, O(blocks x outliers)).  Here a
+// first kernel finds, for all spans of 8192 elements in one pass over the sorted
+// index list, where a span's outliers begin and end; the number of outliers
+// before the span gives its offset into the compacted code stream (position
+// minus outliers before it), so every span is independent.
 //
-// Both directions only move bytes: HBM is the bound (1.04 bytes read per element, 2 or 1 written).  A span's outlier
-// positions become a bit mask with a prefix count per word, its codes are staged with 16-byte loads, and a thread
-// builds 16 bytes of output at a time: one unaligned read of the staged codes, a zero byte slipped in per set bit
-// (an outlier sits in every 20th such unit), one 16-byte store.
+// Both directions only move bytes: HBM is the bound in principle (1.04 bytes read per element, 2 or 1 written), memory latency
+// and instructions in practice.  A span's outlier positions become a bit mask with a code offset per word, its codes are
+// staged with 16-byte copies, and a thread builds 16 bytes of output at a time from one unaligned read of the staged codes;
+// units that hold outliers (every 20th to 40th) are left out of that and built afterwards, one per thread.
+// 11008 x 4096 in blocks of 128: dequantize 52.7 -> 34.9 us (3.9 TB/s; 4096 x 4096 27.2 -> 18.5, 512 x 512 9.3 -> 6.3) against a
+// search of four dependent round trips per span of 16384 and zero bytes slipped in per outlier under divergence; repack
+// 45.2 -> 47 (4096 x 4096 20.6 -> 21.2, 4096 x 11008 45.2 -> 45.5): its strips' lists take as long.  Spans of 4096 and CTAs of
+// 128 threads: 33.6 and 44, but 62 for the repack of 4096 x 11008, whose strips hold 530 outliers.
 #include "common.cuh"
 
 namespace atlas {
 namespace {
 
 constexpr int DQ_THREADS = 256;
-constexpr int DQ_SPAN = 16384;                // padded elements per CTA
-constexpr int DQ_WORDS = DQ_SPAN / 32;        // outlier-mask words: two per thread
-static_assert(DQ_WORDS == 2 * DQ_THREADS, "two mask words per thread");
+constexpr int DQ_SPAN = 8192;                 // padded elements per CTA
+constexpr int DQ_WORDS = DQ_SPAN / 32;        // outlier-mask words
+static_assert(DQ_WORDS == DQ_THREADS, "a mask word per thread");
+constexpr int64_t DQ_SEARCHED = 1024;         // up to as many outliers a CTA searches for its own: two round trips
 constexpr int DQ_MAX_REPACK = 8;              // tensors one repack launch takes
 constexpr int RP_STRIP_CAP = 2560;            // outliers of a strip kept in shared memory (16 x 4096 weights: 200 at 0.3 %)
 constexpr int RP_SCALE_KB = 16;               // scale blocks per CTA of the scale transposition (one 32-byte sector a row)
@@ -40,54 +45,82 @@ __device__ __forceinline__ int64_t warp_lower_bound(const int64_t *idx, int64_t 
     return lo + __popc(__ballot_sync(0xffffffffu, lo + lane < hi && __ldg(idx + lo + lane) < key));
 }
 
+// Where a span's outliers are in the outlier list is found beforehand, by one pass over the list in a kernel of its own:
+// every thread compares two neighbours, which is one round trip to memory (2 to 3 us here) for all spans together, where a
+// search is four for each.  Both ends go to the first 16 bytes of the span's own output, which the span's CTA reads and
+// overwrites; no other memory is needed.
+struct Ends {
+    int64_t lo, hi;
+};
+// Thread i's part of it: the spans that begin after outlier i - 1 and not after outlier i.  `put(span)` is where a span's
+// ends go.  A whole warp calls it: long runs of spans without outliers are shared out.
+template <class Put>
+__device__ __forceinline__ void mark_spans(const int64_t *oidx, int64_t n_out, int64_t spans, int64_t i, int lane, const Put &put) {
+    int64_t first = 1, last = 0;
+    if (i <= n_out) {
+        first = i > 0 ? max((int64_t)0, __ldg(oidx + i - 1) / DQ_SPAN + 1) : 0;
+        last = i < n_out ? min(__ldg(oidx + i) / DQ_SPAN, spans) : spans;
+    }
+    auto mark = [&](int64_t s, int64_t at) {
+        if (s < spans) put(s)->lo = at;
+        if (s > 0) put(s - 1)->hi = at;
+    };
+    const bool many = last - first >= 8;
+    if (!many)
+        for (int64_t s = first; s <= last; ++s) mark(s, i);
+    for (unsigned m = __ballot_sync(0xffffffffu, many); m; m &= m - 1) {
+        const int from = __ffs(m) - 1;
+        const int64_t f = __shfl_sync(0xffffffffu, first, from), l = __shfl_sync(0xffffffffu, last, from), at = __shfl_sync(0xffffffffu, i, from);
+        for (int64_t s = f + lane; s <= l; s += 32) mark(s, at);
+    }
+}
+
 struct Span {
-    __align__(16) uint32_t mask[DQ_WORDS];                  // bit p: position p of the span is an outlier
-    __align__(16) uint32_t before[DQ_WORDS];                // outliers of the span before the word
+    uint32_t mask[DQ_WORDS];                  // bit p: position p of the span is an outlier
+    uint32_t start[DQ_WORDS];                 // where the word's first code lies in `codes`
     uint32_t warp_total[DQ_THREADS / 32];
     int64_t lo, hi;                           // the span's outliers in the outlier streams
     __align__(16) uint8_t codes[DQ_SPAN + 48];
-    int shift;                                // where the span's first code sits in `codes` (the misalignment of its address)
 };
 
-// Stages the span [span0, span1): mask, prefix counts and codes.  Nothing outside codes[0, n_codes) and oidx[0, n_out)
-// is read, whatever oidx holds; if it is not ascending (a damaged file) the values are arbitrary, but hi >= lo keeps the
-// staged length within the span and, as every bit of the mask stands for an index in [lo, hi), the outliers read within
-// [lo, hi) too.
-__device__ __forceinline__ void stage_span(Span &s, const int8_t *codes, int64_t n_codes, const int64_t *oidx,
-                                           int64_t n_out, int64_t span0, int64_t span1) {
+// Stages the span [span0, span1), whose outliers are [lo, hi): mask, code offsets and codes.  Nothing outside
+// codes[0, n_codes) and oidx[0, n_out) is read, whatever oidx and the ends hold; if oidx is not ascending (a damaged file) the
+// values are arbitrary, but hi >= lo keeps the staged length within the span and, as every bit of the mask stands for an index
+// in [lo, hi), the outliers read within [lo, hi) too.
+__device__ __forceinline__ void stage_span(Span &s, const int8_t *codes, int64_t n_codes, const int64_t *oidx, int64_t n_out, Ends ends,
+                                           int64_t span0, int64_t span1) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    *reinterpret_cast<uint2 *>(s.mask + 2 * tid) = make_uint2(0u, 0u);
-    if (warp < 2) {
-        const int64_t r = warp_lower_bound(oidx, n_out, warp == 0 ? span0 : span1, lane);
-        if (lane == 0) (warp == 0 ? s.lo : s.hi) = r;
-    }
-    __syncthreads();
-    const int64_t lo = s.lo, hi = max(lo, s.hi);
-    for (int64_t i = lo + tid; i < hi; i += DQ_THREADS) {
-        const int64_t p = __ldg(oidx + i) - span0;
-        if (p >= 0 && p < DQ_SPAN) atomicOr(&s.mask[p >> 5], 1u << (p & 31));
+    const int64_t lo = max((int64_t)0, min(ends.lo, n_out)), hi = max(lo, min(ends.hi, n_out));
+    const int64_t first = lo + tid < hi ? __ldg(oidx + lo + tid) - span0 : -1;   // (a span has 12 at 0.3 %)
+    s.mask[tid] = 0u;
+    if (tid == 0) {
+        s.lo = lo;
+        s.hi = hi;
     }
     const int64_t c0 = span0 - lo;            // the span's first code
     const int len = (int)max((int64_t)0, span1 - span0 - (hi - lo));
     const int shift = (int)((uintptr_t)(codes + c0) & 15);
-    if (tid == 0) s.shift = shift;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s.codes);
     for (int c = tid; c * 16 < shift + len; c += DQ_THREADS) {
         const int64_t g = c0 - shift + c * 16;
-        uint4 v;
         if (g >= 0 && g + 16 <= n_codes) {
-            v = __ldg(reinterpret_cast<const uint4 *>(codes + g));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * 16), "l"(codes + g) : "memory");
         } else {
             uint32_t w[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
             for (int e = 0; e < 16; ++e)
                 if (g + e >= 0 && g + e < n_codes) w[e >> 2] |= (uint32_t)(uint8_t)codes[g + e] << (8 * (e & 3));
-            v = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4 *>(s.codes + c * 16) = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        *reinterpret_cast<uint4 *>(s.codes + c * 16) = v;
     }
     __syncthreads();
-    const uint2 words = *reinterpret_cast<const uint2 *>(s.mask + 2 * tid);
-    const uint32_t own = __popc(words.x) + __popc(words.y);
+    if (first >= 0 && first < DQ_SPAN) atomicOr(&s.mask[first >> 5], 1u << (first & 31));
+    for (int64_t i = lo + tid + DQ_THREADS; i < hi; i += DQ_THREADS) {
+        const int64_t p = __ldg(oidx + i) - span0;
+        if (p >= 0 && p < DQ_SPAN) atomicOr(&s.mask[p >> 5], 1u << (p & 31));
+    }
+    __syncthreads();
+    const uint32_t own = __popc(s.mask[tid]);
     uint32_t inc = own;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -98,36 +131,49 @@ __device__ __forceinline__ void stage_span(Span &s, const int8_t *codes, int64_t
     __syncthreads();
     uint32_t base = 0;
     for (int w = 0; w < warp; ++w) base += s.warp_total[w];
-    *reinterpret_cast<uint2 *>(s.before + 2 * tid) = make_uint2(base + inc - own, base + inc - __popc(words.y));
+    s.start[tid] = (uint32_t)(shift + tid * 32) - (base + inc - own);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 }
 
-// The 4 * W codes of the unit that starts at position p of the span (p a multiple of 4 * W, W = 2 or 4), biased by 128;
-// an outlier's place holds code 0.  `bits` are its outliers, `before` the span's outliers in front of it.
+// Byte of the staged codes where position p's code lies, or would, and the outliers of the 32 positions p is among.
+__device__ __forceinline__ uint32_t code_at(const Span &s, int p, uint32_t &word) {
+    word = s.mask[p >> 5];
+    return s.start[p >> 5] + (uint32_t)(p & 31) - (uint32_t)__popc(word & ((1u << (p & 31)) - 1u));
+}
+// The 4 * W codes from byte `o` of the staged codes on, biased by 128.
 template <int W>
-__device__ __forceinline__ void span_unit(const Span &s, int p, uint32_t (&w)[W], uint32_t &bits, int &before) {
-    const uint32_t word = s.mask[p >> 5];
-    bits = (word >> (p & 31)) & ((1u << (4 * W)) - 1u);
-    before = (int)s.before[p >> 5] + __popc(word & ((1u << (p & 31)) - 1u));
-    const int o = s.shift + p - before, r = (o & 3) * 8;
+__device__ __forceinline__ void codes_at(const Span &s, uint32_t o, uint32_t (&w)[W]) {
     const uint32_t *src = reinterpret_cast<const uint32_t *>(s.codes) + (o >> 2);
+    const uint32_t r = (o & 3u) * 8u;
     uint32_t raw[W + 1];
 #pragma unroll
     for (int i = 0; i <= W; ++i) raw[i] = src[i];
 #pragma unroll
-    for (int i = 0; i < W; ++i) w[i] = __funnelshift_r(raw[i], raw[i + 1], r);
-    for (uint32_t m = bits; m; m &= m - 1) {   // a zero byte in the outlier's place, the later codes move up by one
-        const int j = __ffs(m) - 1, jw = j >> 2;
-        const uint32_t low = (1u << (8 * (j & 3))) - 1u;
+    for (int i = 0; i < W; ++i) w[i] = __funnelshift_r(raw[i], raw[i + 1], r) ^ 0x80808080u;
+}
+// The same for positions with outliers (`bits`) among them: code 0 in their places.
+template <int W>
+__device__ __forceinline__ void codes_around(const Span &s, uint32_t o, uint32_t bits, uint32_t (&w)[W]) {
 #pragma unroll
-        for (int i = W - 1; i >= 0; --i) {
-            const uint32_t up = i > 0 ? __funnelshift_l(w[i > 0 ? i - 1 : 0], w[i], 8) : w[i] << 8;
-            const uint32_t here = (w[i] & low) | ((w[i] & ~low) << 8);
-            w[i] = i > jw ? up : (i == jw ? here : w[i]);
-        }
+    for (int i = 0; i < W; ++i) w[i] = 0u;
+#pragma unroll
+    for (int e = 0; e < 4 * W; ++e) {
+        const bool out = (bits >> e) & 1u;
+        const uint32_t code = out ? 0x80u : (uint32_t)s.codes[o] ^ 0x80u;
+        o += out ? 0u : 1u;
+        w[e >> 2] |= code << (8 * (e & 3));
     }
-#pragma unroll
-    for (int i = 0; i < W; ++i) w[i] ^= 0x80808080u;
+}
+// Calls f(unit) in one thread for every unit (2^SHIFT positions) of the span that holds outliers.  Work per element is what
+// bounds these kernels beside latency, and most warps have some outlier: so units without are written first, without a
+// branch, and those with afterwards, one per thread.
+template <int SHIFT, class F>
+__device__ __forceinline__ void for_units_with_outliers(const Span &s, const int64_t *oidx, int64_t span0, const F &f) {
+    for (int64_t i = s.lo + threadIdx.x; i < s.hi; i += DQ_THREADS) {
+        const int64_t p = __ldg(oidx + i) - span0, before = i > s.lo ? __ldg(oidx + i - 1) - span0 : -1;
+        if (p >= 0 && p < DQ_SPAN && (before < 0 || before >> SHIFT != p >> SHIFT)) f((int)(p >> SHIFT));
+    }
 }
 
 // Two biased codes of a word (bytes 0, 1 or 2, 3) as fp16(code), exact.
@@ -138,66 +184,109 @@ __device__ __forceinline__ __half2 code_pair(uint32_t w) {
     return __hsub2(*reinterpret_cast<const __half2 *>(&h), bias);
 }
 
-// 8 elements (16 bytes of output) per thread and step.  The product of the code and the scale is rounded to fp16 once
-// (adaptive_quantizer.py:216).  11008 x 4096 in blocks of 128:
-// 50 us (2.7 TB/s).  With one binary search per element and 2-byte stores the seven weights of a 7B-shaped layer took
-// 1316 us through the API, now 275.
-__global__ void __launch_bounds__(DQ_THREADS)
-dequantize_kernel(const int8_t *codes, int64_t n_codes, const uint16_t *ovals, const int64_t *oidx,
-                  int64_t n_out, const uint16_t *scales, int64_t numel, int64_t padded, int bs, int bs_shift,
-                  int w_aligned, uint16_t *w) {
+__device__ __forceinline__ void scale_unit(const uint32_t (&c)[2], uint16_t scale, uint32_t (&o)[4]) {
+    const __half2 s2 = __half2half2(__ushort_as_half(scale));
+    __half2 h[4] = {code_pair<0x5140>(c[0]), code_pair<0x5342>(c[0]), code_pair<0x5140>(c[1]), code_pair<0x5342>(c[1])};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        h[i] = __hmul2(h[i], s2);
+        o[i] = *reinterpret_cast<uint32_t *>(&h[i]);
+    }
+}
+
+struct DequantParams {
+    const int8_t *codes;
+    int64_t n_codes;
+    const uint16_t *ovals;
+    const int64_t *oidx;
+    int64_t n_out;
+    const uint16_t *scales;
+    int64_t numel, padded, spans;
+    int bs, bs_shift, w_aligned;
+    int marked;                               // the spans' ends are where mark_dequant_kernel puts them
+    uint16_t *w;
+};
+__global__ void __launch_bounds__(256) mark_dequant_kernel(DequantParams p) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    mark_spans(p.oidx, p.n_out, p.spans, (int64_t)blockIdx.x * 256 + threadIdx.x, threadIdx.x & 31,
+               [&](int64_t span) { return reinterpret_cast<Ends *>(p.w + span * DQ_SPAN); });
+}
+
+// One unit (8 elements, 16 bytes of output) per thread and step.  The product of the code and the scale is rounded to fp16
+// once (adaptive_quantizer.py:216).
+__global__ void __launch_bounds__(DQ_THREADS) dequantize_kernel(DequantParams p) {
     __shared__ Span s;
-    const int64_t span0 = (int64_t)blockIdx.x * DQ_SPAN;
-    const int64_t span1 = min(span0 + DQ_SPAN, padded);
-    stage_span(s, codes, n_codes, oidx, n_out, span0, span1);
-    const int64_t out_lo = s.lo;
-#pragma unroll 1
-    for (int p = threadIdx.x * 8; p < DQ_SPAN; p += DQ_THREADS * 8) {
-        const int64_t gp = span0 + p;
-        if (gp >= numel) break;
-        uint32_t c[2], bits;
-        int before;
-        span_unit<2>(s, p, c, bits, before);
-        __half2 h[4] = {code_pair<0x5140>(c[0]), code_pair<0x5342>(c[0]), code_pair<0x5140>(c[1]), code_pair<0x5342>(c[1])};
-        if ((bs & 7) == 0) {                   // the unit lies in one block
-            const int64_t b = bs_shift >= 0 ? gp >> bs_shift : gp / bs;
-            const __half2 sc = __half2half2(__ushort_as_half(__ldg(scales + b)));
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t span0 = (int64_t)blockIdx.x * DQ_SPAN, span1 = min(span0 + DQ_SPAN, p.padded);
+    const bool whole = span0 + DQ_SPAN <= p.numel && p.w_aligned && p.bs_shift >= 3;   // blocks of whole units
+    constexpr int STEPS = DQ_SPAN / (DQ_THREADS * 8);
+    uint16_t sc[STEPS];
+    const uint32_t in_block = whole ? (uint32_t)(span0 & (p.bs - 1)) : 0u;
+    const uint16_t *scales = p.scales + (whole ? span0 >> p.bs_shift : 0);
+    auto scale_of = [&](int unit) { return __ldg(scales + ((in_block + (uint32_t)unit * 8u) >> p.bs_shift)); };
 #pragma unroll
-            for (int i = 0; i < 4; ++i) h[i] = __hmul2(h[i], sc);
-        } else {
+    for (int k = 0; k < STEPS; ++k) sc[k] = whole ? scale_of(tid + k * DQ_THREADS) : (uint16_t)0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint16_t *w = p.w + span0;
+    Ends ends;
+    if (p.marked && span0 + 8 <= p.numel) {
+        const volatile Ends *at = reinterpret_cast<const volatile Ends *>(w);   // (all threads, before any of them writes)
+        ends = {at->lo, at->hi};
+    } else {
+        if (warp < 2) {
+            const int64_t r = warp_lower_bound(p.oidx, p.n_out, warp == 0 ? span0 : span1, lane);
+            if (lane == 0) (warp == 0 ? s.lo : s.hi) = r;
+        }
+        __syncthreads();
+        ends = {s.lo, s.hi};
+        __syncthreads();
+    }
+    stage_span(s, p.codes, p.n_codes, p.oidx, p.n_out, ends, span0, span1);
+    if (whole) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int64_t b0 = min((gp + 2 * i) / bs, (padded - 1) / bs), b1 = min((gp + 2 * i + 1) / bs, (padded - 1) / bs);
-                h[i] = __hmul2(h[i], __halves2half2(__ushort_as_half(__ldg(scales + b0)), __ushort_as_half(__ldg(scales + b1))));
+        for (int k = 0; k < STEPS; ++k) {
+            const int unit = tid + k * DQ_THREADS;
+            uint32_t word, c[2], o[4];
+            const uint32_t at = code_at(s, unit * 8, word);
+            codes_at<2>(s, at, c);
+            scale_unit(c, sc[k], o);
+            if (!((word >> ((unit & 3) * 8)) & 0xffu)) *reinterpret_cast<uint4 *>(w + unit * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+        for_units_with_outliers<3>(s, p.oidx, span0, [&](int unit) {
+            uint32_t word, c[2], o[4];
+            const uint32_t at = code_at(s, unit * 8, word), bits = (word >> ((unit & 3) * 8)) & 0xffu;
+            const uint32_t before = (uint32_t)((uintptr_t)(p.codes + (span0 - s.lo)) & 15) + (uint32_t)unit * 8u - at;   // outliers in front
+            const uint16_t *val = p.ovals + s.lo + before;
+            codes_around<2>(s, at, bits, c);
+            scale_unit(c, scale_of(unit), o);
+            for (uint32_t m = bits; m; m &= m - 1, ++val) {
+                const int j = __ffs(m) - 1;
+                const uint32_t v = __ldg(val);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (q == j >> 1) o[q] = (j & 1) ? __byte_perm(o[q], v, 0x5410) : __byte_perm(o[q], v, 0x3254);
             }
-        }
-        uint32_t o[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] = *reinterpret_cast<uint32_t *>(&h[i]);
-        int64_t k = out_lo + before;
-        for (uint32_t m = bits; m; m &= m - 1, ++k) {
-            const int j = __ffs(m) - 1;
-            const uint32_t v = __ldg(ovals + k);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (i == j >> 1) o[i] = (j & 1) ? __byte_perm(o[i], v, 0x5410) : __byte_perm(o[i], v, 0x3254);
-        }
-        if (w_aligned && gp + 8 <= numel) {
-            *reinterpret_cast<uint4 *>(w + gp) = make_uint4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<uint4 *>(w + unit * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+        });
+        return;
+    }
+    // the last span, any block size, any alignment: element by element
+    for (int e = tid; e < DQ_SPAN && span0 + e < p.numel; e += DQ_THREADS) {
+        const int64_t gp = span0 + e;
+        uint32_t word;
+        const uint32_t at = code_at(s, e, word);
+        if ((word >> (e & 31)) & 1u) {
+            w[e] = __ldg(p.ovals + s.lo + ((uint32_t)((uintptr_t)(p.codes + (span0 - s.lo)) & 15) + (uint32_t)e - at));
         } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (gp + e < numel) w[gp + e] = (uint16_t)(o[e >> 1] >> (16 * (e & 1)));
+            const __half code = __short2half_rn((short)(int8_t)s.codes[at]);
+            w[e] = __half_as_ushort(__hmul(code, __ushort_as_half(__ldg(p.scales + (p.bs_shift >= 0 ? gp >> p.bs_shift : gp / p.bs)))));
         }
     }
 }
 
-// Byte offset of weight (row, col) inside the tile-major layout.
+// Byte offset of weight (row, col) inside the tile-major layout: 128-row x 64-column tiles, row by row.
 __device__ __forceinline__ int64_t tile_offset(int64_t row, int64_t col, int64_t k_tiles) {
-    const int64_t rt = row >> 7, kt = col >> 6;
-    const int strip = (int)(row & 127) >> 4, h = (int)(row & 15) >> 3, g = (int)(row & 7);
-    const int tig = (int)(col & 63) >> 4, byte = (int)(col & 15);
-    return ((((rt * k_tiles + kt) * 8 + strip) * 2 + h) * 32 + (g * 4 + tig)) * 16 + byte;
+    return ((row >> 7) * k_tiles + (col >> 6)) * 8192 + (row & 127) * 64 + (col & 63);
 }
 
 struct RepackTensor {
@@ -269,8 +358,18 @@ __device__ __forceinline__ void write_strip(const RepackTensor &t, int64_t strip
     }
 }
 
+__global__ void __launch_bounds__(256) mark_repack_kernel(const __grid_constant__ RepackParams p) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const RepackTensor &t = p.t[blockIdx.y];
+    const int64_t spans = (t.n_rows * t.n_cols + DQ_SPAN - 1) / DQ_SPAN;
+    mark_spans(t.oidx, t.n_out, spans, (int64_t)blockIdx.x * 256 + threadIdx.x, threadIdx.x & 31, [&](int64_t span) {
+        const int64_t at = span * DQ_SPAN, row = at / t.n_cols;
+        return reinterpret_cast<Ends *>(t.tiles + tile_offset(row, at - row * t.n_cols, t.n_cols >> 6));
+    });
+}
+
 // One launch expands up to DQ_MAX_REPACK tensors; a CTA does one of three jobs: the outlier lists of a strip (first in
-// the grid: the longest chain of dependent loads), a 128-row x 16-block piece of the scale transposition, or 16384
+// the grid: the longest chain of dependent loads), a 128-row x 16-block piece of the scale transposition, or 8192
 // positions of the code tiles, 16 codes (one unit of the layout; n_cols is a multiple of 64, so a unit never straddles
 // rows) per thread and step.  Rows beyond n_rows in the last 128-row tile get code 0 and scale 0.
 __global__ void __launch_bounds__(DQ_THREADS) repack_kernel(const __grid_constant__ RepackParams p) {
@@ -283,39 +382,62 @@ __global__ void __launch_bounds__(DQ_THREADS) repack_kernel(const __grid_constan
 
     if (blockIdx.x < t.strip_end) {
         const int64_t strip = blockIdx.x - begin;
-        for (int r = warp; r < 17; r += DQ_THREADS / 32) {
-            const int64_t row = min(strip * 16 + r, t.n_rows);
-            const int64_t at = warp_lower_bound(t.oidx, t.n_out, row * t.n_cols, lane);
-            if (lane == 0) sh.strip.row_at[r] = at;
+        const int64_t strip0 = strip * 16 * t.n_cols, strip1 = max(strip0, min(strip * 16 + 16, t.n_rows) * t.n_cols);
+        const uint32_t n_cols = (uint32_t)t.n_cols;   // (a strip has at most 2^28 positions)
+        StripScratch &s = sh.strip;
+        if (warp < 2) {
+            const int64_t at = warp_lower_bound(t.oidx, t.n_out, warp == 0 ? strip0 : strip1, lane);
+            if (lane == 0) s.row_at[warp * 16] = at;
         }
         __syncthreads();
-        const int64_t first = sh.strip.row_at[0];
-        const int total = (int)(sh.strip.row_at[16] - first);
-        if (t.row_ptr && tid < 17 && strip * 16 + tid <= t.n_rows && (tid < 16 || strip * 16 + 16 == t.n_rows))
-            t.row_ptr[strip * 16 + tid] = (int32_t)sh.strip.row_at[tid];
+        const int64_t first = s.row_at[0], end = max(first, s.row_at[16]);
+        const int total = (int)(end - first);
+        __syncthreads();
         // The ranks below are a permutation, and what the linear kernels index with the entries lies in the strip, only if
-        // the strip's positions ascend and its rows begin where the searches say.  A strip of which that is not true (a
-        // damaged file) gets an empty list.
-        const int64_t strip0 = strip * 16 * t.n_cols, strip1 = min(strip * 16 + 16, t.n_rows) * t.n_cols;
-        const uint32_t n_cols = (uint32_t)t.n_cols;   // (a strip has at most 2^28 positions)
+        // the strip's positions ascend and lie in it; then its rows begin where the rows of two neighbours differ (which takes
+        // one more round trip to memory, where a search per row took four, three times over).
         int bad = 0;
-        if (tid < 17) {
-            const int64_t at = sh.strip.row_at[tid], end = sh.strip.row_at[16], key = min(strip0 + tid * t.n_cols, strip1);
-            bad = at < first || at > end || (tid < 16 && sh.strip.row_at[tid + 1] < at);
-            if (!bad) bad = (at > first && __ldg(t.oidx + at - 1) >= key) || (at < end && __ldg(t.oidx + at) < key);
+        for (int i = tid; i < total && total <= RP_STRIP_CAP; i += DQ_THREADS) {
+            const int64_t at = __ldg(t.oidx + first + i) - strip0, before = i > 0 ? __ldg(t.oidx + first + i - 1) - strip0 : -1;
+            if (before >= at || at < 0 || at >= strip1 - strip0) {
+                bad = 1;
+            } else {
+                const int row = (int)((uint32_t)at / n_cols), above = before >= 0 ? (int)((uint32_t)before / n_cols) : -1;
+                s.col[i] = (uint32_t)at - (uint32_t)row * n_cols;
+                for (int r = above + 1; r <= row; ++r) s.row_at[r] = first + i;
+                if (i == total - 1)
+                    for (int r = row + 1; r <= 16; ++r) s.row_at[r] = end;
+            }
         }
-        for (int i = tid; i < total; i += DQ_THREADS) {
-            const int64_t *at = t.oidx + first + i;
-            bad |= i > 0 && __ldg(at - 1) >= __ldg(at);
-            if (i < RP_STRIP_CAP) sh.strip.col[i] = (uint32_t)(__ldg(at) - strip0) % n_cols;
+        if (total == 0 && tid < 17) s.row_at[tid] = first;
+        bad = __syncthreads_or(bad);
+        if (bad || total > RP_STRIP_CAP) {
+            // Many outliers, or a damaged file: a search per row.  A strip whose positions do not ascend or whose rows do not
+            // begin where the searches say gets an empty list.
+            for (int r = warp; r < 17; r += DQ_THREADS / 32) {
+                const int64_t at = warp_lower_bound(t.oidx, t.n_out, min(strip * 16 + r, t.n_rows) * t.n_cols, lane);
+                if (lane == 0) s.row_at[r] = at;
+            }
+            __syncthreads();
+            if (!bad) {
+                if (tid < 17) {
+                    const int64_t at = s.row_at[tid], key = min(strip0 + tid * t.n_cols, strip1);
+                    bad = at < first || at > end || (tid < 16 && s.row_at[tid + 1] < at);
+                    if (!bad) bad = (at > first && __ldg(t.oidx + at - 1) >= key) || (at < end && __ldg(t.oidx + at) < key);
+                }
+                for (int i = tid + 1; i < total; i += DQ_THREADS) bad |= __ldg(t.oidx + first + i - 1) >= __ldg(t.oidx + first + i);
+            }
+            bad = __syncthreads_or(bad);
         }
-        if (__syncthreads_or(bad)) {
+        if (t.row_ptr && tid < 17 && strip * 16 + tid <= t.n_rows && (tid < 16 || strip * 16 + 16 == t.n_rows))
+            t.row_ptr[strip * 16 + tid] = (int32_t)s.row_at[tid];
+        if (bad) {
             const int n_chunks = (int)(n_cols >> 6);
             for (int c = tid; c <= n_chunks; c += DQ_THREADS) t.chunk_ptr[strip * (n_chunks + 1) + c] = (int32_t)(t.entry_base + first);
         } else if (total <= RP_STRIP_CAP) {
-            write_strip(t, strip, sh.strip, [&](int i) { return sh.strip.col[i]; });
+            write_strip(t, strip, s, [&](int i) { return s.col[i]; });
         } else {
-            write_strip(t, strip, sh.strip, [&](int i) { return (uint32_t)(__ldg(t.oidx + first + i) - strip0) % n_cols; });
+            write_strip(t, strip, s, [&](int i) { return (uint32_t)(__ldg(t.oidx + first + i) - strip0) % n_cols; });
         }
         return;
     }
@@ -339,16 +461,47 @@ __global__ void __launch_bounds__(DQ_THREADS) repack_kernel(const __grid_constan
     const int64_t span1 = min(span0 + DQ_SPAN, numel);
     const int64_t row0 = span0 / t.n_cols;
     const uint32_t col0 = (uint32_t)(span0 - row0 * t.n_cols), n_cols = (uint32_t)t.n_cols;
-    if (span0 < numel) stage_span(sh.span, t.codes, t.n_codes, t.oidx, t.n_out, span0, span1);
-#pragma unroll 1
-    for (int q = tid * 16; q < DQ_SPAN; q += DQ_THREADS * 16) {
-        if (span0 + q >= padded) break;
-        uint32_t w[4] = {0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u}, bits;
-        int before;
-        if (span0 + q < numel) span_unit<4>(sh.span, q, w, bits, before);
-        const uint32_t c = col0 + (uint32_t)q, dr = c / n_cols;
-        *reinterpret_cast<uint4 *>(t.tiles + tile_offset(row0 + dr, c - dr * n_cols, n_cols >> 6)) = make_uint4(w[0], w[1], w[2], w[3]);
+    const uint32_t k_tiles = n_cols >> 6, in_tile = (uint32_t)row0 & 127u;
+    uint8_t *tiles = t.tiles + (row0 >> 7) * (int64_t)k_tiles * 8192;
+    auto place = [&](uint32_t q) -> uint8_t * {
+        const uint32_t c = col0 + q, dr = c / n_cols, col = c - dr * n_cols, row = in_tile + dr;
+        return tiles + ((uint64_t)((row >> 7) * k_tiles + (col >> 6)) * 8192u + (row & 127u) * 64u + (col & 63u));
+    };
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the marks
+    if (span0 < numel) {
+        const volatile Ends *at = reinterpret_cast<const volatile Ends *>(place(0));   // (all threads, before any of them writes)
+        stage_span(sh.span, t.codes, t.n_codes, t.oidx, t.n_out, Ends{at->lo, at->hi}, span0, span1);
     }
+#pragma unroll
+    for (int k = 0; k < DQ_SPAN / (DQ_THREADS * 16); ++k) {
+        const int q = tid * 16 + k * DQ_THREADS * 16;
+        if (span0 + q >= padded) break;
+        uint32_t w[4] = {0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u}, word = 0u;
+        if (span0 + q < numel) codes_at<4>(sh.span, code_at(sh.span, q, word), w);
+        if (!((word >> (q & 31)) & 0xffffu)) *reinterpret_cast<uint4 *>(place(q)) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    if (span0 < numel)
+        for_units_with_outliers<4>(sh.span, t.oidx, span0, [&](int unit) {
+            uint32_t word, w[4];
+            const uint32_t at = code_at(sh.span, unit * 16, word);
+            codes_around<4>(sh.span, at, (word >> ((unit & 1) * 16)) & 0xffffu, w);
+            *reinterpret_cast<uint4 *>(place(unit * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
+        });
+}
+
+// Launches a kernel whose CTAs may start while the marking kernel in front of it still runs.
+template <class Kernel, class Params>
+int launch_beside(Kernel kernel, unsigned grid, bool beside, cudaStream_t st, const Params &p) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(DQ_THREADS);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = beside ? 1 : 0;
+    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, p), "dequantize / repack launch");
 }
 
 }  // namespace
@@ -372,13 +525,29 @@ int atlas_dequantize(const int8_t *codes, int64_t n_codes, const void *outlier_v
                     ATLAS_ERR_BAD_ARGUMENT, "atlas_dequantize: null buffer");
     int rc = check_device();
     if (rc) return rc;
-    const int64_t grid = ceil_div_i64(padded, DQ_SPAN);
-    ATLAS_RETURN_IF(grid > 0x7fffffff, ATLAS_ERR_UNSUPPORTED, "atlas_dequantize: tensor too large");
-    const int bs_shift = (block_size & (block_size - 1)) == 0 ? __builtin_ctz((unsigned)block_size) : -1;
-    dequantize_kernel<<<(unsigned)grid, DQ_THREADS, 0, (cudaStream_t)stream>>>(
-        codes, n_codes, (const uint16_t *)outlier_vals, outlier_idx, n_outliers, (const uint16_t *)scales,
-        numel, padded, block_size, bs_shift, ((uintptr_t)w_out & 15) == 0, (uint16_t *)w_out);
-    return check_cuda(cudaGetLastError(), "dequantize_kernel launch");
+    const int64_t spans = ceil_div_i64(padded, DQ_SPAN);
+    ATLAS_RETURN_IF(spans > 0x7fffffff, ATLAS_ERR_UNSUPPORTED, "atlas_dequantize: tensor too large");
+    DequantParams p;
+    p.codes = codes;
+    p.n_codes = n_codes;
+    p.ovals = (const uint16_t *)outlier_vals;
+    p.oidx = outlier_idx;
+    p.n_out = n_outliers;
+    p.scales = (const uint16_t *)scales;
+    p.numel = numel;
+    p.padded = padded;
+    p.spans = ceil_div_i64(numel, DQ_SPAN) - (numel % DQ_SPAN > 0 && numel % DQ_SPAN < 8 ? 1 : 0);   // those with room for their ends
+    p.bs = block_size;
+    p.bs_shift = (block_size & (block_size - 1)) == 0 ? __builtin_ctz((unsigned)block_size) : -1;
+    p.w_aligned = ((uintptr_t)w_out & 15) == 0;
+    p.marked = p.w_aligned && n_outliers > DQ_SEARCHED;
+    p.w = (uint16_t *)w_out;
+    if (p.marked) {
+        mark_dequant_kernel<<<(unsigned)ceil_div_i64(n_outliers + 1, 256), 256, 0, (cudaStream_t)stream>>>(p);
+        rc = check_cuda(cudaGetLastError(), "mark_dequant_kernel launch");
+        if (rc) return rc;
+    }
+    return launch_beside(dequantize_kernel, (unsigned)spans, p.marked, (cudaStream_t)stream, p);
 }
 
 size_t atlas_tiles_bytes(int64_t n_rows, int64_t n_cols) {
@@ -443,8 +612,12 @@ int atlas_repack_many(int count, const AtlasRepackItem *items, void *stream) {
             end += strips + scale_ctas + code_ctas;
             t.block_end = (uint32_t)end;
         }
-        repack_kernel<<<(unsigned)end, DQ_THREADS, 0, (cudaStream_t)stream>>>(p);
-        rc = check_cuda(cudaGetLastError(), "repack_kernel launch");
+        int64_t most = 0;
+        for (int i = 0; i < p.n; ++i) most = p.t[i].n_out > most ? p.t[i].n_out : most;
+        mark_repack_kernel<<<dim3((unsigned)ceil_div_i64(most + 1, 256), (unsigned)p.n), 256, 0, (cudaStream_t)stream>>>(p);
+        rc = check_cuda(cudaGetLastError(), "mark_repack_kernel launch");
+        if (rc) return rc;
+        rc = launch_beside(repack_kernel, (unsigned)end, true, (cudaStream_t)stream, p);
         if (rc) return rc;
     }
     return ATLAS_OK;
