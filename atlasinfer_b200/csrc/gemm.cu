@@ -9,12 +9,14 @@
 // tile by tile in tensor memory and consumed at once by the 5th-generation
 // tensor cores, so it never exists in global memory.
 //
-// One CTA computes a 128 (output features) x BN (tokens) tile.  The rebuilt fp16 weights never touch
+// One CTA computes a 128 (output features) x BN (tokens) tile; beyond 256 tokens (the most an MMA takes) it has two
+// accumulators and uses every rebuilt weight tile twice.  The rebuilt fp16 weights never touch
 // shared memory: the dequantizer warps write them straight into tensor memory and the MMA takes its A
 // operand from there, so shared memory only carries what comes from global memory (the kernel is bound
 // by the shared-memory data pipe, not by the tensor pipe).  A pipeline stage is two k-tiles (128 columns
 // of K).  Rings: codes (4 stages of 2 x (8 KB + 256 B of scales)), activations (2 stages of 2 x BN x 64
-// fp16, L2-resident), rebuilt weights (4 stages of 64 TMEM columns beside the accumulator; 2 for BN < 256).
+// fp16, L2-resident), rebuilt weights (4 stages of 64 TMEM columns beside the accumulator; 2 for up to 128 and more than
+// 256 tokens).
 //   warp 0      activation producer: per 64-wide K step a 2-D TMA load of the BN x 64 fp16
 //               activation tile (128-byte swizzle) completing on the step's `ready` barrier
 //   warp 2      code producer: a 1-D bulk copy of the step's 8 KB code tile (contiguous in the
@@ -70,24 +72,27 @@ constexpr int GM_PH = 4;    // K-stage phases of the dequantizers = `ready` / `m
 constexpr int GM_A_COLS = GM_SK * GM_BK / 2;     // TMEM columns of one A stage: two fp16 per 32-bit cell
 constexpr uint32_t C_BYTES = GM_BM * GM_BK;      // 8 KB code tile
 constexpr uint32_t S_BYTES = 256;                // one scale block: 128 rows x fp16
-// shared-memory map for a tile of BN tokens (BN = 32, 64, 128 or 256 = UMMA N)
+// shared-memory map for a tile of BN tokens (UMMA N up to 256; beyond, two accumulators of BN / 2 tokens)
 template <int BN>
 struct Smem {
+    static constexpr int SUBS = BN > 256 ? 2 : 1;         // MMAs that use a rebuilt weight tile
+    static constexpr int SUB_N = BN / SUBS;               // their N
+    static_assert(SUB_N % 16 == 0 && BN % 32 == 0, "UMMA N; epilogue chunks");
     static constexpr uint32_t B_BYTES = BN * GM_BK * 2;   // fp16 activation tile of one k-tile
     // Code ring depth, in stages of GM_SK k-tiles (16 KB): the bytes an SM keeps in flight.  Decode-sized token
     // tiles are HBM-bound and leave the room for a deep ring (160 KB in flight covers ~3 us of loaded DRAM latency
     // at an SM's share of the bandwidth); the 256-token tile is compute-bound and needs the room for activations.
-    static constexpr int CS = BN <= 32 ? 10 : (BN == 64 ? 8 : (BN == 128 ? 6 : 4));
+    static constexpr int CS = BN <= 32 ? 10 : (BN == 64 ? 8 : (BN == 128 ? 6 : (BN <= 256 ? 4 : (BN <= 320 ? 3 : 2))));
     // Activation ring depth, in stages.  Decode-sized token tiles are filled by a warp (loads, conversion, stores:
     // a microsecond of latency per stage), which a deeper ring hides; the wide tiles come in by TMA.
-    static constexpr int XS = BN <= 64 ? 4 : 2;
+    static constexpr int XS = BN <= 64 ? 4 : (BN == 160 || BN == 192 ? 3 : 2);
     static constexpr uint32_t OFF_B = 0;
     static constexpr uint32_t OFF_C = OFF_B + XS * GM_SK * B_BYTES;
     static constexpr uint32_t OFF_BAR = OFF_C + CS * GM_SK * C_BYTES;
     static constexpr uint32_t OFF_S = OFF_BAR + 512;
     static constexpr uint32_t TOTAL = OFF_S + CS * GM_SK * S_BYTES + 1024 /*alignment slack*/;
     // A stages in tensor memory (64 columns each) beside the accumulator columns [0, BN); allocations are powers of two
-    static constexpr int A_STAGES = BN == 256 ? 4 : 2;
+    static constexpr int A_STAGES = BN > 128 && BN <= 256 ? 4 : 2;
     static constexpr uint32_t TMEM_COLS = BN + A_STAGES * GM_A_COLS <= 256 ? 256 : 512;
     static_assert(BN + A_STAGES * GM_A_COLS <= 512, "tensor memory");
     // the epilogue stages the output tile over the (then idle) activation and code rings
@@ -97,7 +102,7 @@ struct Smem {
 // Instruction descriptor, kind::f16: D fp32 (1 at bit 4), A and B fp16 (0 at bits 7 and 10),
 // both K-major (0 at bits 15, 16), N >> 3 at bit 17, M >> 4 at bit 24.
 template <int BN>
-constexpr uint32_t gm_idesc() { return (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(GM_BM >> 4) << 24); }
+constexpr uint32_t gm_idesc() { return (1u << 4) | ((uint32_t)(Smem<BN>::SUB_N >> 3) << 17) | ((uint32_t)(GM_BM >> 4) << 24); }
 
 struct GemmParams {
     const uint8_t *tiles;
@@ -146,9 +151,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
     auto mma_done = [&](int s) { return bars + 8u * (GM_PH + s); };
     auto full_c = [&](int s) { return bars + 8u * (2 * GM_PH + s); };
     constexpr int CS = SM::CS, XS = SM::XS;
-    auto empty_c = [&](int s) { return bars + 8u * (2 * GM_PH + CS + s); };
-    auto x_landed = [&](int s) { return bars + 8u * (2 * GM_PH + 2 * CS + s); };   // bf16 tile in its slot, to be converted
-    constexpr int N_BARS = 2 * GM_PH + 2 * CS + XS + 1;
+    // A dequantizer comes back to a code slot rounds later.  With a short ring two landings of a slot alternate between two
+    // barriers, so that a parity tells its landings apart: at stage st the warp knows that the codes of stage st - 4 (its own
+    // last) have landed, and, as it then waited for that A stage, those of st - 4 - AS too.
+    constexpr int FB = CS < GM_PH ? 2 * CS : CS;
+    static_assert(FB == GM_PH || FB == GM_PH + SM::A_STAGES || FB > GM_PH + SM::A_STAGES, "code ring parity");
+    auto empty_c = [&](int s) { return bars + 8u * (2 * GM_PH + FB + s); };
+    auto x_landed = [&](int s) { return bars + 8u * (2 * GM_PH + FB + CS + s); };   // bf16 tile in its slot, to be converted
+    constexpr int N_BARS = 2 * GM_PH + FB + CS + XS + 1;
     static_assert(N_BARS * 8 + 16 <= 512, "barrier area");
     const uint32_t accfull_bar = bars + 8u * (N_BARS - 1);
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(base_ptr + OFF_BAR + 8 * N_BARS);
@@ -176,10 +186,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
             mbar_init(mma_done(s), 1);
         }
         for (int s = 0; s < XS; ++s) mbar_init(x_landed(s), 1);
-        for (int s = 0; s < CS; ++s) {
-            mbar_init(full_c(s), 1);
-            mbar_init(empty_c(s), 4);
-        }
+        for (int s = 0; s < FB; ++s) mbar_init(full_c(s), 1);
+        for (int s = 0; s < CS; ++s) mbar_init(empty_c(s), 4);
         mbar_init(accfull_bar, 1);
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -224,7 +232,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
             const uint32_t rb = p.x_bf16 ? x_landed(slot) : ready_bar(st % GM_PH);
             mbar_arrive_expect_tx(rb, (uint32_t)nk * B_BYTES);
             for (int j = 0; j < nk; ++j)
-                tma_load_2d(base + OFF_B + (slot * GM_SK + j) * B_BYTES, &x_map, (kt_begin + st * GM_SK + j) * GM_BK, m0, rb);
+#pragma unroll
+                for (int u = 0; u < SM::SUBS; ++u)
+                    tma_load_2d(base + OFF_B + (slot * GM_SK + j) * B_BYTES + u * (B_BYTES / SM::SUBS), &x_map,
+                                (kt_begin + st * GM_SK + j) * GM_BK, m0 + u * SM::SUB_N, rb);
             return true;
         };
         if (BN <= 64 && p.x_bf16) {
@@ -283,15 +294,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
                 if (round > 0 && !mbar_wait<200>(empty_c(slot), (round - 1) & 1)) { *s_abort = 1; break; }
                 if (*s_abort) break;
                 const int nk = min(GM_SK, KT - st * GM_SK);
-                mbar_arrive_expect_tx(full_c(slot), (uint32_t)nk * (C_BYTES + (p.bs_tiles ? S_BYTES : 0)));
+                mbar_arrive_expect_tx(full_c(st % FB), (uint32_t)nk * (C_BYTES + (p.bs_tiles ? S_BYTES : 0)));
                 for (int j = 0; j < nk; ++j) {
                     const int kt = st * GM_SK + j;
                     // an 8 KB code tile is a 128-row x 64-byte matrix; the 64-byte swizzle spreads a column of 16-byte
                     // chunks over all banks for the dequantizers (thread = row)
-                    tma_load_2d(base + OFF_C + (slot * GM_SK + j) * C_BYTES, &c_map, 0, (int)((crow0 + kt) * GM_BM), full_c(slot));
+                    tma_load_2d(base + OFF_C + (slot * GM_SK + j) * C_BYTES, &c_map, 0, (int)((crow0 + kt) * GM_BM), full_c(st % FB));
                     if (p.bs_tiles)
                         bulk_load_1d(base + OFF_S + (slot * GM_SK + j) * S_BYTES,
-                                     p.scales_t + ((size_t)blockIdx.x * bpr + (kt_begin + kt) / p.bs_tiles) * 128, S_BYTES, full_c(slot));
+                                     p.scales_t + ((size_t)blockIdx.x * bpr + (kt_begin + kt) / p.bs_tiles) * 128, S_BYTES, full_c(st % FB));
                 }
             }
         }
@@ -310,18 +321,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
                 const uint64_t dbs = db0 + (uint64_t)(((st % XS) * GM_SK * B_BYTES) >> 4);   // the address field counts 16-byte units
                 const uint32_t ta = ta0 + (uint32_t)((st % AS) * GM_A_COLS);
                 const bool two = KT - st * GM_SK >= 2;
-                umma_f16_ts(tmem_base, ta, dbs, gm_idesc<BN>(), st != 0);
-                umma_f16_ts(tmem_base, ta + 8u, dbs + 2u, gm_idesc<BN>(), 1u);
+                // (a rebuilt tile is used for all accumulators before the next one)
+                auto mma = [&](int k, uint64_t db, uint32_t accumulate) {
+#pragma unroll
+                    for (int u = 0; u < SM::SUBS; ++u)
+                        umma_f16_ts(tmem_base + (uint32_t)(u * SM::SUB_N), ta + (uint32_t)(k * 8),
+                                    db + (uint64_t)((k & 3) * 2) + (uint64_t)((u * (B_BYTES / SM::SUBS)) >> 4), gm_idesc<BN>(), accumulate);
+                };
+                mma(0, dbs, st != 0);
+                mma(1, dbs, 1u);
                 // the next stage's barrier: one poll now, looked at after the commit
                 const uint32_t rbn = ready_bar((st + 1) % GM_PH);
                 const uint32_t pn = (uint32_t)(((st + 1) / GM_PH) & 1);
                 const bool next_ready = st + 1 < NST ? mbar_try_wait(rbn, pn) : true;
-                umma_f16_ts(tmem_base, ta + 16u, dbs + 4u, gm_idesc<BN>(), 1u);
-                umma_f16_ts(tmem_base, ta + 24u, dbs + 6u, gm_idesc<BN>(), 1u);
+                mma(2, dbs, 1u);
+                mma(3, dbs, 1u);
                 if (two) {
-                    const uint64_t db1 = dbs + (uint64_t)(B_BYTES >> 4);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) umma_f16_ts(tmem_base, ta + 32u + (uint32_t)(k * 8), db1 + (uint64_t)(k * 2), gm_idesc<BN>(), 1u);
+                    for (int k = 4; k < 8; ++k) mma(k, dbs + (uint64_t)(B_BYTES >> 4), 1u);
                 }
                 umma_commit(done_bar_of(st));  // arrives when these MMAs have finished reading the slot and the A stage
                 if (!next_ready) ok = mbar_wait(rbn, pn);
@@ -410,8 +427,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ C
             }
             const uint32_t second = __ballot_sync(0xffffffffu, (pk0 >> 22) & 1u);   // entries of the stage's second k-tile
 
-            const int sc_ = st % CS, cround = st / CS;   // code slot
-            if (!mbar_wait_warp<40>(full_c(sc_), cround & 1, s_abort)) { ok = false; break; }
+            const int sc_ = st % CS;   // code slot
+            if (!mbar_wait_warp<40>(full_c(st % FB), (st / FB) & 1, s_abort)) { ok = false; break; }
 #pragma unroll
             for (int j = 0; j < GM_SK; ++j) {
                 if (j < nk) {
@@ -758,31 +775,67 @@ cudaLaunchConfig_t pdl_config(dim3 grid, dim3 block, size_t smem, cudaStream_t s
     return cfg;
 }
 
-// tokens per tile for a batch of m rows
-int gemm_bn_for(int64_t m) { return m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256)); }
-
-// K slices (one CTA per SM, `tiles` output tiles).
-// Decode-sized tiles: the count that minimises waves x (k-tiles per CTA + the fixed cost of a CTA, about 12 k-tiles'
-// worth of streaming), so that neither a nearly empty last wave nor many short CTAs dominate.
-// Prompts: a CTA takes 0.4 us per k-tile and 7 us besides; slicing adds a second kernel (2.5 us) and the fp32 partial
-// sums' way through L2 and back (about 4 TB/s).  Few row tiles and one or two token tiles leave most of the chip idle
-// otherwise: 4096 x 11008 at 301 tokens is 64 tiles.
-int gemm_splits_for(int64_t m, int64_t n_rows, int64_t n_cols, int sms) {
-    const int bn = gemm_bn_for(m);
-    if (bn == 128) return 1;   // (few row tiles at 65 to 128 rows: the kernel in gemm_tile.cu slices K)
-    const int64_t tiles = ceil_div_i64(n_rows, GM_BM) * ceil_div_i64(m, bn);
-    const int k_tiles = (int)(n_cols / 64);
-    int best = 1;
-    double best_cost = 0;
-    for (int s = 1; s <= 16; s = bn > 64 ? s + 1 : s * 2) {
-        if (s > 1 && k_tiles / s < 8) break;
-        const double waves = (double)ceil_div_i64(tiles * s, sms);
-        double cost = waves * (double)(ceil_div_i64(k_tiles, s) + 12);
-        if (bn > 64) cost = waves * (0.4 * (double)ceil_div_i64(k_tiles, s) + 7.0) + (s > 1 ? 2.5 + 2e-6 * s * (double)m * (double)n_rows : 0.0);
-        if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
-    }
-    return best;
+// Tokens per tile and K slices for a batch of m rows (one CTA per SM).
+// Decode-sized tiles: the slices that minimise waves x (k-tiles per CTA + the fixed cost of a CTA, about 12 k-tiles' worth
+// of streaming), so that neither a nearly empty last wave nor many short CTAs dominate.
+// Prompts.  Rebuilding a k-tile of weights takes 0.35 us however many tokens use it, so the best tile is the one that holds
+// all tokens, or an even share of them: 300 tokens in one tile of 320 instead of two of 256 take 37 us instead of 58 at
+// 11008 x 4096, 36 instead of 48 at 4096 x 11008; 2048 tokens in six tiles of 384 instead of eight 193 instead of 228 at
+// 12288 x 4096, 359 instead of 415 at 22016 x 4096.  How that works out in waves of one CTA per SM is what PROMPT_TILES
+// models: fitted to 5751 runs (16 shapes of 1024 x 1024 to 22016 x 4096, 129 to 2048 tokens, every tile and up to 8 slices),
+// 6.5 % off (rms).  A CTA takes `kt` per k-tile, more when all SMs work, and `fixed` besides; slicing adds a second kernel
+// and the fp32 partial sums' way through L2 and back.  A tile of 256 tokens sliced by its own, older rule is kept unless the
+// model sees a gain of 8 %, more than its error: of 239 shapes 4 are then slower than with that rule (by up to 15 %), and the
+// mean time is 0.92 of it (0.91 without the margin, with 13 slower; the best choices 0.89).
+struct GemmPlan {
+    int bn, splits;
+};
+struct PromptTile {
+    int bn;
+    double kt, fixed;   // us
+};
+constexpr PromptTile PROMPT_TILES[] = {{160, .356, 2.55}, {192, .358, 2.9}, {224, .383, 2.75}, {256, .402, 3.25}, {320, .480, 3.4}, {384, .540, 3.5}};
+double prompt_us(const PromptTile &c, int64_t m, int64_t n_rows, int64_t row_tiles, int k_tiles, int s, int sms) {
+    const int64_t ctas = row_tiles * ceil_div_i64(m, c.bn) * s;
+    const double busy = ctas < sms ? (double)ctas / sms : 1.;
+    return 1.95 + (double)ceil_div_i64(ctas, sms) * (c.kt * (.88 + .24 * busy) * (double)ceil_div_i64(k_tiles, s) + c.fixed) +
+           (s > 1 ? 2.1 + 1.4e-6 * s * (double)m * (double)n_rows : 0.);
 }
+GemmPlan make_plan(int64_t m, int64_t n_rows, int64_t n_cols, int sms) {
+    GemmPlan plan = {m <= 32 ? 32 : (m <= 64 ? 64 : (m <= 128 ? 128 : 256)), 1};
+    if (plan.bn == 128) return plan;   // (few row tiles at 65 to 128 rows: the kernel in gemm_tile.cu slices K)
+    const int64_t row_tiles = ceil_div_i64(n_rows, GM_BM), tiles = row_tiles * ceil_div_i64(m, plan.bn);
+    const int k_tiles = (int)(n_cols / 64);
+    double best = 0;
+    for (int s = 1; s <= 16; s = plan.bn > 64 ? s + 1 : s * 2) {
+        if (s > 1 && k_tiles / s < 8) break;
+        const double waves = (double)ceil_div_i64(tiles * s, sms), kt = (double)ceil_div_i64(k_tiles, s);
+        const double cost = plan.bn <= 64 ? waves * (kt + 12) : waves * (0.4 * kt + 7.0) + (s > 1 ? 2.5 + 2e-6 * s * (double)m * (double)n_rows : 0.0);
+        if (s == 1 || cost < best) { plan.splits = s; best = cost; }
+    }
+    if (plan.bn <= 64) return plan;
+    best = .92 * prompt_us(PROMPT_TILES[3], m, n_rows, row_tiles, k_tiles, plan.splits, sms);
+    for (const PromptTile &c : PROMPT_TILES)
+        for (int s = 1; s <= 8 && (s == 1 || k_tiles / s >= 8); ++s) {
+            const double us = prompt_us(c, m, n_rows, row_tiles, k_tiles, s, sms);
+            if (us < best) {
+                plan = {c.bn, s};
+                best = us;
+            }
+        }
+    return plan;
+}
+// (The sizes decide everything, and a call asks three times: the answers for the last sizes a thread has asked about are kept.)
+GemmPlan gemm_plan(int64_t m, int64_t n_rows, int64_t n_cols, int sms) {
+    struct Entry { int64_t m, n_rows, n_cols; int sms; GemmPlan plan; };
+    constexpr int KEPT = 64;
+    static thread_local Entry kept[KEPT] = {};
+    const uint64_t h = ((uint64_t)m * 0x9e3779b97f4a7c15ull) ^ ((uint64_t)n_rows * 0xc2b2ae3d27d4eb4full) ^ ((uint64_t)n_cols * 0x165667b19e3779f9ull);
+    Entry &e = kept[(h >> 58) % KEPT];
+    if (e.m != m || e.n_rows != n_rows || e.n_cols != n_cols || e.sms != sms) e = {m, n_rows, n_cols, sms, make_plan(m, n_rows, n_cols, sms)};
+    return e.plan;
+}
+int gemm_splits_for(int64_t m, int64_t n_rows, int64_t n_cols, int sms) { return gemm_plan(m, n_rows, n_cols, sms).splits; }
 
 // bf16 rows of decode-sized token tiles are converted in the kernel when the weight is small: one more kernel in the chain
 // then costs more than the conversion's share of the producer warp over the few stages of a CTA
@@ -943,7 +996,8 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
         route = route_for(Shape{m, n_rows, n_cols, gemm_sm_count(), (bf16 ? 1 : 0) | (tma_ok ? 2 : 0) | (aligned ? 4 : 0)});
     }
     const bool tile = route.tile;
-    const int bn = tile ? tile_tokens_for(m) : gemm_bn_for(m);
+    const GemmPlan plan = tile ? GemmPlan{tile_tokens_for(m), route.plan.splits} : gemm_plan(m, n_rows, n_cols, gemm_sm_count());
+    const int bn = plan.bn;
 
     // operand B must be fp16 with rows on 16-byte boundaries for the tensor map
     const void *xb = x;
@@ -974,7 +1028,7 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
     CUtensorMap x_map;
     const cuuint64_t gdim[2] = {(cuuint64_t)n_cols, (cuuint64_t)m};
     const cuuint64_t gstride[1] = {(cuuint64_t)ldb * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)GM_BK, (cuuint32_t)bn};
+    const cuuint32_t box[2] = {(cuuint32_t)GM_BK, (cuuint32_t)(bn > 256 ? bn / 2 : bn)};
     const cuuint32_t estride[2] = {1, 1};
     CUresult cr = encode(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(xb), gdim, gstride, box,
                          estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1030,7 +1084,7 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
     p.n_chunks = (int)(n_cols / 64);
     p.bs_tiles = block_size % 64 == 0 ? block_size / 64 : 0;
     p.out_bf16 = dtype == ATLAS_DTYPE_BF16;
-    p.splits = gemm_splits_for(m, n_rows, n_cols, gemm_sm_count());
+    p.splits = plan.splits;
     p.partials = (float *)((char *)workspace + GM_WS_HEADER + xcopy);
     p.to_partials = gather != nullptr;   // the gather is the second kernel's job
     p.x_bf16 = in_kernel_bf16;
@@ -1043,7 +1097,12 @@ int gemm_entry(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *
         case 32: rc = launch_gemm<32>(x_map, c_map, p, st); break;
         case 64: rc = launch_gemm<64>(x_map, c_map, p, st); break;
         case 128: rc = launch_gemm<128>(x_map, c_map, p, st); break;
-        default: rc = launch_gemm<256>(x_map, c_map, p, st); break;
+        case 160: rc = launch_gemm<160>(x_map, c_map, p, st); break;
+        case 192: rc = launch_gemm<192>(x_map, c_map, p, st); break;
+        case 224: rc = launch_gemm<224>(x_map, c_map, p, st); break;
+        case 256: rc = launch_gemm<256>(x_map, c_map, p, st); break;
+        case 320: rc = launch_gemm<320>(x_map, c_map, p, st); break;
+        default: rc = launch_gemm<384>(x_map, c_map, p, st); break;
     }
     if (rc) return rc;
     if (p.splits > 1 || p.to_partials) {
