@@ -181,7 +181,7 @@ ATLAS_API int atlas_repack(const int8_t *codes, int64_t n_codes, const void *out
                            void *scales_tiled, int32_t *outlier_row_ptr, int32_t *outlier_chunk_ptr,
                            uint32_t *outlier_entries, void *outlier_vals_sorted, void *stream);
 
-/* Several tensors in one launch (8 at a time).  The arguments of one tensor are those of atlas_repack, except that
+/* Several tensors in one pair of launches (8 at a time).  The arguments of one tensor are those of atlas_repack, except that
  * outlier_row_ptr may be NULL (not wanted) and that entry_base is added to what outlier_chunk_ptr holds: a tensor
  * whose tiles, scales, chunk pointers and entries are written behind one another's into common buffers (rows padded
  * to 128, entry_base = entries of the tensors before it) becomes a run of rows of one joined weight. */
