@@ -149,25 +149,26 @@ std::vector<std::array<at::Tensor, 4>> quantize_many(const std::vector<at::Tenso
     const auto bytes_opt = flats[0].options().dtype(at::kByte);
     const size_t n = flats.size();
     std::vector<int64_t> capacity(n);
-    int64_t workspace_bytes = 0, outlier_bytes = 0;
+    int64_t workspace_bytes = 0;
     for (size_t i = 0; i < n; ++i) {
         // |z| > t bounds the outliers of a block by (block_size - 1) / t^2, but weight-like data has well under
         // 1 %: start with 1/32 of the tensor and retry with full capacity in the rare case that is short
         const int64_t padded = (flats[i].numel() + bs - 1) / bs * bs;
         capacity[i] = std::min(padded, padded / 32 + 1024);
         workspace_bytes += atlas_quantize_workspace_bytes(flats[i].numel(), (int)bs);
-        outlier_bytes += up16(capacity[i] * 8) + up16(capacity[i] * 2);
     }
     // counts, and behind them the workspace: cleared together
     at::Tensor scratch = at::empty({(int64_t)n * 32 + workspace_bytes}, bytes_opt);
-    at::Tensor outliers = at::empty({outlier_bytes}, bytes_opt);
     int64_t *counts = (int64_t *)scratch.data_ptr();
     std::vector<Job> jobs;
     std::vector<AtlasQuantizeItem> items;
-    char *at_byte = (char *)outliers.data_ptr();
+    // (a buffer per tensor: one for all of them is the largest block of the call, which the caching allocator then cuts up
+    // for the next caller's tensors)
+    std::vector<at::Tensor> held;   // until the copies are enqueued
     for (size_t i = 0; i < n; ++i) {
+        held.push_back(at::empty({up16(capacity[i] * 8) + up16(capacity[i] * 2)}, bytes_opt));
+        char *at_byte = (char *)held[i].data_ptr();
         jobs.push_back(make_job(flats[i], bs, capacity[i], at_byte + up16(capacity[i] * 8), at_byte, counts + 4 * i));
-        at_byte += up16(capacity[i] * 8) + up16(capacity[i] * 2);
         items.push_back(jobs[i].item);
     }
     check(atlas_quantize_many((int)n, items.data(), (int)bs, z, counts + 4 * n, (size_t)workspace_bytes, stream), "atlas_quantize");
@@ -175,7 +176,6 @@ std::vector<std::array<at::Tensor, 4>> quantize_many(const std::vector<at::Tenso
     const int64_t *c = (const int64_t *)host.data_ptr();
     std::vector<std::array<at::Tensor, 4>> out;
     std::vector<AtlasCopyItem> copies;
-    std::vector<at::Tensor> held;   // buffers of a second attempt, until the copies are enqueued
     for (size_t i = 0; i < n; ++i) {
         int64_t n_codes = c[4 * i], n_out = c[4 * i + 1], timed_out = c[4 * i + 2];
         Job &j = jobs[i];
