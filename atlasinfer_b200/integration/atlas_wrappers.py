@@ -238,6 +238,11 @@ def slice_layout(fused: KernelLayout, row_offset: int, n_rows: int, source, entr
                         fused.entries, fused.vals_sorted, n_rows, k, bs, fused.ready)
 
 
+def _final(layout: KernelLayout) -> KernelLayout:
+    """``layout`` with nothing left to wait for (as ``_replace(ready=None)``, in a third of its 1.5 us)."""
+    return KernelLayout(*layout[:-1], None)
+
+
 class FusedLinearGroup:
     """Several ``QuantizedLinear`` layers that read the same activations, computed by one launch.
 
@@ -304,7 +309,7 @@ class FusedLinearGroup:
         if self.layout is None or self.layout.tiles.device != x.device:
             self.build(x.device)
         elif self.layout.ready is not None and self.layout.ready.wait():
-            self.layout = self.layout._replace(ready=None)
+            self.layout = _final(self.layout)
         c = self._cache
         if c is None or c[0] is not x or c[1] != x._version or index in c[3]:
             y_all = quantized_linear_forward(x, self.layout, self.bias)
@@ -397,7 +402,7 @@ class QuantizedLinear(nn.Module):
         if lay is not None and lay.source is q_tensor and x.is_cuda and lay.tiles.device == x.device and (
                 bias is None or bias.device == x.device):
             if lay.ready is not None and lay.ready.wait():
-                self._kernel_layout = lay = lay._replace(ready=None)
+                self.__dict__["_kernel_layout"] = lay = _final(lay)   # (past Module.__setattr__: 2 us)
             return quantized_linear_forward(x, lay, self._bias_for(bias))
         # the kernels need a GPU; CPU activations are staged through it and the result returned
         compute_device = x.device if x.device.type == "cuda" else _capi.require_cuda()
