@@ -22,6 +22,10 @@ int check_cuda(cudaError_t e, const char *what) {
     return ATLAS_ERR_LAUNCH;
 }
 
+static thread_local bool g_plain_launch = false;
+
+bool early_start() { return !g_plain_launch; }
+
 int check_device() {
     int dev = -1;
     cudaError_t e = cudaGetDevice(&dev);
@@ -54,6 +58,12 @@ int check_device() {
 extern "C" {
 
 int atlas_version(void) { return 100; /* 0.1.0 */ }
+
+int atlas_qlinear_plain_launch(int on) {
+    const bool was = atlas::g_plain_launch;
+    atlas::g_plain_launch = on != 0;
+    return was;
+}
 
 const char *atlas_last_error(void) { return atlas::g_err; }
 

@@ -17,6 +17,11 @@ void clear_error();
 // Returns ATLAS_OK, or records `what` + the CUDA error text and returns ATLAS_ERR_LAUNCH.
 int check_cuda(cudaError_t e, const char *what);
 
+// Whether the calling thread's linears may start while the kernel in front of them still runs (atlas_qlinear_plain_launch).
+// They read weights, scales, outlier lists and the bias at once, before griddepcontrol.wait, and only that instruction or an
+// ordinary launch makes the stores of the kernel in front visible.
+bool early_start();
+
 // ATLAS_OK if the current device is compute capability 10.x, else ATLAS_ERR_NO_DEVICE.
 int check_device();
 

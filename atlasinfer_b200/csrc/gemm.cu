@@ -760,7 +760,7 @@ constexpr size_t GM_WS_HEADER = 256;  // reserved; the fp16 copy of x follows
 namespace atlas {
 namespace {
 
-// launch configuration with programmatic dependent launch allowed
+// launch configuration with programmatic dependent launch, where the caller allows it
 cudaLaunchConfig_t pdl_config(dim3 grid, dim3 block, size_t smem, cudaStream_t st) {
     static thread_local cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -771,7 +771,7 @@ cudaLaunchConfig_t pdl_config(dim3 grid, dim3 block, size_t smem, cudaStream_t s
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early_start() ? 1 : 0;
     return cfg;
 }
 

@@ -389,8 +389,9 @@ int launch_tile_bn(const CUtensorMap &x_map, const CUtensorMap &c_map, const Til
     cfg.blockDim = dim3(TL_THREADS);
     cfg.dynamicSmemBytes = TileSmem<BN>::TOTAL;
     cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = p.splits > 1 ? 2 : 1;
+    const bool early = early_start();
+    cfg.attrs = attr + (early ? 0 : 1);
+    cfg.numAttrs = (early ? 1 : 0) + (p.splits > 1 ? 1 : 0);
     return check_cuda(cudaLaunchKernelEx(&cfg, tile_kernel<BN>, x_map, c_map, p), "tile_kernel launch");
 }
 

@@ -401,7 +401,7 @@ int launch_gemv_strip(const GemvParams &p, bool vec, cudaStream_t st) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early_start() ? 1 : 0;
     if (stage) {
         auto kern = two ? gemv_strip_kernel<true, true, 1, true, true, 2>
                         : (fast ? gemv_strip_kernel<true, true, 1, true, true> : gemv_strip_kernel<true, true, 1, true, false>);

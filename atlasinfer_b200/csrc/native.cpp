@@ -28,9 +28,10 @@ void check(int status, const char *what) {
 const void *ptr_or_null(const at::Tensor &t) { return t.numel() ? t.data_ptr() : nullptr; }
 
 // Stands for a layout that may still be written by the stream it was enqueued on.  The linear kernels read weights before
-// the stream's earlier work has completed (programmatic dependent launch), but no kernel of that stream starts before the
-// one that writes the layout has ended, since that one does not let others start early.  So only a use on another stream, or
-// in a capture, whose kernels run who knows where, has to wait; it waits on the host, once.
+// the stream's earlier work has completed (programmatic dependent launch): a dependent starts once the kernel in front has
+// ended, but sees its stores for certain only behind griddepcontrol.wait.  Until the layout is known to be final, a linear
+// on that stream is therefore launched plainly; a use on another stream, or in a capture, whose kernels run who knows where,
+// waits on the host, once.
 class LayoutReady {
    public:
     LayoutReady() {
@@ -41,7 +42,7 @@ class LayoutReady {
     }
     ~LayoutReady() { cudaEventDestroy(event_); }
     LayoutReady(const LayoutReady &) = delete;
-    // True once the layout is final.  False: not yet, but work enqueued on the current stream comes after it.
+    // True once the layout is final.  False: not yet, but what is launched plainly on the current stream comes after it.
     bool wait() {
         if (done_.load(std::memory_order_acquire)) return true;
         const cudaStream_t on = at::cuda::getCurrentCUDAStream(device_).stream();
@@ -82,10 +83,23 @@ class LayoutReady {
     std::atomic<bool> done_{false};
 };
 
-// x @ W^T + bias for a kernel layout; `gemv` chooses the per-strip kernel, else the tcgen05 kernels.
+// The linears of this scope are launched plainly (`on`), or as the thread has it.
+class PlainLaunch {
+   public:
+    explicit PlainLaunch(bool on) : on_(on) { if (on_) was_ = atlas_qlinear_plain_launch(1); }
+    ~PlainLaunch() { if (on_) atlas_qlinear_plain_launch(was_); }
+    PlainLaunch(const PlainLaunch &) = delete;
+
+   private:
+    bool on_;
+    int was_ = 0;
+};
+
+// x @ W^T + bias for a kernel layout; `gemv` chooses the per-strip kernel, else the tcgen05 kernels.  `pending`: the stream's
+// earlier work may still write the layout.
 at::Tensor linear(const at::Tensor &x, const at::Tensor &tiles, const at::Tensor &scales, const at::Tensor &chunk_ptr,
                   const at::Tensor &entries, const at::Tensor &vals, int64_t n, int64_t k, int64_t bs,
-                  const std::optional<at::Tensor> &bias, const at::Tensor &status, int64_t gemv_max_rows) {
+                  const std::optional<at::Tensor> &bias, const at::Tensor &status, int64_t gemv_max_rows, bool pending) {
     const int dtype = x.scalar_type() == at::kHalf ? ATLAS_DTYPE_F16 : ATLAS_DTYPE_BF16;   // (the caller has looked)
     if (x.dim() < 1 || x.size(-1) != k)
         throw std::runtime_error("QuantizedLinear: input has " + std::to_string(x.dim() ? x.size(-1) : 0) + " features, weight expects " + std::to_string(k));
@@ -104,6 +118,8 @@ at::Tensor linear(const at::Tensor &x, const at::Tensor &tiles, const at::Tensor
     if (m == 0) return y;
     at::Tensor b;
     if (bias.has_value()) b = bias->to(at::kHalf).contiguous();
+    // (a bias converted just now is written by the kernel in front)
+    const PlainLaunch plain(pending || (b.defined() && !b.is_same(*bias)));
     void *stream = at::cuda::getCurrentCUDAStream(x.get_device()).stream();
     const void *bp = b.defined() ? ptr_or_null(b) : nullptr;
     if (m <= gemv_max_rows) {

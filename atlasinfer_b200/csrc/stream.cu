@@ -780,7 +780,7 @@ int launch_stream(const StreamParams &p, int grid, size_t smem, cudaStream_t st)
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early_start() ? 1 : 0;
     return check_cuda(cudaLaunchKernelEx(&cfg, kern, p), "qlinear_stream_kernel launch");
 }
 

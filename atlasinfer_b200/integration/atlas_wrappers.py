@@ -119,7 +119,8 @@ def build_joined_layout(qs, wait: bool = True):
     pointers of the canonical streams are only written for a single tensor.
 
     With ``wait`` the buffers are final on return.  Without, ``layout.ready`` stands for the work under way:
-    ``quantized_linear_forward`` may be called at once, any other use outside the current stream waits for it."""
+    ``quantized_linear_forward`` may be called at once (it launches plainly until the work is done), any other use
+    outside the current stream waits for it."""
     for q in qs:
         reason = kernel_layout_supported(q.original_shape, int(q.block_size))
         if reason is not None:
@@ -164,10 +165,9 @@ def quantized_linear_forward(x: torch.Tensor, layout: KernelLayout, bias: Option
         gemv_rows = _ANY_ROWS if force == "gemv" else 0
     else:
         raise ValueError(f"force={force!r}")
-    if layout.ready is not None:
-        layout.ready.wait()
+    pending = layout.ready is not None and not layout.ready.wait()
     return _capi.native().linear(x, layout.tiles, layout.scales_tiled, layout.chunk_ptr, layout.entries, layout.vals_sorted,
-                                 layout.n_rows, layout.n_cols, layout.block_size, bias, status_word(x.device), gemv_rows)
+                                 layout.n_rows, layout.n_cols, layout.block_size, bias, status_word(x.device), gemv_rows, pending)
 
 
 def _stream_forward(x: torch.Tensor, layout: KernelLayout, bias: Optional[torch.Tensor]) -> torch.Tensor:
@@ -177,8 +177,7 @@ def _stream_forward(x: torch.Tensor, layout: KernelLayout, bias: Optional[torch.
     n, k = layout.n_rows, layout.n_cols
     if x.shape[-1] != k:
         raise RuntimeError(f"QuantizedLinear: input has {x.shape[-1]} features, weight expects {k}")
-    if layout.ready is not None:
-        layout.ready.wait()
+    pending = layout.ready is not None and not layout.ready.wait()
     x2 = x.reshape(-1, k)
     if x2.stride(-1) != 1 or (x2.shape[0] > 1 and x2.stride(0) < k):
         x2 = x2.contiguous()
@@ -188,12 +187,18 @@ def _stream_forward(x: torch.Tensor, layout: KernelLayout, bias: Optional[torch.
     if m:
         b = None if bias is None else bias.to(torch.float16).contiguous()
         ws = stream_workspace(dev)
-        with torch.cuda.device(dev):
-            status = L.atlas_qlinear_stream(
-                x2.data_ptr(), _capi.DTYPE_F16 if x.dtype == torch.float16 else _capi.DTYPE_BF16, m, ldx,
-                layout.tiles.data_ptr(), layout.scales_tiled.data_ptr(), layout.chunk_ptr.data_ptr(),
-                _capi.ptr(layout.entries), _capi.ptr(layout.vals_sorted), n, k, layout.block_size, _capi.ptr(b),
-                y.data_ptr(), n, ws.data_ptr(), ws.numel(), status_word(dev).data_ptr(), _capi.stream_ptr(dev))
+        # (a bias converted just now, like a layout still under way, is written by the kernels in front)
+        was = L.atlas_qlinear_plain_launch(1) if pending or b is not bias else None
+        try:
+            with torch.cuda.device(dev):
+                status = L.atlas_qlinear_stream(
+                    x2.data_ptr(), _capi.DTYPE_F16 if x.dtype == torch.float16 else _capi.DTYPE_BF16, m, ldx,
+                    layout.tiles.data_ptr(), layout.scales_tiled.data_ptr(), layout.chunk_ptr.data_ptr(),
+                    _capi.ptr(layout.entries), _capi.ptr(layout.vals_sorted), n, k, layout.block_size, _capi.ptr(b),
+                    y.data_ptr(), n, ws.data_ptr(), ws.numel(), status_word(dev).data_ptr(), _capi.stream_ptr(dev))
+        finally:
+            if was is not None:
+                L.atlas_qlinear_plain_launch(was)
         _capi.check(status, "atlas_qlinear_stream")
     return y.view(*x.shape[:-1], n)
 

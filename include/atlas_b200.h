@@ -221,8 +221,8 @@ ATLAS_API int atlas_repack_many(int count, const AtlasRepackItem *items, void *s
  * loads, dequantises in registers and adds the outlier products in the same
  * launch (passes after the first find most of the weight in L2).  Activations
  * that are not 16-byte aligned are read two bytes at a time.  Launched with
- * programmatic dependent launch: only weights are read before the stream's
- * earlier work has completed.  The kernel has no bounded wait: `status` is
+ * programmatic dependent launch: only weights and the bias are read before the
+ * stream's earlier work has completed.  The kernel has no bounded wait: `status` is
  * accepted for symmetry and never written.
  *
  * atlas_qlinear_gemm: larger batches (any m >= 1 accepted).  Code tiles and
@@ -262,11 +262,18 @@ ATLAS_API int atlas_qlinear_gemv(const void *x, int dtype, int64_t m, int64_t ld
  * zero it again.
  *
  * Preconditions shared by the three linear entry points: the weight-side
- * buffers (tiles, scales_tiled, outlier_*) are read before the stream's
- * earlier work has completed, so they must be final before the kernel that
- * precedes the call on the stream was launched (synchronise once after
- * atlas_repack).  x, bias, y, workspace and status are only touched afterwards.
+ * buffers (tiles, scales_tiled, outlier_*) and the bias are read before the
+ * stream's earlier work has completed, so they must be final before the kernel
+ * that precedes the call on the stream was launched: synchronise once after
+ * atlas_repack, or launch plainly (below) until the repack is known to be
+ * finished.  x, y, workspace and status are only touched afterwards.
  */
+/* Switches programmatic dependent launch off (on = 1) or back on (on = 0) for
+ * the linear calls of the calling thread and returns what it was.  A plainly
+ * launched linear starts after everything before it on the stream has ended and
+ * sees all it has written, the repack of its own weights included. */
+ATLAS_API int atlas_qlinear_plain_launch(int on);
+
 ATLAS_API size_t atlas_qlinear_stream_workspace_bytes(int64_t m);
 ATLAS_API int atlas_qlinear_stream(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *tiles,
                                    const void *scales_tiled, const int32_t *outlier_chunk_ptr,
