@@ -67,7 +67,9 @@ class LayoutReady {
         if (done) done_.store(true, std::memory_order_release);
         return done;
     }
+    // Returns once the layout is final, for uses whose order this cannot see (copies, other libraries' kernels).
     void finish() {
+        if (done_.load(std::memory_order_acquire)) return;
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
         const cudaError_t e = cudaEventSynchronize(event_), back = cudaThreadExchangeStreamCaptureMode(&mode);
@@ -283,13 +285,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     py::class_<LayoutReady, std::shared_ptr<LayoutReady>>(m, "LayoutReady")
         .def(py::init<>())
         .def("wait", &LayoutReady::wait, py::call_guard<py::gil_scoped_release>())
-        .def("__reduce__", [](LayoutReady &r) {   // copied or saved: what it stands for is final first, and nothing is left to wait for
-            {
-                py::gil_scoped_release release;
-                r.finish();
-            }
-            return py::make_tuple(py::type::of(py::none()), py::tuple());
-        });
+        .def("finish", &LayoutReady::finish, py::call_guard<py::gil_scoped_release>());
     m.def("build_layout", &build_layout, py::call_guard<py::gil_scoped_release>());
     m.def("quantize_many", &quantize_many, py::call_guard<py::gil_scoped_release>());
     m.def("linear", &linear, py::call_guard<py::gil_scoped_release>());

@@ -49,6 +49,17 @@ class KernelLayout(NamedTuple):
     block_size: int
     ready: object = None           # while the buffers may still be written: what a use on another stream waits for
 
+    def finished(self) -> "KernelLayout":
+        """This layout with its buffers final (the host waits for them) and nothing left to wait for."""
+        if self.ready is None:
+            return self
+        self.ready.finish()
+        return KernelLayout(*self[:-1], None)
+
+    def __reduce__(self):
+        # copies and pickles read the buffers field by field on whatever stream is current: wait before the first one
+        return KernelLayout, tuple(self.finished())
+
 
 _status_words = {}
 

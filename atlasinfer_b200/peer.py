@@ -131,7 +131,7 @@ class GatheredLinear:
             raise ValueError(f"kernel={kernel!r}")
         self.kernel = kernel
         self.arena = arena
-        self.layout = layout
+        self.layout = layout = layout.finished()   # its buffers go straight to the kernels
         self.bias = bias
         self.m_max = int(m_max)
         self.dtype = dtype

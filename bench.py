@@ -414,7 +414,7 @@ def measure_tp70b(rank, world, steps, warmup, barrier, all_forms=False, shard_of
         by_first = {g.members[0]: g for g in layer.groups}
         for names in (("q_proj", "k_proj", "v_proj"), ("o_proj",), ("gate_proj", "up_proj"), ("down_proj",)):
             first = layer.mods[names[0]]
-            lay = by_first[first].layout if first in by_first else first._kernel_layout
+            lay = (by_first[first].layout if first in by_first else first._kernel_layout).finished()
             launches.append((lay, lay.n_rows))
     widths = sorted({w for _, w in launches})
     gathered = {w: torch.empty(world * m, w, dtype=torch.bfloat16, device=dev) for w in widths}

@@ -36,7 +36,7 @@ def _check(got, want):
 
 @pytest.mark.parametrize("fused", [False, True])
 @pytest.mark.parametrize("m", [1, 40, 300])
-@pytest.mark.parametrize("how", ["same", "other", "capture", "copied", "pickled", "freed"])
+@pytest.mark.parametrize("how", ["same", "other", "capture", "copied", "pickled", "copied elsewhere", "pickled elsewhere", "freed"])
 def test_first_uses_of_a_layout(fused, m, how, cuda_device):
     x = torch.randn(m, 1024, device=cuda_device).half()
     mods = _modules(cuda_device, fused)
@@ -68,8 +68,12 @@ def test_first_uses_of_a_layout(fused, m, how, cuda_device):
             got = [mod(x) for mod in mods]
             del trash
         else:
-            again = copy.deepcopy(mods) if how == "copied" else pickle.loads(pickle.dumps(mods))
-            got = [mod(x) for mod in again]
+            # (on a stream that nothing orders behind the one that writes the layouts)
+            side = torch.cuda.Stream() if how.endswith("elsewhere") else torch.cuda.current_stream()
+            with torch.cuda.stream(side):
+                again = copy.deepcopy(mods) if how.startswith("copied") else pickle.loads(pickle.dumps(mods))
+                got = [mod(x) for mod in again]
+            side.synchronize()
     torch.cuda.synchronize()
     _check(first, want)
     _check(got, want)

@@ -1,4 +1,6 @@
 """A kernel layout that is still being written: what its first uses do (no GPU: stand-ins for the event and the kernels)."""
+import copy
+import pickle
 import types
 
 import pytest
@@ -16,6 +18,24 @@ class Ready:
     def wait(self):
         self.left -= 1
         return self.left < 0
+
+    def finish(self):
+        self.left = 0
+        self.log.append("finish")
+
+
+class Buffer(torch.Tensor):
+    """A buffer of a layout that notes when it is copied or pickled."""
+
+    log = []
+
+    def __deepcopy__(self, memo):
+        self.log.append("buffer")
+        return self
+
+    def __reduce_ex__(self, protocol):
+        self.log.append("buffer")
+        return super().__reduce_ex__(protocol)
 
 
 def _layout(ready, n=128, k=64, source=None):
@@ -65,3 +85,50 @@ def test_streaming_form_is_launched_plainly_until_the_layout_is_final(left, monk
         aw.quantized_linear_forward(x, lay, None, force="stream")
     aw.quantized_linear_forward(x, lay, torch.zeros(128), force="stream")   # the conversion of the bias is in front
     assert seen == [int(i < left) for i in range(3)] + [1] and state[-1] == 0
+
+
+def _copies(thing):
+    """``thing`` copied and pickled, each with what happened in which order."""
+    for make in (copy.deepcopy, lambda t: pickle.loads(pickle.dumps(t))):
+        Buffer.log.clear()
+        yield make(thing), list(Buffer.log)
+
+
+def _watched(source, **kw):
+    lay = _layout(Ready(9, Buffer.log), source=source, **kw)
+    return lay._replace(tiles=lay.tiles.as_subclass(Buffer), scales_tiled=lay.scales_tiled.as_subclass(Buffer))
+
+
+def test_a_copied_layout_is_final_before_its_first_buffer_is_read():
+    for again, log in _copies(_watched(None)):
+        assert log[0] == "finish" and log.count("finish") == 1 and "buffer" in log
+        assert type(again) is aw.KernelLayout and again.ready is None and (again.n_rows, again.n_cols) == (128, 64)
+        assert torch.equal(again.tiles, torch.zeros(128 * 64, dtype=torch.uint8))
+    for again, log in _copies(_watched(None)._replace(ready=None)):
+        assert "finish" not in log and again.ready is None
+
+
+def test_copied_modules_and_groups_keep_their_layouts():
+    q = aw.QuantizedTensor(torch.zeros(128 * 64, dtype=torch.int8), torch.zeros(0, dtype=torch.float16),
+                           torch.zeros(0, dtype=torch.long), torch.ones(128, dtype=torch.float16), torch.Size([128, 64]), 64)
+    mods = [aw.QuantizedLinear(q, None), aw.QuantizedLinear(q._replace(block_size=64), None)]
+    group = aw.fuse_linears(mods)
+    lay = _watched((q, mods[1].quantized_weights), n=256)
+    group.layout, group.offsets = lay, [0, 128]
+    for i, mod in enumerate(mods):
+        mod._kernel_layout = aw.slice_layout(lay, 128 * i, 128, mod.quantized_weights)
+    for again, log in _copies(mods):
+        assert log[0] == "finish" and "buffer" in log
+        for mod in again:
+            assert mod._has_layout_for(mod.quantized_weights) and mod._kernel_layout.ready is None
+            assert mod._group.layout.ready is None and mod._group.members[mod._group_index] is mod
+
+
+def test_a_gathered_linear_takes_a_final_layout():
+    from atlasinfer_b200 import peer
+
+    arena = types.SimpleNamespace(world=1, rank=0, bases=[0], state_ptr=0, carve=lambda n: 0, flags_ptr=lambda d: 0,
+                                  local_tensor=lambda off, shape, dtype: None)
+    log = []
+    lin = peer.GatheredLinear(arena, _layout(Ready(9, log)), 4, torch.float16)
+    assert log == ["finish"] and lin.layout.ready is None
