@@ -14,7 +14,8 @@
 // staged with 16-byte copies, and a thread builds 16 bytes of output at a time from one unaligned read of the staged codes;
 // units that hold outliers (every 20th to 40th) are left out of that and built afterwards, one per thread.
 // 11008 x 4096 in blocks of 128: dequantize 52.7 -> 34.9 us (3.9 TB/s; 4096 x 4096 27.2 -> 18.5, 512 x 512 9.3 -> 6.3) against a
-// search of four dependent round trips per span of 16384 and zero bytes slipped in per outlier under divergence; repack
+// search of four dependent round trips per span of 16384 and zero bytes slipped in per outlier under divergence; in blocks of 96
+// or 160 55 -> 35, of 100 101 -> 70, to an output on no 16-byte boundary 84 -> 72; repack
 // 45.2 -> 47 (4096 x 4096 20.6 -> 21.2, 4096 x 11008 45.2 -> 45.5): its strips' lists take as long.  Spans of 4096 and CTAs of
 // 128 threads: 33.6 and 44, but 62 for the repack of 4096 x 11008, whose strips hold 530 outliers.
 #include "common.cuh"
@@ -213,17 +214,23 @@ __global__ void __launch_bounds__(256) mark_dequant_kernel(DequantParams p) {
 }
 
 // One unit (8 elements, 16 bytes of output) per thread and step.  The product of the code and the scale is rounded to fp16
-// once (adaptive_quantizer.py:216).
+// once (adaptive_quantizer.py:216).  POW2: the block size is a power of two; others divide, 32 bits wide, once per unit.
+// Both in one kernel cost the powers of two 1 us of 34 at 11008 x 4096.
+template <bool POW2>
 __global__ void __launch_bounds__(DQ_THREADS) dequantize_kernel(DequantParams p) {
     __shared__ Span s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t span0 = (int64_t)blockIdx.x * DQ_SPAN, span1 = min(span0 + DQ_SPAN, p.padded);
-    const bool whole = span0 + DQ_SPAN <= p.numel && p.w_aligned && p.bs_shift >= 3;   // blocks of whole units
+    const bool in_one_block = (p.bs & 7) == 0;   // blocks are whole units
+    const bool whole = span0 + DQ_SPAN <= p.numel && p.w_aligned && in_one_block;
     constexpr int STEPS = DQ_SPAN / (DQ_THREADS * 8);
     uint16_t sc[STEPS];
-    const uint32_t in_block = whole ? (uint32_t)(span0 & (p.bs - 1)) : 0u;
-    const uint16_t *scales = p.scales + (whole ? span0 >> p.bs_shift : 0);
-    auto scale_of = [&](int unit) { return __ldg(scales + ((in_block + (uint32_t)unit * 8u) >> p.bs_shift)); };
+    // the span's first block, and the place of its first element in it: below, 32 bits do
+    const int64_t block0 = POW2 ? span0 >> p.bs_shift : span0 / p.bs;
+    const uint32_t in_block = POW2 ? (uint32_t)(span0 & (p.bs - 1)) : (uint32_t)(span0 - block0 * p.bs);
+    const uint16_t *scales = p.scales + block0;
+    auto block_of = [&](uint32_t e) { return POW2 ? (in_block + e) >> p.bs_shift : (in_block + e) / (uint32_t)p.bs; };
+    auto scale_of = [&](int unit) { return __ldg(scales + block_of((uint32_t)unit * 8u)); };
 #pragma unroll
     for (int k = 0; k < STEPS; ++k) sc[k] = whole ? scale_of(tid + k * DQ_THREADS) : (uint16_t)0;
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -242,6 +249,18 @@ __global__ void __launch_bounds__(DQ_THREADS) dequantize_kernel(DequantParams p)
         __syncthreads();
     }
     stage_span(s, p.codes, p.n_codes, p.oidx, p.n_out, ends, span0, span1);
+    // the outliers of a unit (`bits`), the first of which is the span's outlier number `before`, into its output
+    auto put_outliers = [&](uint32_t (&o)[4], uint32_t bits, uint32_t before) {
+        const uint16_t *val = p.ovals + s.lo + before;
+        for (uint32_t m = bits; m; m &= m - 1, ++val) {
+            const int j = __ffs(m) - 1;
+            const uint32_t v = __ldg(val);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (q == j >> 1) o[q] = (j & 1) ? __byte_perm(o[q], v, 0x5410) : __byte_perm(o[q], v, 0x3254);
+        }
+    };
+    const uint32_t shift = (uint32_t)((uintptr_t)(p.codes + (span0 - s.lo)) & 15);   // where stage_span put the first code
     if (whole) {
 #pragma unroll
         for (int k = 0; k < STEPS; ++k) {
@@ -255,31 +274,69 @@ __global__ void __launch_bounds__(DQ_THREADS) dequantize_kernel(DequantParams p)
         for_units_with_outliers<3>(s, p.oidx, span0, [&](int unit) {
             uint32_t word, c[2], o[4];
             const uint32_t at = code_at(s, unit * 8, word), bits = (word >> ((unit & 3) * 8)) & 0xffu;
-            const uint32_t before = (uint32_t)((uintptr_t)(p.codes + (span0 - s.lo)) & 15) + (uint32_t)unit * 8u - at;   // outliers in front
-            const uint16_t *val = p.ovals + s.lo + before;
             codes_around<2>(s, at, bits, c);
             scale_unit(c, scale_of(unit), o);
-            for (uint32_t m = bits; m; m &= m - 1, ++val) {
-                const int j = __ffs(m) - 1;
-                const uint32_t v = __ldg(val);
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (q == j >> 1) o[q] = (j & 1) ? __byte_perm(o[q], v, 0x5410) : __byte_perm(o[q], v, 0x3254);
-            }
+            put_outliers(o, bits, shift + (uint32_t)unit * 8u - at);
             *reinterpret_cast<uint4 *>(w + unit * 8) = make_uint4(o[0], o[1], o[2], o[3]);
         });
         return;
     }
-    // the last span, any block size, any alignment: element by element
-    for (int e = tid; e < DQ_SPAN && span0 + e < p.numel; e += DQ_THREADS) {
-        const int64_t gp = span0 + e;
-        uint32_t word;
-        const uint32_t at = code_at(s, e, word);
-        if ((word >> (e & 31)) & 1u) {
-            w[e] = __ldg(p.ovals + s.lo + ((uint32_t)((uintptr_t)(p.codes + (span0 - s.lo)) & 15) + (uint32_t)e - at));
+    const int real = (int)min((int64_t)DQ_SPAN, p.numel - span0);   // (none or less: blocks of padding alone)
+    if (!p.w_aligned) {
+        // an output on no 16-byte boundary: element by element, so that a warp's 2-byte stores are neighbours (eight of a
+        // thread's own in a row are 10 % slower)
+        const uint32_t bs = (uint32_t)p.bs, blocks_on = POW2 ? 0u : DQ_THREADS / bs, in_block_on = POW2 ? 0u : DQ_THREADS % bs;
+        uint32_t block = block_of(tid), place = POW2 ? 0u : in_block + tid - block * bs;
+        for (int e = tid; e < real; e += DQ_THREADS) {
+            if (POW2) block = block_of(e);
+            const uint16_t scale = __ldg(scales + block);
+            if (!POW2) {   // the next element's block, without another division
+                block += blocks_on;
+                place += in_block_on;
+                if (place >= bs) {
+                    place -= bs;
+                    ++block;
+                }
+            }
+            uint32_t word;
+            const uint32_t at = code_at(s, e, word);
+            if ((word >> (e & 31)) & 1u) {
+                w[e] = __ldg(p.ovals + s.lo + (shift + (uint32_t)e - at));
+            } else {
+                const __half code = __short2half_rn((short)(int8_t)s.codes[at]);
+                w[e] = __half_as_ushort(__hmul(code, __ushort_as_half(scale)));
+            }
+        }
+        return;
+    }
+    // the last span, and blocks that end inside a unit
+#pragma unroll 1
+    for (int unit = tid; unit * 8 < real; unit += DQ_THREADS) {
+        uint32_t word, c[2], o[4];
+        const uint32_t at = code_at(s, unit * 8, word), bits = (word >> ((unit & 3) * 8)) & 0xffu;
+        if (bits) codes_around<2>(s, at, bits, c);
+        else codes_at<2>(s, at, c);
+        if (in_one_block) {
+            scale_unit(c, scale_of(unit), o);
         } else {
-            const __half code = __short2half_rn((short)(int8_t)s.codes[at]);
-            w[e] = __half_as_ushort(__hmul(code, __ushort_as_half(__ldg(p.scales + (p.bs_shift >= 0 ? gp >> p.bs_shift : gp / p.bs)))));
+            // (at most every place has a block of its own, and places beyond the padded end have none)
+            __half2 h[4] = {code_pair<0x5140>(c[0]), code_pair<0x5342>(c[0]), code_pair<0x5140>(c[1]), code_pair<0x5342>(c[1])};
+            const int last = real - 1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint16_t a = __ldg(scales + block_of((uint32_t)min(unit * 8 + 2 * i, last)));
+                const uint16_t b = __ldg(scales + block_of((uint32_t)min(unit * 8 + 2 * i + 1, last)));
+                h[i] = __hmul2(h[i], __halves2half2(__ushort_as_half(a), __ushort_as_half(b)));
+                o[i] = *reinterpret_cast<uint32_t *>(&h[i]);
+            }
+        }
+        put_outliers(o, bits, shift + (uint32_t)unit * 8u - at);
+        if (unit * 8 + 8 <= real) {
+            *reinterpret_cast<uint4 *>(w + unit * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (unit * 8 + e < real) w[unit * 8 + e] = (uint16_t)(o[e >> 1] >> (16 * (e & 1)));
         }
     }
 }
@@ -547,7 +604,7 @@ int atlas_dequantize(const int8_t *codes, int64_t n_codes, const void *outlier_v
         rc = check_cuda(cudaGetLastError(), "mark_dequant_kernel launch");
         if (rc) return rc;
     }
-    return launch_beside(dequantize_kernel, (unsigned)spans, p.marked, (cudaStream_t)stream, p);
+    return launch_beside(p.bs_shift >= 0 ? dequantize_kernel<true> : dequantize_kernel<false>, (unsigned)spans, p.marked, (cudaStream_t)stream, p);
 }
 
 size_t atlas_tiles_bytes(int64_t n_rows, int64_t n_cols) {

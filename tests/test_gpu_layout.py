@@ -1,9 +1,10 @@
-"""The dequantizer and the kernel layout at the edges of their 16384-element spans, byte for byte."""
+"""The dequantizer and the kernel layout at the edges of their 8192-element spans, byte for byte."""
 import numpy as np
 import pytest
 import torch
 
 import atlasinfer_b200 as ab
+from atlasinfer_b200 import _capi
 from atlasinfer_b200.integration import atlas_wrappers as aw
 from atlasinfer_b200.quant import adaptive_quantizer as aq
 from oracle import atlas_oracle as O
@@ -31,6 +32,22 @@ def test_dequantize_span_edges(numel, bs, share, cuda_device):
     o = _streams(numel, bs, share, numel + bs)
     got = aq._dequantize_on_device(ab.QuantizedTensor(*o).to(cuda_device), cuda_device)
     assert torch.equal(bits(got.cpu()), bits(O.dequantize(o)))
+
+
+# blocks of whole units and others, whole spans and a last one that ends inside a unit, outputs on any boundary
+@pytest.mark.parametrize("numel", [3 * 8192, 3 * 8192 + 20, 40000])
+@pytest.mark.parametrize("bs", [4, 8, 24, 96, 100, 128, 160, 288, 20000])
+@pytest.mark.parametrize("share", [0.003, 0.06])   # outliers searched for and marked
+@pytest.mark.parametrize("off", [0, 1, 4, 8])
+def test_dequantize_every_block_and_alignment(numel, bs, share, off, cuda_device):
+    o = _streams(numel, bs, share, numel + bs)
+    q, room = ab.QuantizedTensor(*o).to(cuda_device), torch.full((numel + 16,), 7, dtype=torch.float16, device=cuda_device)
+    _capi.check(_capi.load().atlas_dequantize(
+        _capi.ptr(q.fp8_data), q.fp8_data.numel(), _capi.ptr(q.fp16_outliers), _capi.ptr(q.outlier_indices), q.outlier_indices.numel(),
+        q.scale_factors.data_ptr(), numel, bs, room.data_ptr() + 2 * off, _capi.stream_ptr(cuda_device)), "atlas_dequantize")
+    room = room.cpu()
+    assert torch.equal(bits(room[off:off + numel]), bits(O.dequantize(o)))
+    assert (room[:off] == 7).all() and (room[off + numel:] == 7).all()
 
 
 @pytest.mark.parametrize("off", [1, 5, 15])
