@@ -10,7 +10,10 @@
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <algorithm>
 #include <atomic>
+#include <memory>
+#include <mutex>
 
 #include "atlas_b200.h"
 
@@ -27,6 +30,63 @@ void check(int status, const char *what) {
 
 const void *ptr_or_null(const at::Tensor &t) { return t.numel() ? t.data_ptr() : nullptr; }
 
+// The layouts that one stream writes: an event that is recorded again behind every further one, so that one look at it settles
+// all of them.  An event of each layout's own costs the first pass after loading a query and a destruction per launch (a small
+// layer for one token, six modules in four launches, best of twelve first passes: 97 us, so 87, with the host waiting at
+// every build instead 80).  A use on another stream may wait for later layouts of that stream too.
+struct StreamLayouts {
+    const int device;
+    const unsigned long long id;   // of the stream, for the life of the process (a handle may be used again)
+    cudaEvent_t event = nullptr;
+    std::mutex lock;               // the event, and what it stands behind
+    uint64_t enqueued = 0;         // layouts; the event stands behind the last
+    std::atomic<uint64_t> final{0};   // of them known to be final
+
+    StreamLayouts(int device, unsigned long long id) : device(device), id(id) {
+        C10_CUDA_CHECK(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
+    }
+    ~StreamLayouts() { cudaEventDestroy(event); }
+    StreamLayouts(const StreamLayouts &) = delete;
+
+    void settle(uint64_t upto) {
+        uint64_t was = final.load(std::memory_order_relaxed);
+        while (was < upto && !final.compare_exchange_weak(was, upto, std::memory_order_release, std::memory_order_relaxed)) {}
+    }
+    // The host waits for all layouts enqueued so far.
+    cudaError_t synchronize() {
+        uint64_t upto;
+        {
+            const std::lock_guard<std::mutex> held(lock);
+            upto = enqueued;
+        }
+        const cudaError_t e = cudaEventSynchronize(event);
+        if (e == cudaSuccess) settle(upto);
+        return e;
+    }
+    // cudaSuccess: all layouts enqueued so far are final; cudaErrorNotReady: not yet.
+    cudaError_t look() {
+        const std::lock_guard<std::mutex> held(lock);
+        const cudaError_t e = cudaEventQuery(event);
+        if (e == cudaSuccess) settle(enqueued);
+        return e;
+    }
+};
+
+// The current stream's.  Those of streams that no layout looks at any more are given back once there are more than 16.
+std::shared_ptr<StreamLayouts> stream_layouts(int device, cudaStream_t stream) {
+    static std::mutex lock;
+    static auto *known = new std::vector<std::shared_ptr<StreamLayouts>>;   // (never destroyed: the driver may be gone by then)
+    unsigned long long id = 0;
+    C10_CUDA_CHECK(cudaStreamGetId(stream, &id));
+    const std::lock_guard<std::mutex> held(lock);
+    for (const auto &s : *known)
+        if (s->device == device && s->id == id) return s;
+    if (known->size() >= 16)
+        known->erase(std::remove_if(known->begin(), known->end(), [](const auto &s) { return s.use_count() == 1; }), known->end());
+    known->push_back(std::make_shared<StreamLayouts>(device, id));
+    return known->back();
+}
+
 // Stands for a layout that may still be written by the stream it was enqueued on.  The linear kernels read weights before
 // the stream's earlier work has completed (programmatic dependent launch): a dependent starts once the kernel in front has
 // ended, but sees its stores for certain only behind griddepcontrol.wait.  Until the layout is known to be final, a linear
@@ -35,54 +95,53 @@ const void *ptr_or_null(const at::Tensor &t) { return t.numel() ? t.data_ptr() :
 class LayoutReady {
    public:
     LayoutReady() {
-        device_ = at::cuda::current_device();
-        stream_ = at::cuda::getCurrentCUDAStream(device_).stream();
-        C10_CUDA_CHECK(cudaEventCreateWithFlags(&event_, cudaEventDisableTiming));
-        C10_CUDA_CHECK(cudaEventRecord(event_, stream_));
+        const int device = at::cuda::current_device();
+        const cudaStream_t stream = at::cuda::getCurrentCUDAStream(device).stream();
+        on_ = stream_layouts(device, stream);
+        const std::lock_guard<std::mutex> held(on_->lock);
+        C10_CUDA_CHECK(cudaEventRecord(on_->event, stream));
+        number_ = ++on_->enqueued;
     }
-    ~LayoutReady() { cudaEventDestroy(event_); }
     LayoutReady(const LayoutReady &) = delete;
     // True once the layout is final.  False: not yet, but what is launched plainly on the current stream comes after it.
     bool wait() {
-        if (done_.load(std::memory_order_acquire)) return true;
-        const cudaStream_t on = at::cuda::getCurrentCUDAStream(device_).stream();
-        // (none of these calls touches a capture of this or another thread)
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+        if (is_final()) return true;
+        const cudaStream_t stream = at::cuda::getCurrentCUDAStream(on_->device).stream();
+        const CaptureUntouched scope;
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        cudaError_t e = cudaStreamIsCapturing(on, &capture);
-        bool done = false;
-        if (e == cudaSuccess && on == stream_ && capture == cudaStreamCaptureStatusNone) {
-            const cudaError_t q = cudaEventQuery(event_);
-            done = q == cudaSuccess;
-            if (q == cudaErrorNotReady) (void)cudaGetLastError();
-            else e = q;
-        } else if (e == cudaSuccess) {
-            e = cudaEventSynchronize(event_);
-            done = e == cudaSuccess;
+        unsigned long long id = on_->id;
+        C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &capture));
+        if (capture == cudaStreamCaptureStatusNone) C10_CUDA_CHECK(cudaStreamGetId(stream, &id));   // (refused in a capture)
+        if (id == on_->id && capture == cudaStreamCaptureStatusNone) {
+            const cudaError_t e = on_->look();
+            if (e == cudaErrorNotReady) {
+                (void)cudaGetLastError();
+                return false;
+            }
+            C10_CUDA_CHECK(e);
+        } else {
+            C10_CUDA_CHECK(on_->synchronize());
         }
-        const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
-        C10_CUDA_CHECK(e);
-        C10_CUDA_CHECK(back);
-        if (done) done_.store(true, std::memory_order_release);
-        return done;
+        return true;
     }
     // Returns once the layout is final, for uses whose order this cannot see (copies, other libraries' kernels).
     void finish() {
-        if (done_.load(std::memory_order_acquire)) return;
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
-        const cudaError_t e = cudaEventSynchronize(event_), back = cudaThreadExchangeStreamCaptureMode(&mode);
-        C10_CUDA_CHECK(e);
-        C10_CUDA_CHECK(back);
-        done_.store(true, std::memory_order_release);
+        if (is_final()) return;
+        const CaptureUntouched scope;
+        C10_CUDA_CHECK(on_->synchronize());
     }
 
    private:
-    int device_;
-    cudaStream_t stream_;
-    cudaEvent_t event_ = nullptr;
-    std::atomic<bool> done_{false};
+    // None of the calls in its scope touches a capture of this or another thread.
+    struct CaptureUntouched {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        CaptureUntouched() { C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode)); }
+        ~CaptureUntouched() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    };
+    bool is_final() const { return on_->final.load(std::memory_order_acquire) >= number_; }
+
+    std::shared_ptr<StreamLayouts> on_;
+    uint64_t number_ = 0;
 };
 
 // The linears of this scope are launched plainly (`on`), or as the thread has it.
