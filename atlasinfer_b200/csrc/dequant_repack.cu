@@ -3,11 +3,12 @@
 //
 // Replaces dequantize_tensor (atlasinfer_core/quant/adaptive_quantizer.py:156-251).
 // The reference keeps a running offset into the code stream and, per block,
-// masks the whole outlier index list (:194-196, O(blocks x outliers)).  Here a
-// first kernel finds, for all spans of 8192 elements in one pass over the sorted
-// index list, where a span's outliers begin and end; the number of outliers
-// before the span gives its offset into the compacted code stream (position
-// minus outliers before it), so every span is independent.
+// masks the whole outlier index list (:194-196, O(blocks x outliers)).  Here
+// every span of 8192 elements finds where its outliers begin and end in the
+// sorted index list, by a search or, dequantizing, from a first kernel's one pass
+// over the list for all spans; the number of outliers before the span gives its
+// offset into the compacted code stream (position minus outliers before it), so
+// every span is independent.
 //
 // Both directions only move bytes: HBM is the bound in principle (1.04 bytes read per element, 2 or 1 written), memory latency
 // and instructions in practice.  A span's outlier positions become a bit mask with a code offset per word, its codes are
@@ -16,8 +17,9 @@
 // 11008 x 4096 in blocks of 128: dequantize 52.7 -> 34.9 us (3.9 TB/s; 4096 x 4096 27.2 -> 18.5, 512 x 512 9.3 -> 6.3) against a
 // search of four dependent round trips per span of 16384 and zero bytes slipped in per outlier under divergence; in blocks of 96
 // or 160 55 -> 35, of 100 101 -> 70, to an output on no 16-byte boundary 84 -> 72; repack
-// 45.2 -> 47 (4096 x 4096 20.6 -> 21.2, 4096 x 11008 45.2 -> 45.5): its strips' lists take as long.  Spans of 4096 and CTAs of
-// 128 threads: 33.6 and 44, but 62 for the repack of 4096 x 11008, whose strips hold 530 outliers.
+// 43.2 -> 39.9 (4096 x 4096 18.6 -> 18.6, 4096 x 11008 43.1 -> 40.4; with the spans marked beforehand 45.2, 20.6 and 44.2, and
+// with ten times the outliers 4096 x 4096 343 instead of 234): its strips' lists take as long.  Spans of 4096 and CTAs of 128
+// threads: 33.6 for the dequantizer, but 62 for the repack of 4096 x 11008, whose strips hold 530 outliers.
 #include "common.cuh"
 
 namespace atlas {
@@ -84,10 +86,24 @@ struct Span {
     __align__(16) uint8_t codes[DQ_SPAN + 48];
 };
 
+// The ends of the span [span0, span1) in the outlier list, searched for by two warps of the CTA.
+__device__ __forceinline__ Ends search_span(Span &s, const int64_t *oidx, int64_t n_out, int64_t span0, int64_t span1) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < 2) {
+        const int64_t r = warp_lower_bound(oidx, n_out, warp == 0 ? span0 : span1, lane);
+        if (lane == 0) (warp == 0 ? s.lo : s.hi) = r;
+    }
+    __syncthreads();
+    const Ends ends = {s.lo, s.hi};
+    __syncthreads();
+    return ends;
+}
+
 // Stages the span [span0, span1), whose outliers are [lo, hi): mask, code offsets and codes.  Nothing outside
 // codes[0, n_codes) and oidx[0, n_out) is read, whatever oidx and the ends hold; if oidx is not ascending (a damaged file) the
-// values are arbitrary, but hi >= lo keeps the staged length within the span and, as every bit of the mask stands for an index
-// in [lo, hi), the outliers read within [lo, hi) too.
+// values are arbitrary and need not repeat (a marked span may have no ends of its own, nor all of its codes be staged), but
+// hi >= lo keeps the staged length within the span and, as every bit of the mask stands for an index in [lo, hi), the
+// outliers read within [lo, hi) too.
 __device__ __forceinline__ void stage_span(Span &s, const int8_t *codes, int64_t n_codes, const int64_t *oidx, int64_t n_out, Ends ends,
                                            int64_t span0, int64_t span1) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -219,7 +235,7 @@ __global__ void __launch_bounds__(256) mark_dequant_kernel(DequantParams p) {
 template <bool POW2>
 __global__ void __launch_bounds__(DQ_THREADS) dequantize_kernel(DequantParams p) {
     __shared__ Span s;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const int64_t span0 = (int64_t)blockIdx.x * DQ_SPAN, span1 = min(span0 + DQ_SPAN, p.padded);
     const bool in_one_block = (p.bs & 7) == 0;   // blocks are whole units
     const bool whole = span0 + DQ_SPAN <= p.numel && p.w_aligned && in_one_block;
@@ -240,13 +256,7 @@ __global__ void __launch_bounds__(DQ_THREADS) dequantize_kernel(DequantParams p)
         const volatile Ends *at = reinterpret_cast<const volatile Ends *>(w);   // (all threads, before any of them writes)
         ends = {at->lo, at->hi};
     } else {
-        if (warp < 2) {
-            const int64_t r = warp_lower_bound(p.oidx, p.n_out, warp == 0 ? span0 : span1, lane);
-            if (lane == 0) (warp == 0 ? s.lo : s.hi) = r;
-        }
-        __syncthreads();
-        ends = {s.lo, s.hi};
-        __syncthreads();
+        ends = search_span(s, p.oidx, p.n_out, span0, span1);
     }
     stage_span(s, p.codes, p.n_codes, p.oidx, p.n_out, ends, span0, span1);
     // the outliers of a unit (`bits`), the first of which is the span's outlier number `before`, into its output
@@ -415,16 +425,6 @@ __device__ __forceinline__ void write_strip(const RepackTensor &t, int64_t strip
     }
 }
 
-__global__ void __launch_bounds__(256) mark_repack_kernel(const __grid_constant__ RepackParams p) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const RepackTensor &t = p.t[blockIdx.y];
-    const int64_t spans = (t.n_rows * t.n_cols + DQ_SPAN - 1) / DQ_SPAN;
-    mark_spans(t.oidx, t.n_out, spans, (int64_t)blockIdx.x * 256 + threadIdx.x, threadIdx.x & 31, [&](int64_t span) {
-        const int64_t at = span * DQ_SPAN, row = at / t.n_cols;
-        return reinterpret_cast<Ends *>(t.tiles + tile_offset(row, at - row * t.n_cols, t.n_cols >> 6));
-    });
-}
-
 // One launch expands up to DQ_MAX_REPACK tensors; a CTA does one of three jobs: the outlier lists of a strip (first in
 // the grid: the longest chain of dependent loads), a 128-row x 16-block piece of the scale transposition, or 8192
 // positions of the code tiles, 16 codes (one unit of the layout; n_cols is a multiple of 64, so a unit never straddles
@@ -524,10 +524,11 @@ __global__ void __launch_bounds__(DQ_THREADS) repack_kernel(const __grid_constan
         const uint32_t c = col0 + q, dr = c / n_cols, col = c - dr * n_cols, row = in_tile + dr;
         return tiles + ((uint64_t)((row >> 7) * k_tiles + (col >> 6)) * 8192u + (row & 127u) * 64u + (col & 63u));
     };
-    asm volatile("griddepcontrol.wait;" ::: "memory");   // the marks
     if (span0 < numel) {
-        const volatile Ends *at = reinterpret_cast<const volatile Ends *>(place(0));   // (all threads, before any of them writes)
-        stage_span(sh.span, t.codes, t.n_codes, t.oidx, t.n_out, Ends{at->lo, at->hi}, span0, span1);
+        // (a search in every CTA: they begin while the strips are at work, and marking the spans beforehand, as the
+        // dequantizer does, only held them up: 11008 x 4096 45 us, so 40)
+        const Ends ends = search_span(sh.span, t.oidx, t.n_out, span0, span1);
+        stage_span(sh.span, t.codes, t.n_codes, t.oidx, t.n_out, ends, span0, span1);
     }
 #pragma unroll
     for (int k = 0; k < DQ_SPAN / (DQ_THREADS * 16); ++k) {
@@ -546,9 +547,8 @@ __global__ void __launch_bounds__(DQ_THREADS) repack_kernel(const __grid_constan
         });
 }
 
-// Launches a kernel whose CTAs may start while the marking kernel in front of it still runs.
-template <class Kernel, class Params>
-int launch_beside(Kernel kernel, unsigned grid, bool beside, cudaStream_t st, const Params &p) {
+// Launches the dequantizer, whose CTAs may start while the marking kernel in front of it still runs (`beside`).
+int launch_dequantize(unsigned grid, bool beside, cudaStream_t st, const DequantParams &p) {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -558,7 +558,7 @@ int launch_beside(Kernel kernel, unsigned grid, bool beside, cudaStream_t st, co
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = beside ? 1 : 0;
-    return check_cuda(cudaLaunchKernelEx(&cfg, kernel, p), "dequantize / repack launch");
+    return check_cuda(cudaLaunchKernelEx(&cfg, p.bs_shift >= 0 ? dequantize_kernel<true> : dequantize_kernel<false>, p), "dequantize_kernel launch");
 }
 
 }  // namespace
@@ -604,7 +604,7 @@ int atlas_dequantize(const int8_t *codes, int64_t n_codes, const void *outlier_v
         rc = check_cuda(cudaGetLastError(), "mark_dequant_kernel launch");
         if (rc) return rc;
     }
-    return launch_beside(p.bs_shift >= 0 ? dequantize_kernel<true> : dequantize_kernel<false>, (unsigned)spans, p.marked, (cudaStream_t)stream, p);
+    return launch_dequantize((unsigned)spans, p.marked, (cudaStream_t)stream, p);
 }
 
 size_t atlas_tiles_bytes(int64_t n_rows, int64_t n_cols) {
@@ -669,12 +669,8 @@ int atlas_repack_many(int count, const AtlasRepackItem *items, void *stream) {
             end += strips + scale_ctas + code_ctas;
             t.block_end = (uint32_t)end;
         }
-        int64_t most = 0;
-        for (int i = 0; i < p.n; ++i) most = p.t[i].n_out > most ? p.t[i].n_out : most;
-        mark_repack_kernel<<<dim3((unsigned)ceil_div_i64(most + 1, 256), (unsigned)p.n), 256, 0, (cudaStream_t)stream>>>(p);
-        rc = check_cuda(cudaGetLastError(), "mark_repack_kernel launch");
-        if (rc) return rc;
-        rc = launch_beside(repack_kernel, (unsigned)end, true, (cudaStream_t)stream, p);
+        repack_kernel<<<(unsigned)end, DQ_THREADS, 0, (cudaStream_t)stream>>>(p);
+        rc = check_cuda(cudaGetLastError(), "repack_kernel launch");
         if (rc) return rc;
     }
     return ATLAS_OK;

@@ -50,6 +50,58 @@ def test_dequantize_every_block_and_alignment(numel, bs, share, off, cuda_device
     assert (room[:off] == 7).all() and (room[off + numel:] == 7).all()
 
 
+def _clustered(n, k, bs, clusters, seed):
+    """Streams of an [n, k] tensor whose outliers fill ``clusters`` (first position, length, every how many)."""
+    gen = torch.Generator().manual_seed(seed)
+    out = torch.zeros(n * k, dtype=torch.bool)
+    for first, length, step in clusters:
+        out[first:first + length:step] = True
+    idx = out.nonzero().flatten()
+    codes = torch.randint(-127, 128, (n * k - idx.numel(),), generator=gen).to(torch.int8)
+    scales = (torch.rand(n * k // bs, generator=gen) * 1e-3 + 1e-6).half()
+    return O.OracleQuantized(codes, torch.randn(idx.numel(), generator=gen).half(), idx, scales, torch.Size([n, k]), bs)
+
+
+# long runs of spans without outliers before, between and behind clusters of more of them than are searched for
+@pytest.mark.parametrize("clusters", [
+    [(0, 2000, 1)], [(300 * 4096 - 2000, 2000, 1)], [(40 * 8192 - 1, 4000, 2), (120 * 8192 + 8191, 2, 1)],
+    [(17, 1, 1), (50 * 8192, 8192, 1), (58 * 8192, 8192, 3), (100 * 8192 + 5, 1, 1)], [(i * 32 * 8192 - 64, 700, 3) for i in range(1, 5)]])
+@pytest.mark.parametrize("bs", [128, 64])
+def test_clusters_of_outliers(clusters, bs, cuda_device):
+    o = _clustered(300, 4096, bs, clusters, bs)
+    assert o.outlier_indices.numel() > 900
+    q = ab.QuantizedTensor(*o).to(cuda_device)
+    assert torch.equal(bits(aq._dequantize_on_device(q, cuda_device).cpu()), bits(O.dequantize(o)))
+    _assert_layout(aw.build_kernel_layout(q), _layout_reference(o))
+
+
+@pytest.mark.parametrize("damage", ["shuffled", "reversed", "negative", "beyond", "equal"])
+def test_damaged_indices_stay_inside_the_output(damage, cuda_device):
+    """The values are arbitrary, but nothing outside the buffers is written, and a layout points into its own lists."""
+    o = _clustered(300, 4096, 128, [(100 * 8192, 3000, 1)], 9)
+    idx = o.outlier_indices.clone()
+    if damage == "shuffled":
+        idx = idx[torch.randperm(idx.numel(), generator=torch.Generator().manual_seed(2))]
+    elif damage == "reversed":
+        idx = idx.flip(0)
+    elif damage == "negative":
+        idx[1500] = -(1 << 40)
+    elif damage == "beyond":
+        idx[1500:] = 1 << 60
+    else:
+        idx[:] = idx[0]
+    q, numel = ab.QuantizedTensor(*o._replace(outlier_indices=idx)).to(cuda_device), 300 * 4096
+    room = torch.full((numel + 4096,), 7, dtype=torch.float16, device=cuda_device)
+    _capi.check(_capi.load().atlas_dequantize(
+        q.fp8_data.data_ptr(), q.fp8_data.numel(), q.fp16_outliers.data_ptr(), q.outlier_indices.data_ptr(), idx.numel(),
+        q.scale_factors.data_ptr(), numel, 128, room.data_ptr() + 4096, _capi.stream_ptr(cuda_device)), "atlas_dequantize")
+    assert (room[:2048] == 7).all() and (room[2048 + numel:] == 7).all()
+    lay = aw.build_kernel_layout(q)
+    again = aw.build_kernel_layout(q)
+    assert torch.equal(lay.chunk_ptr, again.chunk_ptr)
+    assert int(lay.chunk_ptr.min()) >= 0 and int(lay.chunk_ptr.max()) <= idx.numel()
+
+
 @pytest.mark.parametrize("off", [1, 5, 15])
 def test_dequantize_unaligned_codes(off, cuda_device):
     o = _streams(30000, 128, 0.01, off)
