@@ -25,7 +25,7 @@ EXPORTS = (
     "atlas_quantize_many_workspace_bytes", "atlas_quantize_many", "atlas_copy_many",
     "atlas_tiles_bytes", "atlas_repack", "atlas_repack_many", "atlas_qlinear_gemv",
     "atlas_qlinear_stream_workspace_bytes", "atlas_qlinear_stream", "atlas_qlinear_stream_gather",
-    "atlas_qlinear_plain_launch", "atlas_peer_wait", "atlas_peer_push", "atlas_peer_alloc", "atlas_peer_free", "atlas_peer_export", "atlas_peer_import",
+    "atlas_qlinear_plain_launch", "atlas_qlinear_gemm_plan", "atlas_peer_wait", "atlas_peer_push", "atlas_peer_alloc", "atlas_peer_free", "atlas_peer_export", "atlas_peer_import",
     "atlas_peer_release",
     "atlas_qlinear_gemm_workspace_bytes", "atlas_qlinear_gemm", "atlas_qlinear_gemm_gather",
 )
@@ -116,6 +116,8 @@ def load() -> ctypes.CDLL:
     lin = [vp, i32, i64, i64, vp, vp, vp, vp, vp, i64, i64, i32, vp, vp, i64]
     L.atlas_qlinear_gemv.restype = i32
     L.atlas_qlinear_gemv.argtypes = lin + [vp, vp]
+    L.atlas_qlinear_gemm_plan.restype = i32
+    L.atlas_qlinear_gemm_plan.argtypes = [i64, i64, i64, ctypes.POINTER(i32), ctypes.POINTER(i32)]
     L.atlas_qlinear_plain_launch.restype = i32
     L.atlas_qlinear_plain_launch.argtypes = [i32]
     L.atlas_qlinear_stream_workspace_bytes.restype = sz

@@ -233,7 +233,8 @@ ATLAS_API int atlas_repack_many(int count, const AtlasRepackItem *items, void *s
  * memory (token tiles of 32 to 128) and K is sliced over up to 16 CTAs whose
  * partial tiles a second kernel adds in slice order: whichever a model of the
  * two takes to be faster for the shape.  More rows: the latter, with token tiles
- * of 256 and slices only where the tiles leave much of the chip idle.
+ * of 160 to 384 and slices only where the tiles leave much of the chip idle
+ * (atlas_qlinear_gemm_plan).
  * Deterministic either way.
  * `workspace` must hold atlas_qlinear_gemm_workspace_bytes(m, n_rows, n_cols)
  * bytes, 256-byte aligned.
@@ -368,6 +369,9 @@ ATLAS_API int atlas_peer_export(void *ptr, unsigned char *handle);
 ATLAS_API int atlas_peer_import(const unsigned char *handle, void **ptr);
 ATLAS_API int atlas_peer_release(void *ptr);
 
+/* How atlas_qlinear_gemm runs more than 128 rows: the tokens of a tile and the
+ * K slices (on the current device; without one, as on 148 SMs). */
+ATLAS_API int atlas_qlinear_gemm_plan(int64_t m, int64_t n_rows, int64_t n_cols, int *tokens, int *slices);
 ATLAS_API size_t atlas_qlinear_gemm_workspace_bytes(int64_t m, int64_t n_rows, int64_t n_cols);
 ATLAS_API int atlas_qlinear_gemm(const void *x, int dtype, int64_t m, int64_t ldx, const uint8_t *tiles,
                                  const void *scales_tiled, const int32_t *outlier_chunk_ptr,
