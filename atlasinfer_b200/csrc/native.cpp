@@ -31,9 +31,8 @@ void check(int status, const char *what) {
 const void *ptr_or_null(const at::Tensor &t) { return t.numel() ? t.data_ptr() : nullptr; }
 
 // The layouts that one stream writes: an event that is recorded again behind every further one, so that one look at it settles
-// all of them.  An event of each layout's own costs the first pass after loading a query and a destruction per launch (a small
-// layer for one token, six modules in four launches, best of twelve first passes: 97 us, so 87, with the host waiting at
-// every build instead 80).  A use on another stream may wait for later layouts of that stream too.
+// all of them (an event of each layout's own costs the first pass after loading a query and a destruction per launch).  A use
+// on another stream may wait for later layouts of that stream too.
 struct StreamLayouts {
     const int device;
     const unsigned long long id;   // of the stream, for the life of the process (a handle may be used again)
@@ -114,16 +113,23 @@ class LayoutReady {
         if (capture == cudaStreamCaptureStatusNone) C10_CUDA_CHECK(cudaStreamGetId(stream, &id));   // (refused in a capture)
         if (id == on_->id && capture == cudaStreamCaptureStatusNone) {
             const cudaError_t e = on_->look();
-            if (e == cudaErrorNotReady) {
-                (void)cudaGetLastError();
-                return false;
-            }
-            C10_CUDA_CHECK(e);
-        } else {
-            C10_CUDA_CHECK(on_->synchronize());
+            if (e == cudaErrorNotReady) (void)cudaGetLastError();
+            else C10_CUDA_CHECK(e);
+            return e == cudaSuccess;
         }
+        C10_CUDA_CHECK(on_->synchronize());
         return true;
     }
+    // Whether it is final, whatever stream is current.
+    bool done() {
+        if (is_final()) return true;
+        const CaptureUntouched scope;
+        const cudaError_t e = on_->look();
+        if (e == cudaErrorNotReady) (void)cudaGetLastError();
+        else C10_CUDA_CHECK(e);
+        return e == cudaSuccess;
+    }
+    std::pair<int, unsigned long long> stream() const { return {on_->device, on_->id}; }
     // Returns once the layout is final, for uses whose order this cannot see (copies, other libraries' kernels).
     void finish() {
         if (is_final()) return;
@@ -344,6 +350,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     py::class_<LayoutReady, std::shared_ptr<LayoutReady>>(m, "LayoutReady")
         .def(py::init<>())
         .def("wait", &LayoutReady::wait, py::call_guard<py::gil_scoped_release>())
+        .def("done", &LayoutReady::done, py::call_guard<py::gil_scoped_release>())
+        .def_property_readonly("stream", &LayoutReady::stream)
         .def("finish", &LayoutReady::finish, py::call_guard<py::gil_scoped_release>());
     m.def("build_layout", &build_layout, py::call_guard<py::gil_scoped_release>());
     m.def("quantize_many", &quantize_many, py::call_guard<py::gil_scoped_release>());
