@@ -780,13 +780,15 @@ cudaLaunchConfig_t pdl_config(dim3 grid, dim3 block, size_t smem, cudaStream_t s
 // of streaming), so that neither a nearly empty last wave nor many short CTAs dominate.
 // Prompts.  Rebuilding a k-tile of weights takes 0.35 us however many tokens use it, so the best tile is the one that holds
 // all tokens, or an even share of them: 300 tokens in one tile of 320 instead of two of 256 take 37 us instead of 58 at
-// 11008 x 4096, 36 instead of 48 at 4096 x 11008; 2048 tokens in six tiles of 384 instead of eight 193 instead of 228 at
-// 12288 x 4096, 359 instead of 415 at 22016 x 4096.  How that works out in waves of one CTA per SM is what PROMPT_TILES
+// 11008 x 4096, 36 instead of 48 at 4096 x 11008; 2048 tokens in six tiles of 384 instead of eight 195 instead of 224 at
+// 12288 x 4096.  How that works out in waves of one CTA per SM is what PROMPT_TILES
 // models: fitted to 5751 runs (16 shapes of 1024 x 1024 to 22016 x 4096, 129 to 2048 tokens, every tile and up to 8 slices),
-// 6.5 % off (rms).  A CTA takes `kt` per k-tile, more when all SMs work, and `fixed` besides; slicing adds a second kernel
+// 6.5 % off (rms), but it knows nothing of the power cap: where all SMs work for many waves it is
+// 15 to 20 % low (2048 x 22016 x 4096 in tiles of 256: 323 us for 376), and there the margin below keeps the tile of 256 where
+// one of 384 measured 6 % less.  A CTA takes `kt` per k-tile, more when all SMs work, and `fixed` besides; slicing adds a second kernel
 // and the fp32 partial sums' way through L2 and back.  A tile of 256 tokens sliced by its own, older rule is kept unless the
 // model sees a gain of 8 %, more than its error: of 239 shapes 4 are then slower than with that rule (by up to 15 %), and the
-// mean time is 0.92 of it (0.91 without the margin, with 13 slower; the best choices 0.89).
+// mean time is 0.92 of it (0.91 without the margin, with 13 slower; the best choices 0.89; all without the next rule).
 // No tile is cut into fewer slices than by that rule, since a longer run of products in one accumulator is less exact: with two
 // slices 2.2 % of the fp16 outputs of 4096 x 11008 at 301 tokens are not the product in 64 bits rounded once, with four 1.2 %.
 // This changes the choice for 45 of 3696 shapes, which take 12 % longer by the model.
